@@ -409,10 +409,15 @@ int topo_impl(int prec, int mem, int L, int N, const double* starts, const int32
   const int pad = topo_charge_pad(prec);
   const int64_t n_pad = ((std::max(N, 1) + int64_t(pad) - 1) / pad) * pad;
   unsigned char* packed = nullptr;
-  int* queue = nullptr;
+  int* queue = nullptr;  // the queue counter and, per round, the count of lines handed over
+  TopoState* left = nullptr;
+  const int rounds = topo_team_rounds(c->sms, L, topo_diag_steps(half, step));
+  const bool hand = rounds > 1 || L > int64_t(c->sms) * kTeamLinesPerSm;
+  const int left_cap = hand ? topo_left_capacity(c->sms, L) : 0;
   CK(S.get(&packed, size_t(n_pad) * topo_source_bytes(prec, source)), "alloc packed charges");
-  CK(S.get(&queue, 1), "alloc queue");
-  CK(cudaMemsetAsync(queue, 0, sizeof(int), s), "zero queue");
+  CK(S.get(&queue, size_t(1 + rounds)), "alloc queue");
+  CK(cudaMemsetAsync(queue, 0, (1 + rounds) * sizeof(int), s), "zero queue");
+  if (left_cap) CK(S.get(&left, 2 * size_t(left_cap)), "alloc hand-over records");
   if (reinterpret_cast<uintptr_t>(packed) % 16 != 0)
     return fail(CPETGB_ECUDA, "scratch allocation is not 16-byte aligned");
   if (source == kDipoles)
@@ -432,6 +437,10 @@ int topo_impl(int prec, int mem, int L, int N, const double* starts, const int32
   p.ends = dends;
   p.steps = dsteps;
   p.queue = queue;
+  p.left = left;
+  p.left_records = left_cap;
+  p.left_count = queue + 1;
+  p.rounds = rounds;
   p.status = c->status;
   CK(launch_topo(prec, p, c->sms, s), "topo kernel launch");
   if (mem == CPETGB_HOST) {
@@ -452,13 +461,21 @@ struct TopoTables {
   std::vector<TopoFrame> frames;
   std::vector<int64_t> src;  // per frame {charge offset, charge count} into x/q
   int64_t tot_lines = 0, tot_ch = 0, packed_elems = 0;
-  int max_res = 0, max_pairs = 0;
+  int64_t sum_lines = 0;      // lines of all frames (frames may share ranges)
+  int64_t left_records = 0;   // hand-over records of all frames
+  int rounds = 1;             // team kernel launches
+  double diag_steps = 0.0;    // the frames' largest box diagonal in steps
+  int max_res = 0, max_team_res = 0, max_pairs = 0;
   bool all_resident = true;  // every frame entirely in shared memory (tuner class 1)
 };
 
 // Frame table of a streamline launch: padded sizes, packed offsets (FP32C
 // frames occupy n_pad float4 -- the pair block A then B --, FP64 frames n_pad
-// Charge64), how many charges of each frame stay resident in shared memory.
+// Charge64), how many charges of each frame stay resident in shared memory, and
+// each frame's hand-over records (at most kMaxLeft in all; frames beyond that
+// have none and their lines end where they started).
+constexpr int64_t kMaxLeft = int64_t(1) << 18;  // two lists of 42 MB
+
 int build_topo_tables(int prec, int F, const int64_t* desc, const double* params, TopoTables& t) {
   if (!valid_prec(prec)) return fail(CPETGB_EINVAL, "bad precision %d", prec);
   if (F < 0 || (F > 0 && (!desc || !params))) return fail(CPETGB_EINVAL, "bad frame table");
@@ -481,7 +498,10 @@ int build_topo_tables(int prec, int F, const int64_t* desc, const double* params
     fr.line_off = lo;
     fr.n_lines = static_cast<int32_t>(L);
     fr.resident = topo_resident_count(prec, kCharges, fr.n_pad);
-    fr.pad_ = 0;
+    fr.team_resident = topo_team_resident(prec, kCharges, fr.n_pad);
+    t.max_team_res = std::max(t.max_team_res, int(fr.team_resident));
+    t.sum_lines += L;
+    t.diag_steps = std::max(t.diag_steps, topo_diag_steps(pr + 1, pr[0]));
     fr.step = pr[0];
     for (int k = 0; k < 3; ++k) fr.half[k] = pr[1 + k];
     t.max_res = std::max(t.max_res, int(fr.resident));
@@ -494,6 +514,17 @@ int build_topo_tables(int prec, int F, const int64_t* desc, const double* params
   }
   if (t.tot_lines > INT_MAX) return fail(CPETGB_EINVAL, "too many lines");
   return CPETGB_OK;
+}
+
+void plan_hand_over(int sms, TopoTables& t) {
+  t.rounds = topo_team_rounds(sms, t.sum_lines, t.diag_steps);
+  const bool hand = t.rounds > 1 || t.sum_lines > int64_t(sms) * kTeamLinesPerSm;
+  for (TopoFrame& fr : t.frames) {
+    const int64_t cap = hand ? topo_left_capacity(sms, fr.n_lines) : 0;
+    fr.left_off = static_cast<int32_t>(t.left_records);
+    fr.left_cap = t.left_records + cap <= kMaxLeft ? static_cast<int32_t>(cap) : 0;
+    t.left_records += fr.left_cap;
+  }
 }
 
 int topo_batch_impl(int prec, int mem, int F, const int64_t* desc, const double* params,
@@ -514,6 +545,7 @@ int topo_batch_impl(int prec, int mem, int F, const int64_t* desc, const double*
   int rc;
   Ctx* c = context(&rc);
   if (!c) return rc;
+  plan_hand_over(c->sms, t);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (mem == CPETGB_HOST && !s) s = c->stream;
   const size_t L = size_t(tot_lines);
@@ -543,8 +575,10 @@ int topo_batch_impl(int prec, int mem, int F, const int64_t* desc, const double*
     return fail(CPETGB_ECUDA, "scratch allocation is not 16-byte aligned");
   CK(h2d(&d_frames, S, frames.data(), frames.size()), "copy frame table");
   CK(h2d(&d_src, S, src.data(), src.size()), "copy frame sources");
-  CK(S.get(&queues, size_t(F)), "alloc queues");
-  CK(cudaMemsetAsync(queues, 0, sizeof(int) * size_t(F), s), "zero queues");
+  TopoState* left = nullptr;
+  CK(S.get(&queues, size_t(1 + t.rounds) * F), "alloc queues");
+  CK(cudaMemsetAsync(queues, 0, sizeof(int) * size_t(1 + t.rounds) * F, s), "zero queues");
+  if (t.left_records) CK(S.get(&left, 2 * size_t(t.left_records)), "alloc hand-over records");
   CK(launch_pack_topo_frames(prec, F, d_frames, d_src, dx, dq, packed, max_pairs, s),
      "pack charges");
   TopoParams p{};
@@ -556,10 +590,16 @@ int topo_batch_impl(int prec, int mem, int F, const int64_t* desc, const double*
   p.ends = dends;
   p.steps = dsteps;
   p.queue = queues;
+  p.left = left;
+  p.left_records = t.left_records;
+  p.left_count = queues + F;
+  p.rounds = t.rounds;
   p.status = c->status;
   p.frames = d_frames;
   p.n_frames = F;
   p.max_resident_pad = max_res;
+  p.max_team_resident = t.max_team_res;
+  p.sum_lines = t.sum_lines;
   p.all_resident = all_resident ? 1 : 0;
   CK(launch_topo_frames(prec, p, c->sms, s), "topo kernel launch");
   if (mem == CPETGB_HOST) {
@@ -964,17 +1004,20 @@ int topo_plan_impl(cpetgb_plan** out_plan, int prec, int F, const int64_t* desc,
   if (t.tot_ch > 0 && (!x || !q)) return fail(CPETGB_EINVAL, "charge pointer is NULL");
   Ctx* c = context(&rc);
   if (!c) return rc;
+  plan_hand_over(c->sms, t);
   cpetgb_plan* pl = new cpetgb_plan();
   cudaGetDevice(&pl->device);
   unsigned char* packed = nullptr;
   TopoFrame* d_frames = nullptr;
   int64_t* d_src = nullptr;
   int* queues = nullptr;
+  TopoState* left = nullptr;
   cudaError_t e =
       plan_alloc(pl->bufs, &packed, size_t(std::max<int64_t>(t.packed_elems, 1)) * packed_size(prec));
   if (e == cudaSuccess) e = plan_alloc(pl->bufs, &d_frames, t.frames.size());
   if (e == cudaSuccess) e = plan_alloc(pl->bufs, &d_src, t.src.size());
-  if (e == cudaSuccess) e = plan_alloc(pl->bufs, &queues, size_t(std::max(F, 1)));
+  if (e == cudaSuccess) e = plan_alloc(pl->bufs, &queues, size_t(1 + t.rounds) * std::max(F, 1));
+  if (e == cudaSuccess && t.left_records) e = plan_alloc(pl->bufs, &left, 2 * size_t(t.left_records));
   if (e == cudaSuccess && F > 0)
     e = cudaMemcpy(d_frames, t.frames.data(), t.frames.size() * sizeof(TopoFrame),
                    cudaMemcpyHostToDevice);
@@ -997,14 +1040,20 @@ int topo_plan_impl(cpetgb_plan** out_plan, int prec, int F, const int64_t* desc,
   p.ends = ends;
   p.steps = steps;
   p.queue = queues;
+  p.left = left;
+  p.left_records = t.left_records;
+  p.left_count = queues + F;
+  p.rounds = t.rounds;
   p.status = c->status;
   p.frames = d_frames;
   p.n_frames = F;
   p.max_resident_pad = t.max_res;
+  p.max_team_resident = t.max_team_res;
+  p.sum_lines = t.sum_lines;
   p.all_resident = t.all_resident ? 1 : 0;
   const int max_pairs = t.max_pairs;
   rc = capture_plan(pl, [&](cudaStream_t cs) -> int {
-    CK(cudaMemsetAsync(queues, 0, sizeof(int) * size_t(std::max(F, 1)), cs), "zero queues");
+    CK(cudaMemsetAsync(queues, 0, sizeof(int) * size_t(1 + p.rounds) * std::max(F, 1), cs), "zero queues");
     CK(launch_pack_topo_frames(prec, F, d_frames, d_src, x, q, packed, max_pairs, cs),
        "pack charges");
     CK(launch_topo_frames(prec, p, c->sms, cs), "topo kernel launch");

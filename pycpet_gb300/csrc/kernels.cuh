@@ -97,11 +97,21 @@ struct TopoFrame {
   int32_t n_pad;       // padded charge count (a multiple of topo_charge_pad(prec))
   int32_t n_lines;
   int32_t resident;    // charges staged in shared memory: n_pad, a prefix, or 0
-  int32_t pad_;
+  int32_t team_resident;  // the same in the team kernel (topo_team.cu)
+  int32_t left_off;    // the frame's hand-over records: first one and how many (0: none)
+  int32_t left_cap;
   double step;
   double half[3];
 };
-static_assert(sizeof(TopoFrame) == 64, "TopoFrame layout");
+static_assert(sizeof(TopoFrame) == 72, "TopoFrame layout");
+
+// A line in flight, handed from the persistent kernel to the team kernel.
+struct TopoState {
+  double x0[3], xip[3], xipp[3], xend[3], xe1[3];
+  double pos[3];
+  int32_t line, phase, steps, cap;
+};
+static_assert(sizeof(TopoState) == 160, "TopoState layout");
 
 struct TopoParams {
   int n_lines;
@@ -115,10 +125,16 @@ struct TopoParams {
   double* ends;              // [L][3] or null
   int32_t* steps;            // [L] or null (Euler steps of the main loop)
   int* queue;                // work-queue counter(s), one per frame (zeroed by the caller)
+  TopoState* left = nullptr;   // two lists of left_records hand-over records, or null: no hand-over
+  int64_t left_records = 0;
+  int* left_count = nullptr;   // records written: [rounds][n_frames] counters (zeroed by the caller)
+  int rounds = 1;              // team kernel launches (topo_team_rounds)
   int* status;
   const TopoFrame* frames;   // device frame table (multi-frame launches) or null
   int n_frames;              // frames in the table
   int max_resident_pad;      // largest TopoFrame::resident of the launch (shared-memory size)
+  int max_team_resident = 0;  // largest TopoFrame::team_resident of the launch
+  int64_t sum_lines = 0;      // lines of all frames of the table
   int all_resident = 0;      // 1: every frame entirely in shared memory (tuner class)
   int source = kCharges;     // kDipoles: packed holds dipoles (single-frame launches only)
 };
@@ -131,6 +147,23 @@ cudaError_t launch_topo_frames(int prec, const TopoParams& p, int num_sms, cudaS
 cudaError_t launch_pack_topo_frames(int prec, int n_frames, const TopoFrame* d_frames,
                                     const int64_t* d_src, const double* x, const double* q,
                                     void* packed, int max_pairs, cudaStream_t s);
+// Hand-over records of a frame of n_lines in each list (TopoFrame::left_cap).
+int topo_left_capacity(int num_sms, int64_t n_lines);
+
+// topo_team.cu: lines stepped by teams of warps, in p.rounds launches.  fresh !=
+// 0: the lines of the frames' tables from their start points; 0: the lines
+// handed over (p.left).
+cudaError_t launch_topo_team(int prec, const TopoParams& p, const TopoFrame& f0, int fresh,
+                             int num_sms, cudaStream_t s);
+int topo_team_resident(int prec, int source, int n_pad);
+// Launches of the team kernel for sum_lines lines whose box diagonal is crossed
+// in diag_steps steps (the largest of the launch's frames).
+int topo_team_rounds(int num_sms, int64_t sum_lines, double diag_steps);
+double topo_diag_steps(const double* half, double step);
+// a launch of at most this many lines per SM goes to the team kernel at once, and a CTA
+// of the persistent kernel hands its last lines over once it holds no more than this many
+constexpr int kTeamLinesPerSm = 16;
+
 // max sources (charges or dipoles) held resident in shared memory
 size_t topo_resident_limit(int prec, int source = kCharges);
 // sources of a frame of n_pad held in shared memory: n_pad when it fits, else

@@ -41,478 +41,93 @@
 
 #include "common.cuh"
 #include "kernels.cuh"
+#include "topo_lines.cuh"
 
 namespace cpetgb {
 namespace {
 
 constexpr int kTopoThreads = 512;
 constexpr int kTopoWarps = kTopoThreads / 32;
-constexpr int kLanePairs = 32;                  // charge pairs per lane between Kahan steps
-constexpr int kChargePad32 = 64;                // FP32C frames: one charge pair per lane
-constexpr int kChargePad64 = 256;               // FP64 frames
 // Line slots per warp S (template parameter): 4 (default) or 2.
-
-enum Phase : int { kMain = 0, kStart1 = 1, kStart2 = 2, kEnd1 = 3, kEnd2 = 4 };
-
-struct SlotRec {      // per-slot record in shared memory (owner lane only)
-  double x0[3], xip[3], xipp[3], xend[3], xe1[3];
-};
-
-__device__ __forceinline__ bool outside(const double p[3], const double h[3]) {
-  return p[0] < -h[0] || p[0] > h[0] || p[1] < -h[1] || p[1] > h[1] || p[2] < -h[2] ||
-         p[2] > h[2];
-}
-
-// Exact strict box test from the FP32 image pf = RN(p) of an FP64 position:
-// RN is monotonic, so |pf| > RN(h) implies |p| > h and |pf| < RN(h) implies
-// |p| < h; only a tie needs the FP64 comparison.
-__device__ __forceinline__ bool outside_fast(const double p[3], const float pf[3],
-                                             const double h[3], const float hf[3]) {
-  bool out = false;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const float a = fabsf(pf[k]);
-    if (a > hf[k] || (a == hf[k] && fabs(p[k]) > h[k])) out = true;
-  }
-  return out;
-}
-
-__device__ __forceinline__ double curve_f64(const double a[3], const double b[3]) {
-  const double c0 = a[1] * b[2] - a[2] * b[1];
-  const double c1 = a[2] * b[0] - a[0] * b[2];
-  const double c2 = a[0] * b[1] - a[1] * b[0];
-  const double nc = sqrt(c0 * c0 + c1 * c1 + c2 * c2);
-  const double na = sqrt(a[0] * a[0] + a[1] * a[1] + a[2] * a[2]);
-  return nc / (na * na * na);
-}
-
-// The frame a CTA is working on (uniform across the CTA).
-struct FrameCtx {
-  int64_t line_off;
-  int n_lines;
-  double step;
-  double half[3];
-  float hf[3];  // RN(half): the FP32 side of the exact box test
-};
-
-// Per-lane slot state (meaningful in lanes 0..S-1 only).
-struct Slot {
-  int line;     // -1 = idle
-  int phase;
-  int steps;
-  int cap;
-  double pos[3];  // where the next field evaluation happens
-  float posf[3];  // its FP32 image (FP32C pair terms)
-};
-
-__device__ __forceinline__ void set_pos(Slot& sl, const double v[3]) {
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    sl.pos[k] = v[k];
-    sl.posf[k] = static_cast<float>(v[k]);
-  }
-}
-
-__device__ void slot_load(Slot& sl, SlotRec& rec, int line, const TopoParams& p) {
-  sl.line = line;
-  if (line < 0) return;
-  const double* s = p.starts + 3 * static_cast<int64_t>(line);
-  double st[3];
-  for (int k = 0; k < 3; ++k) rec.x0[k] = st[k] = s[k];
-  set_pos(sl, st);
-  sl.cap = max(p.n_iter[line], 0);
-  if (sl.cap > kMaxLineCap) {  // refuse rather than run for hours
-    atomicCAS(p.status, kDevOk, kDevBadCap);
-    sl.cap = 0;
-  }
-  sl.steps = 0;
-  if (sl.cap > 0) {
-    sl.phase = kMain;
-  } else {  // no loop step: the end point is the start point
-    sl.phase = kStart1;
-    for (int k = 0; k < 3; ++k) rec.xend[k] = s[k];
-  }
-}
-
-// Advance one slot given the new position `nx` (= pos + step vector).
-// Returns true when the line has finished (result written).
-template <bool FAST_BOX>
-__device__ bool slot_advance(Slot& sl, SlotRec& rec, const double nx[3], const TopoParams& p,
-                             const FrameCtx& fc) {
-  switch (sl.phase) {
-    case kMain: {
-      sl.steps += 1;
-      if (sl.steps == 1)
-        for (int k = 0; k < 3; ++k) rec.xip[k] = nx[k];
-      if (sl.steps == 2)
-        for (int k = 0; k < 3; ++k) rec.xipp[k] = nx[k];
-      set_pos(sl, nx);
-      const bool out =
-          FAST_BOX ? outside_fast(sl.pos, sl.posf, fc.half, fc.hf) : outside(nx, fc.half);
-      if (out || sl.steps >= sl.cap) {
-        for (int k = 0; k < 3; ++k) rec.xend[k] = nx[k];
-        if (sl.steps >= 2) {
-          sl.phase = kEnd1;  // next evaluation at the end point (= nx)
-        } else {
-          sl.phase = kStart2;  // steps == 1: the end point is also x_init_plus
-        }
-      }
-      return false;
-    }
-    case kStart1:
-      for (int k = 0; k < 3; ++k) rec.xip[k] = nx[k];
-      set_pos(sl, nx);
-      sl.phase = kStart2;
-      return false;
-    case kStart2:
-      for (int k = 0; k < 3; ++k) rec.xipp[k] = nx[k];
-      set_pos(sl, rec.xend);
-      sl.phase = kEnd1;
-      return false;
-    case kEnd1:
-      for (int k = 0; k < 3; ++k) rec.xe1[k] = nx[k];
-      set_pos(sl, nx);
-      sl.phase = kEnd2;
-      return false;
-    default: {  // kEnd2: nx is the second step after the end point
-      double v1[3], v2[3], w1[3], w2[3], dd = 0.0;
-      for (int k = 0; k < 3; ++k) {
-        v1[k] = rec.xip[k] - rec.x0[k];
-        v2[k] = rec.xipp[k] - 2.0 * rec.xip[k] + rec.x0[k];
-        w1[k] = rec.xe1[k] - rec.xend[k];
-        w2[k] = nx[k] - 2.0 * rec.xe1[k] + rec.xend[k];
-        const double d = rec.x0[k] - rec.xend[k];
-        dd += d * d;
-      }
-      const int64_t li = sl.line;
-      p.result[2 * li + 0] = sqrt(dd);
-      p.result[2 * li + 1] = 0.5 * (curve_f64(v1, v2) + curve_f64(w1, w2));
-      if (p.ends)
-        for (int k = 0; k < 3; ++k) p.ends[3 * li + k] = rec.xend[k];
-      if (p.steps) p.steps[li] = sl.steps;
-      return true;
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Field sweep over the charges for NA active slots.
-// ---------------------------------------------------------------------------
-
-// FP32C.  Charges in "pair" layout: A[p] = {x_2p, x_2p+1, y_2p, y_2p+1},
-// B[p] = {z_2p, z_2p+1, q_2p, q_2p+1}, so each 64-bit half of a 16-byte load is
-// a ready operand of the packed f32x2 instructions: one instruction evaluates
-// a pair term for two charges.  Lanes take pairs lane-strided; every
-// kLanePairs pairs (fewer in a frame's last run: frames are padded to one pair
-// per lane only) the two packed streams are added and Kahan-accumulated.
-template <int NA, int S, int UNROLL>
-__device__ __forceinline__ void pair_run(const ulonglong2* __restrict__ A,
-                                         const ulonglong2* __restrict__ B, int base, int cnt,
-                                         const uint64_t (&ex2)[S][3], uint64_t (&part)[NA][3]) {
-#pragma unroll UNROLL
-  for (int i = 0; i < cnt; ++i) {
-    const ulonglong2 a = A[base + 32 * i];  // {x pair, y pair}
-    const ulonglong2 b = B[base + 32 * i];  // {z pair, q pair}
-#pragma unroll
-    for (int e = 0; e < NA; ++e) {
-      const uint64_t dx = sub2(ex2[e][0], a.x);
-      const uint64_t dy = sub2(ex2[e][1], a.y);
-      const uint64_t dz = sub2(ex2[e][2], b.x);
-      const uint64_t r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
-      const uint64_t ri = rsqrt2(r2);
-      const uint64_t w = mul2(mul2(b.y, ri), mul2(ri, ri));
-      part[e][0] = fma2(w, dx, part[e][0]);
-      part[e][1] = fma2(w, dy, part[e][1]);
-      part[e][2] = fma2(w, dz, part[e][2]);
-    }
-  }
-}
-
-// Dipole pairs: A[p] = {x pair, y pair}, B[p] = {z pair, 3 mu_x pair},
-// C[p] = {mu_y pair, mu_z pair}.  Per dipole the term of
-// calc_field_base_dipole (CPET/utils/math_module.c:335-371) without the
-// constant factor (the step only uses the field's direction):
-//   r^-5 ((3 mu_x R_x + mu_y R_y + mu_z R_z) R_c - mu_c r^2)
-//   = w R_c - r^-3 mu_c,  w = (3 mu_x R_x + mu_y R_y + mu_z R_z) r^-5,
-// the x component taking mu_x as (3 mu_x) * (-1/3) r^-3.
-template <int NA, int S, int UNROLL>
-__device__ __forceinline__ void dipole_run(const ulonglong2* __restrict__ A,
-                                           const ulonglong2* __restrict__ B,
-                                           const ulonglong2* __restrict__ C, int base, int cnt,
-                                           const uint64_t (&ex2)[S][3], uint64_t (&part)[NA][3]) {
-  const uint64_t m_third = pk2(-1.f / 3.f, -1.f / 3.f), m_one = pk2(-1.f, -1.f);
-#pragma unroll UNROLL
-  for (int i = 0; i < cnt; ++i) {
-    const ulonglong2 a = A[base + 32 * i];  // {x pair, y pair}
-    const ulonglong2 b = B[base + 32 * i];  // {z pair, 3 mu_x pair}
-    const ulonglong2 c = C[base + 32 * i];  // {mu_y pair, mu_z pair}
-#pragma unroll
-    for (int e = 0; e < NA; ++e) {
-      const uint64_t dx = sub2(ex2[e][0], a.x);
-      const uint64_t dy = sub2(ex2[e][1], a.y);
-      const uint64_t dz = sub2(ex2[e][2], b.x);
-      const uint64_t r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
-      const uint64_t ri = rsqrt2(r2);
-      const uint64_t ri2 = mul2(ri, ri);
-      const uint64_t ri3 = mul2(ri2, ri);
-      const uint64_t w = mul2(fma2(b.y, dx, fma2(c.x, dy, mul2(c.y, dz))), mul2(ri3, ri2));
-      const uint64_t t3 = mul2(ri3, m_third), tn = mul2(ri3, m_one);
-      part[e][0] = fma2(t3, b.y, fma2(w, dx, part[e][0]));
-      part[e][1] = fma2(tn, c.x, fma2(w, dy, part[e][1]));
-      part[e][2] = fma2(tn, c.y, fma2(w, dz, part[e][2]));
-    }
-  }
-}
-
-// Sources of a sweep.  kSrcOne: every pair from (A, B, C) -- a frame held
-// entirely in shared memory, or one read entirely from global memory.
-// kSrcSplit: pairs [0, res_pairs) from (sA, sB, sC), the shared-memory copy of
-// a frame's first pairs, the rest from (A, B, C) in global memory (L2);
-// res_pairs is a multiple of the 32 x kLanePairs pairs of one Kahan run, so
-// every run reads one source and the sums are the same whichever part is
-// resident.  The single-source loop is compiled on its own: with both sources
-// in one loop the all-resident sweep ran 12% slower.
-constexpr int kSrcOne = 0;
-constexpr int kSrcSplit = 1;
-
-// DIP: point dipoles (dipole_run, C used); otherwise point charges (pair_run).
-template <int NA, int S, bool DIP = false, int SRC = kSrcOne>
-__device__ __forceinline__ void sweep_f32x2(const ulonglong2* __restrict__ sA,
-                                            const ulonglong2* __restrict__ sB,
-                                            const ulonglong2* __restrict__ sC, int res_pairs,
-                                            const ulonglong2* __restrict__ A,
-                                            const ulonglong2* __restrict__ B,
-                                            const ulonglong2* __restrict__ C, int n_pairs,
-                                            int lane, const uint64_t (&ex2)[S][3], float& total) {
-  float acc[NA][3], cmp[NA][3];
-#pragma unroll
-  for (int e = 0; e < NA; ++e)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) acc[e][c] = cmp[e][c] = 0.f;
-
-  // n_pairs is a multiple of 32: every lane runs the same number of pairs
-  for (int base = 0; base < n_pairs; base += 32 * kLanePairs) {
-    uint64_t part[NA][3];
-#pragma unroll
-    for (int e = 0; e < NA; ++e)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) part[e][c] = 0ull;
-    const int left = (n_pairs - base) >> 5;
-    // about eight independent pair chains in flight per lane: unroll 8 / NA
-    constexpr int kUnroll = NA >= 3 ? 2 : (NA == 2 ? 4 : 8);
-    const int cnt = left >= kLanePairs ? kLanePairs : left;
-    if (SRC == kSrcSplit && base < res_pairs) {  // shared-memory copy
-      if constexpr (DIP) {
-        if (cnt == kLanePairs)
-          dipole_run<NA, S, kUnroll>(sA, sB, sC, base + lane, kLanePairs, ex2, part);
-        else
-          dipole_run<NA, S, 1>(sA, sB, sC, base + lane, cnt, ex2, part);
-      } else {
-        if (cnt == kLanePairs)
-          pair_run<NA, S, kUnroll>(sA, sB, base + lane, kLanePairs, ex2, part);
-        else
-          pair_run<NA, S, 1>(sA, sB, base + lane, cnt, ex2, part);
-      }
-    } else {  // global memory (kSrcSplit), or the one source
-      if constexpr (DIP) {
-        if (cnt == kLanePairs)
-          dipole_run<NA, S, kUnroll>(A, B, C, base + lane, kLanePairs, ex2, part);
-        else
-          dipole_run<NA, S, 1>(A, B, C, base + lane, cnt, ex2, part);
-      } else {
-        if (cnt == kLanePairs)
-          pair_run<NA, S, kUnroll>(A, B, base + lane, kLanePairs, ex2, part);
-        else
-          pair_run<NA, S, 1>(A, B, base + lane, cnt, ex2, part);
-      }
-    }
-#pragma unroll
-    for (int e = 0; e < NA; ++e)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        float lo, hi2;
-        upk2(part[e][c], lo, hi2);
-        kahan_add(acc[e][c], cmp[e][c], __fadd_rn(lo, hi2));
-      }
-  }
-  // Lane partials (acc - cmp, unevaluated pairs) as NV = 4S values v = 3e + c,
-  // reduced across the warp by a reduce-scatter of error-free pair additions:
-  // each of the LV levels halves the values a lane keeps, a butterfly finishes;
-  // afterwards the lanes with (lane >> (5 - LV)) == v hold the total of value v.
-  constexpr int NV = 4 * S;
-  constexpr int LV = (S == 4) ? 4 : 3;
-  float h[NV], l[NV];
-#pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    const int e = v / 3, c = v % 3;
-    h[v] = (e < NA) ? acc[e < NA ? e : 0][c] : 0.f;
-    l[v] = (e < NA) ? -cmp[e < NA ? e : 0][c] : 0.f;
-  }
-#pragma unroll
-  for (int lvl = 0, half = NV / 2; lvl < LV; ++lvl, half >>= 1) {
-    const int off = 16 >> lvl;
-    const bool upper = (lane & off) != 0;
-#pragma unroll
-    for (int j = 0; j < half; ++j) {
-      const float sh = upper ? h[j] : h[j + half];
-      const float sl = upper ? l[j] : l[j + half];
-      const float kh = upper ? h[j + half] : h[j];
-      const float kl = upper ? l[j + half] : l[j];
-      const float rh = __shfl_xor_sync(0xffffffffu, sh, off);
-      const float rl = __shfl_xor_sync(0xffffffffu, sl, off);
-      h[j] = kh;
-      l[j] = kl;
-      pair_add(h[j], l[j], rh, rl);
-    }
-  }
-#pragma unroll
-  for (int off = 16 >> LV; off >= 1; off >>= 1) {
-    const float rh = __shfl_xor_sync(0xffffffffu, h[0], off);
-    const float rl = __shfl_xor_sync(0xffffffffu, l[0], off);
-    pair_add(h[0], l[0], rh, rl);
-  }
-  total = h[0];
-}
-
-// FP64: charges from global memory (padded with zero charges far away).  Every
-// operation in double precision; r^-1 from the double rsqrt (1 ulp), whose few
-// FP64-pipe operations replace a correctly rounded sqrt and division (GB300's
-// FP64 pipe is 1/64 of its FP32 pipe).
-template <int NA, int S>
-__device__ __forceinline__ void sweep_f64(const Charge64* __restrict__ g, int n_pad, int lane,
-                                          const double (&ex)[S][3], double (&E)[S][3]) {
-  double acc[NA][3];
-#pragma unroll
-  for (int e = 0; e < NA; ++e)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) acc[e][c] = 0.0;
-#pragma unroll 2
-  for (int j = lane; j < n_pad; j += 32) {
-    const Charge64 ch = g[j];
-#pragma unroll
-    for (int e = 0; e < NA; ++e) {
-      const double dx = __dsub_rn(ex[e][0], ch.x);
-      const double dy = __dsub_rn(ex[e][1], ch.y);
-      const double dz = __dsub_rn(ex[e][2], ch.z);
-      const double r2 = __fma_rn(dx, dx, __fma_rn(dy, dy, __dmul_rn(dz, dz)));
-      const double ri = rsqrt(r2);  // double-precision reciprocal square root (1 ulp)
-      const double w = __dmul_rn(ch.q, __dmul_rn(ri, __dmul_rn(ri, ri)));
-      acc[e][0] = __fma_rn(w, dx, acc[e][0]);
-      acc[e][1] = __fma_rn(w, dy, acc[e][1]);
-      acc[e][2] = __fma_rn(w, dz, acc[e][2]);
-    }
-  }
-#pragma unroll
-  for (int e = 0; e < NA; ++e)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      double v = acc[e][c];
-#pragma unroll
-      for (int off = 16; off >= 1; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-      E[e][c] = v;
-    }
-}
-
-// FP64 dipoles: Dipole64 records read from global memory (L2), padded with
-// zero moments far away.  Same term as dipole_run, in double precision (r^-1
-// from the double rsqrt, as sweep_f64).
-template <int NA, int S>
-__device__ __forceinline__ void sweep_dipole_f64(const Dipole64* __restrict__ g, int n_pad, int lane,
-                                                 const double (&ex)[S][3], double (&E)[S][3]) {
-  double acc[NA][3];
-#pragma unroll
-  for (int e = 0; e < NA; ++e)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) acc[e][c] = 0.0;
-#pragma unroll 2
-  for (int j = lane; j < n_pad; j += 32) {
-    const Dipole64 d = g[j];
-#pragma unroll
-    for (int e = 0; e < NA; ++e) {
-      const double dx = __dsub_rn(ex[e][0], d.x);
-      const double dy = __dsub_rn(ex[e][1], d.y);
-      const double dz = __dsub_rn(ex[e][2], d.z);
-      const double r2 = __fma_rn(dx, dx, __fma_rn(dy, dy, __dmul_rn(dz, dz)));
-      const double ri = rsqrt(r2);  // double-precision reciprocal square root (1 ulp)
-      const double ri2 = __dmul_rn(ri, ri);
-      const double r5 = __dmul_rn(__dmul_rn(ri2, ri2), ri);
-      const double dot = __fma_rn(3.0 * d.mx, dx, __fma_rn(d.my, dy, __dmul_rn(d.mz, dz)));
-      acc[e][0] = __fma_rn(r5, __fma_rn(dot, dx, -__dmul_rn(d.mx, r2)), acc[e][0]);
-      acc[e][1] = __fma_rn(r5, __fma_rn(dot, dy, -__dmul_rn(d.my, r2)), acc[e][1]);
-      acc[e][2] = __fma_rn(r5, __fma_rn(dot, dz, -__dmul_rn(d.mz, r2)), acc[e][2]);
-    }
-  }
-#pragma unroll
-  for (int e = 0; e < NA; ++e)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      double v = acc[e][c];
-#pragma unroll
-      for (int off = 16; off >= 1; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-      E[e][c] = v;
-    }
-}
 
 // ---------------------------------------------------------------------------
 // Persistent kernel.
 // ---------------------------------------------------------------------------
 
-// Residency of a launch's frames (kernel template RES): kResNone -- every
-// frame read from global memory (L2); kResWhole -- each frame entirely in
-// shared memory or read from L2; kResAny -- also frames of which only a prefix
-// is resident (frames above the shared-memory limit).  The prefix sweeps are
-// compiled only into kResAny kernels: with them in the kernel of whole-frame
-// launches its instruction cache missed (no-instruction stalls 0.31 per issue
-// instead of 0.05) and the 8,000-charge workload ran 6% slower.
-constexpr int kResNone = 0;
-constexpr int kResWhole = 1;
-constexpr int kResAny = 2;
+// Hand-over of a frame's last lines.  Once the queue is empty and a CTA holds at
+// most kTeamLinesPerSm lines, most of its warps have nothing to do and the rest
+// sweep a line alone; its warps then write their lines' states to the frame's
+// records and leave, and the team kernel finishes them, spread over all SMs.
+struct HandOver {
+  TopoState* rec;  // the frame's records
+  int* count;      // records written
+  int cap;         // 0: no hand-over
+};
 
-// The sweep of one frame of a kResAny launch: res_pairs of its n_pairs pairs
-// are in shared memory.
-template <int NA, int S, bool DIP>
-__device__ __forceinline__ void sweep_frame_any(const ulonglong2* smA, const ulonglong2* smB,
-                                                const ulonglong2* smC, int res_pairs,
-                                                const ulonglong2* chA, const ulonglong2* chB,
-                                                const ulonglong2* chC, int n_pairs, int lane,
-                                                const uint64_t (&ex2)[S][3], float& total) {
-  if (res_pairs >= n_pairs)
-    sweep_f32x2<NA, S, DIP, kSrcOne>(nullptr, nullptr, nullptr, 0, smA, smB, smC, n_pairs, lane, ex2,
-                                     total);
-  else if (res_pairs > 0)
-    sweep_f32x2<NA, S, DIP, kSrcSplit>(smA, smB, smC, res_pairs, chA, chB, chC, n_pairs, lane, ex2,
-                                       total);
-  else
-    sweep_f32x2<NA, S, DIP, kSrcOne>(nullptr, nullptr, nullptr, 0, chA, chB, chC, n_pairs, lane, ex2,
-                                     total);
+__device__ __forceinline__ bool hand_over(const HandOver& h, const Slot& sl, const SlotRec& rec,
+                                       unsigned active, int lane) {
+  const int na = __popc(active);
+  const int leader = __ffs(active) - 1;
+  int base = 0;
+  if (lane == leader) {
+    base = atomicAdd(h.count, na);
+    if (base + na > h.cap) {  // no room: taken back, the warp keeps its lines
+      atomicSub(h.count, na);
+      base = -1;
+    }
+  }
+  base = __shfl_sync(0xffffffffu, base, leader);
+  if (base < 0) return false;
+  if ((active >> lane) & 1u) {
+    TopoState* t = h.rec + base + __popc(active & ((1u << lane) - 1u));
+    for (int k = 0; k < 3; ++k) {
+      t->x0[k] = rec.x0[k];
+      t->xip[k] = rec.xip[k];
+      t->xipp[k] = rec.xipp[k];
+      t->xend[k] = rec.xend[k];
+      t->xe1[k] = rec.xe1[k];
+      t->pos[k] = sl.pos[k];
+    }
+    t->line = sl.line;
+    t->phase = sl.phase;
+    t->steps = sl.steps;
+    t->cap = sl.cap;
+  }
+  return true;
 }
 
-// One line slot set per warp; processes the lines of frame `fc` (charge
-// arrays chA/chB in the FP32C pair layout, or g in Charge64) until the frame's
-// queue is exhausted and the warp's slots are drained.
-// resident: the whole frame is in shared memory (kResWhole launches);
-// res_pairs: pairs in shared memory (kResAny launches).
-template <int PREC, int S, bool DIP, int RES>
+// One line slot set per warp; processes the lines of frame `fc` (g: its sources
+// in global memory, FP32C in the pair layout; res_pairs of its pairs also in
+// shared memory at sm_off) until the frame's queue is exhausted and the warp's
+// slots are drained.
+template <int PREC, int S, bool DIP, int SRC>
 __device__ __forceinline__ void run_frame(const TopoParams& p, const FrameCtx& fc, int* queue,
-                                          const ulonglong2* chA, const ulonglong2* chB,
-                                          const ulonglong2* chC, const ulonglong2* smA,
-                                          const ulonglong2* smB, const ulonglong2* smC,
-                                          bool resident, int res_pairs, int n_pad, SlotRec* my_rec,
-                                          int lane) {
+                                          const ulonglong2* g, uint32_t sm_off, int res_pairs, int n_pad,
+                                          SlotRec* my_rec, int lane, const HandOver& hand, int* s_idle) {
   Slot sl;
   sl.line = -1;
   sl.phase = kMain;
   sl.steps = sl.cap = 0;
   sl.pos[0] = sl.pos[1] = sl.pos[2] = 0.0;
   sl.posf[0] = sl.posf[1] = sl.posf[2] = 0.f;
+  // One frame: the first lines are dealt out evenly over the CTAs, the queue
+  // hands out the rest.  A table of frames: all from the queue (a CTA may reach
+  // a frame late, or not at all).
+  const int dealt = p.frames ? 0 : static_cast<int>(gridDim.x) * kTopoWarps * S;
   if (lane < S) {
-    const int li = atomicAdd(queue, 1);
+    const int li = p.frames ? atomicAdd(queue, 1)
+                            : (lane * kTopoWarps + (threadIdx.x >> 5)) * static_cast<int>(gridDim.x) +
+                                  static_cast<int>(blockIdx.x);
+    if (li >= fc.n_lines) atomicAdd(s_idle, 1);
     slot_load(sl, *my_rec, li < fc.n_lines ? static_cast<int>(fc.line_off + li) : -1, p);
   }
   for (;;) {
     const unsigned active = __ballot_sync(0xffffffffu, lane < S && sl.line >= 0);
     const int na = __popc(active);
     if (na == 0) break;
+    if (hand.cap > 0 && *reinterpret_cast<volatile int*>(s_idle) >= kTopoWarps * S - kTeamLinesPerSm &&
+        hand_over(hand, sl, *my_rec, active, lane))
+      break;
     // owner lane of each active slot, in order; this lane's rank among them
     int src_of[S];
     int my_rank = -1;
@@ -528,60 +143,9 @@ __device__ __forceinline__ void run_frame(const TopoParams& p, const FrameCtx& f
 
     double nx[3];
     if constexpr (PREC == kFP32C) {
-      uint64_t ex2[S][3];
-#pragma unroll
-      for (int e = 0; e < S; ++e)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const float v = __shfl_sync(0xffffffffu, sl.posf[c], src_of[e]);
-          ex2[e][c] = pk2(v, v);
-        }
-      float total;
-      const int n_pairs = n_pad / 2;
-      if constexpr (RES == kResAny) {
-        switch (na) {
-          case 1:
-            sweep_frame_any<1, S, DIP>(smA, smB, smC, res_pairs, chA, chB, chC, n_pairs, lane, ex2, total);
-            break;
-          case 2:
-            sweep_frame_any<2, S, DIP>(smA, smB, smC, res_pairs, chA, chB, chC, n_pairs, lane, ex2, total);
-            break;
-          case 3:
-            sweep_frame_any<(S > 2 ? 3 : 2), S, DIP>(smA, smB, smC, res_pairs, chA, chB, chC, n_pairs,
-                                                     lane, ex2, total);
-            break;
-          default:
-            sweep_frame_any<S, S, DIP>(smA, smB, smC, res_pairs, chA, chB, chC, n_pairs, lane, ex2, total);
-            break;
-        }
-      } else if (resident) {  // whole frame in shared memory
-        switch (na) {
-          case 1: sweep_f32x2<1, S, DIP>(nullptr, nullptr, nullptr, 0, smA, smB, smC, n_pairs, lane, ex2, total); break;
-          case 2: sweep_f32x2<2, S, DIP>(nullptr, nullptr, nullptr, 0, smA, smB, smC, n_pairs, lane, ex2, total); break;
-          case 3: sweep_f32x2<(S > 2 ? 3 : 2), S, DIP>(nullptr, nullptr, nullptr, 0, smA, smB, smC, n_pairs, lane, ex2, total); break;
-          default: sweep_f32x2<S, S, DIP>(nullptr, nullptr, nullptr, 0, smA, smB, smC, n_pairs, lane, ex2, total); break;
-        }
-      } else {  // every pair from global memory
-        switch (na) {
-          case 1: sweep_f32x2<1, S, DIP>(nullptr, nullptr, nullptr, 0, chA, chB, chC, n_pairs, lane, ex2, total); break;
-          case 2: sweep_f32x2<2, S, DIP>(nullptr, nullptr, nullptr, 0, chA, chB, chC, n_pairs, lane, ex2, total); break;
-          case 3: sweep_f32x2<(S > 2 ? 3 : 2), S, DIP>(nullptr, nullptr, nullptr, 0, chA, chB, chC, n_pairs, lane, ex2, total); break;
-          default: sweep_f32x2<S, S, DIP>(nullptr, nullptr, nullptr, 0, chA, chB, chC, n_pairs, lane, ex2, total); break;
-        }
-      }
-      // component c of slot rank e sits in lanes (3e + c) << (5 - LV) and up
       float Ef[3];
-      const int rk = my_rank >= 0 ? my_rank : 0;
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        Ef[c] = __shfl_sync(0xffffffffu, total, (3 * rk + c) << (S == 4 ? 1 : 2));
-      if (my_rank >= 0) {
-        // step vector in FP32 (the factor k does not change the direction)
-        const float n2 = __fmaf_rn(Ef[0], Ef[0], __fmaf_rn(Ef[1], Ef[1], __fmul_rn(Ef[2], Ef[2])));
-        const float s = __fdiv_rn(static_cast<float>(fc.step), __fsqrt_rn(n2));
-#pragma unroll
-        for (int c = 0; c < 3; ++c) nx[c] = sl.pos[c] + static_cast<double>(__fmul_rn(Ef[c], s));
-      }
+      sweep_slots<S, DIP, SRC>(na, sl.posf, src_of, max(my_rank, 0), sm_off, res_pairs, g, n_pad / 2, Ef);
+      if (my_rank >= 0) euler_step(Ef, sl.pos, fc.step, nx);
     } else {
       double ex[S][3];
 #pragma unroll
@@ -590,20 +154,20 @@ __device__ __forceinline__ void run_frame(const TopoParams& p, const FrameCtx& f
         for (int c = 0; c < 3; ++c) ex[e][c] = __shfl_sync(0xffffffffu, sl.pos[c], src_of[e]);
       double Es[S][3];
       if constexpr (DIP) {
-        const Dipole64* g = reinterpret_cast<const Dipole64*>(chA);
+        const Dipole64* src = reinterpret_cast<const Dipole64*>(g);
         switch (na) {
-          case 1: sweep_dipole_f64<1, S>(g, n_pad, lane, ex, Es); break;
-          case 2: sweep_dipole_f64<2, S>(g, n_pad, lane, ex, Es); break;
-          case 3: sweep_dipole_f64<(S > 2 ? 3 : 2), S>(g, n_pad, lane, ex, Es); break;
-          default: sweep_dipole_f64<S, S>(g, n_pad, lane, ex, Es); break;
+          case 1: sweep_f64<1, S>(src, n_pad, lane, ex, Es); break;
+          case 2: sweep_f64<2, S>(src, n_pad, lane, ex, Es); break;
+          case 3: sweep_f64<(S > 2 ? 3 : 2), S>(src, n_pad, lane, ex, Es); break;
+          default: sweep_f64<S, S>(src, n_pad, lane, ex, Es); break;
         }
       } else {
-        const Charge64* g = reinterpret_cast<const Charge64*>(chA);
+        const Charge64* src = reinterpret_cast<const Charge64*>(g);
         switch (na) {
-          case 1: sweep_f64<1, S>(g, n_pad, lane, ex, Es); break;
-          case 2: sweep_f64<2, S>(g, n_pad, lane, ex, Es); break;
-          case 3: sweep_f64<(S > 2 ? 3 : 2), S>(g, n_pad, lane, ex, Es); break;
-          default: sweep_f64<S, S>(g, n_pad, lane, ex, Es); break;
+          case 1: sweep_f64<1, S>(src, n_pad, lane, ex, Es); break;
+          case 2: sweep_f64<2, S>(src, n_pad, lane, ex, Es); break;
+          case 3: sweep_f64<(S > 2 ? 3 : 2), S>(src, n_pad, lane, ex, Es); break;
+          default: sweep_f64<S, S>(src, n_pad, lane, ex, Es); break;
         }
       }
       if (my_rank >= 0) {
@@ -613,15 +177,14 @@ __device__ __forceinline__ void run_frame(const TopoParams& p, const FrameCtx& f
           if (e == my_rank)
 #pragma unroll
             for (int c = 0; c < 3; ++c) E[c] = Es[e][c];
-        const double n = sqrt(E[0] * E[0] + E[1] * E[1] + E[2] * E[2]);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) nx[c] = sl.pos[c] + fc.step * E[c] / n;
+        euler_step(E, sl.pos, fc.step, nx);
       }
     }
 
     if (my_rank >= 0) {
       if (slot_advance<PREC == kFP32C>(sl, *my_rec, nx, p, fc)) {
-        const int li = atomicAdd(queue, 1);
+        const int li = dealt + atomicAdd(queue, 1);
+        if (li >= fc.n_lines) atomicAdd(s_idle, 1);
         slot_load(sl, *my_rec, li < fc.n_lines ? static_cast<int>(fc.line_off + li) : -1, p);
       }
     }
@@ -630,26 +193,28 @@ __device__ __forceinline__ void run_frame(const TopoParams& p, const FrameCtx& f
 }
 
 // Frames are visited in table order; a CTA stays on a frame while its line
-// queue lasts, then moves on (after its own warps are done, so the shared
-// copy of the charges can be replaced).  Frames thus overlap only at their
-// tails and every frame switch costs a CTA one line's latency at most.
+// queue lasts, then moves on (after its own warps are done or have handed their
+// lines over, so the shared copy of the charges can be replaced).  Frames thus
+// overlap only at their tails.
 // DIP: the sources are point dipoles (FP32C: three 16-byte pair blocks per
-// frame; FP64: Dipole64 records) instead of point charges.  RES: residency
-// mode of the launch's frames (kResNone, kResWhole, kResAny).
-template <int PREC, int RES, int S, bool DIP>
+// frame; FP64: Dipole64 records) instead of point charges.  SRC: kSrcShared when
+// every frame of the launch fits shared memory, kSrcSplit otherwise (FP64:
+// always, its sources are read from global memory).
+template <int PREC, int S, bool DIP, int SRC>
 __global__ void __launch_bounds__(kTopoThreads, 1) topo_kernel(TopoParams p, TopoFrame frame0) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ int s_skip;
+  __shared__ int s_idle;  // line slots of this CTA that found the frame's queue empty
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   SlotRec* recs = reinterpret_cast<SlotRec*>(smem_raw);  // [kTopoWarps][S]
-  const size_t rec_bytes = sizeof(SlotRec) * kTopoWarps * S;
+  constexpr uint32_t rec_bytes = sizeof(SlotRec) * kTopoWarps * S;
+  constexpr uint32_t sm_off = rec_bytes + 128;  // the resident sources
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + rec_bytes);
-  ulonglong2* sm_ch = reinterpret_cast<ulonglong2*>(smem_raw + rec_bytes + 128);
   SlotRec* my_rec = recs + warp * S + (lane < S ? lane : 0);
   const int n_frames = p.frames ? p.n_frames : 1;
   uint32_t load_parity = 0;
-  if (RES != kResNone && threadIdx.x == 0) {
+  if (PREC == kFP32C && threadIdx.x == 0) {
     mbar_init(bar, 1);
     fence_mbar_init();
   }
@@ -658,53 +223,34 @@ __global__ void __launch_bounds__(kTopoThreads, 1) topo_kernel(TopoParams p, Top
     const TopoFrame fr = p.frames ? p.frames[f] : frame0;
     int* queue = p.queue + f;
     __syncthreads();  // the CTA's warps are done with the previous frame
-    if (threadIdx.x == 0) s_skip = (*reinterpret_cast<volatile int*>(queue) >= fr.n_lines) ? 1 : 0;
+    if (threadIdx.x == 0) {
+      // a table's frame may be used up before this CTA reaches it; a single
+      // frame's first lines are dealt to this CTA whatever the queue says
+      s_skip = p.frames && *reinterpret_cast<volatile int*>(queue) >= fr.n_lines;
+      s_idle = 0;
+    }
     __syncthreads();
     if (s_skip) continue;
-    // sources in shared memory.  kResAny: the frame's first fr.resident
-    // sources -- all of them, or a prefix of whole Kahan runs when the frame
-    // exceeds shared memory -- copied block by block.  Otherwise whole frames
-    // (the host launches kResWhole only when every resident frame is entirely
-    // so) in one contiguous copy of the packed blocks: written as the
-    // block-wise copy, that kernel was compiled to a schedule 6% slower on
-    // the 8,000-charge workload.
-    int res = 0;
-    bool resident = false;
-    if constexpr (RES == kResAny) {
-      res = fr.resident;
-      if (res > 0) {
-        if (threadIdx.x == 0) {
-          const uint32_t blk = static_cast<uint32_t>(res / 2) * 16u;  // bytes of one block's prefix
-          const int n_blk = DIP ? 3 : 2;
-          mbar_arrive_expect_tx(bar, blk * n_blk);
-          const char* src = static_cast<const char*>(p.packed) + fr.packed_off * 16;
-          constexpr uint32_t kChunk = 32768;
-          for (int b = 0; b < n_blk; ++b) {  // block b of the frame starts at b * n_pad/2 pairs
-            const char* bs = src + static_cast<size_t>(b) * (fr.n_pad / 2) * 16;
-            char* bd = reinterpret_cast<char*>(sm_ch) + static_cast<size_t>(b) * blk;
-            for (uint32_t off = 0; off < blk; off += kChunk)
-              bulk_g2s(bd + off, bs + off, min(kChunk, blk - off), bar);
-          }
+    const size_t elem = (PREC == kFP32C) ? 16 : 32;
+    const char* src = static_cast<const char*>(p.packed) + fr.packed_off * elem;
+    if constexpr (PREC == kFP32C) {
+      // the frame's first fr.resident sources -- all of them, or a prefix of
+      // whole Kahan runs when the frame exceeds shared memory -- block by block
+      if (threadIdx.x == 0) {
+        const uint32_t blk = static_cast<uint32_t>(fr.resident / 2) * 16u;  // bytes of one block's prefix
+        constexpr int n_blk = DIP ? 3 : 2;
+        mbar_arrive_expect_tx(bar, blk * n_blk);
+        constexpr uint32_t kChunk = 32768;
+        for (int b = 0; b < n_blk; ++b) {  // block b of the frame starts at b * n_pad/2 pairs
+          const char* bs = src + static_cast<size_t>(b) * (fr.n_pad / 2) * 16;
+          unsigned char* bd = smem_raw + sm_off + static_cast<size_t>(b) * blk;
+          for (uint32_t off = 0; off < blk; off += kChunk)
+            bulk_g2s(bd + off, bs + off, min(kChunk, blk - off), bar);
         }
-        const bool mine = mbar_wait(bar, load_parity, p.status);
-        load_parity ^= 1u;
-        if (!__syncthreads_and(mine)) return;
       }
-    } else {
-      resident = RES == kResWhole && fr.resident;
-      if (resident) {
-        if (threadIdx.x == 0) {
-          const uint32_t total = static_cast<uint32_t>(fr.n_pad) * (DIP ? 24u : 16u);
-          mbar_arrive_expect_tx(bar, total);
-          const char* src = static_cast<const char*>(p.packed) + fr.packed_off * 16;
-          constexpr uint32_t kChunk = 32768;
-          for (uint32_t off = 0; off < total; off += kChunk)
-            bulk_g2s(reinterpret_cast<char*>(sm_ch) + off, src + off, min(kChunk, total - off), bar);
-        }
-        const bool mine = mbar_wait(bar, load_parity, p.status);
-        load_parity ^= 1u;
-        if (!__syncthreads_and(mine)) return;
-      }
+      const bool mine = mbar_wait(bar, load_parity, p.status);
+      load_parity ^= 1u;
+      if (!__syncthreads_and(mine)) return;
     }
     FrameCtx fc;
     fc.line_off = fr.line_off;
@@ -715,20 +261,12 @@ __global__ void __launch_bounds__(kTopoThreads, 1) topo_kernel(TopoParams p, Top
       fc.half[k] = fr.half[k];
       fc.hf[k] = static_cast<float>(fr.half[k]);
     }
-    const size_t elem = (PREC == kFP32C) ? 16 : 32;
-    const ulonglong2* gA = reinterpret_cast<const ulonglong2*>(
-        static_cast<const char*>(p.packed) + fr.packed_off * elem);
-    const ulonglong2* gB = gA + fr.n_pad / 2;
-    const ulonglong2* gC = DIP ? gA + fr.n_pad : nullptr;
-    if constexpr (RES == kResAny) {
-      const ulonglong2* sC = DIP ? sm_ch + res : nullptr;
-      run_frame<PREC, S, DIP, RES>(p, fc, queue, gA, gB, gC, sm_ch, sm_ch + res / 2, sC, false,
-                                   res / 2, fr.n_pad, my_rec, lane);
-    } else {
-      const ulonglong2* sC = DIP ? sm_ch + fr.n_pad : nullptr;
-      run_frame<PREC, S, DIP, RES>(p, fc, queue, gA, gB, gC, sm_ch, sm_ch + fr.n_pad / 2, sC, resident,
-                                   0, fr.n_pad, my_rec, lane);
-    }
+    HandOver hand;
+    hand.rec = p.left + fr.left_off;
+    hand.count = p.left_count + f;
+    hand.cap = p.left ? fr.left_cap : 0;
+    run_frame<PREC, S, DIP, SRC>(p, fc, queue, reinterpret_cast<const ulonglong2*>(src), sm_off, fr.resident / 2,
+                            fr.n_pad, my_rec, lane, hand, &s_idle);
   }
 }
 
@@ -946,7 +484,6 @@ __global__ void __launch_bounds__(kEngineThreads, 2) engine_kernel(EngineParams 
       const int n_pad = L.n_pad;
       const ulonglong2* gA = reinterpret_cast<const ulonglong2*>(
           static_cast<const char*>(E.p.packed) + L.off * static_cast<long long>(elem));
-      const ulonglong2* gB = gA + n_pad / 2;
       int src_of[S];
       int my_rank = -1;
       {
@@ -959,34 +496,9 @@ __global__ void __launch_bounds__(kEngineThreads, 2) engine_kernel(EngineParams 
         }
       }
       if constexpr (PREC == kFP32C) {
-        uint64_t ex2[S][3];
-#pragma unroll
-        for (int e = 0; e < S; ++e)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            const float v = __shfl_sync(0xffffffffu, sl.posf[c], src_of[e]);
-            ex2[e][c] = pk2(v, v);
-          }
-        float total;
-        const int n_pairs = n_pad / 2;
-        switch (na) {
-          case 1: sweep_f32x2<1, S>(nullptr, nullptr, nullptr, 0, gA, gB, nullptr, n_pairs, lane, ex2, total); break;
-          case 2: sweep_f32x2<2, S>(nullptr, nullptr, nullptr, 0, gA, gB, nullptr, n_pairs, lane, ex2, total); break;
-          case 3: sweep_f32x2<(S > 2 ? 3 : 2), S>(nullptr, nullptr, nullptr, 0, gA, gB, nullptr, n_pairs, lane, ex2, total); break;
-          default: sweep_f32x2<S, S>(nullptr, nullptr, nullptr, 0, gA, gB, nullptr, n_pairs, lane, ex2, total); break;
-        }
         float Ef[3];
-        const int rk = my_rank >= 0 ? my_rank : 0;
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-          Ef[c] = __shfl_sync(0xffffffffu, total, (3 * rk + c) << (S == 4 ? 1 : 2));
-        if (my_rank >= 0) {
-          const float n2 =
-              __fmaf_rn(Ef[0], Ef[0], __fmaf_rn(Ef[1], Ef[1], __fmul_rn(Ef[2], Ef[2])));
-          const float st = __fdiv_rn(static_cast<float>(my.step), __fsqrt_rn(n2));
-#pragma unroll
-          for (int c = 0; c < 3; ++c) nx[c] = sl.pos[c] + static_cast<double>(__fmul_rn(Ef[c], st));
-        }
+        sweep_slots<S, false, kSrcGlobal>(na, sl.posf, src_of, max(my_rank, 0), 0, 0, gA, n_pad / 2, Ef);
+        if (my_rank >= 0) euler_step(Ef, sl.pos, my.step, nx);
       } else {
         double ex[S][3];
 #pragma unroll
@@ -1008,9 +520,7 @@ __global__ void __launch_bounds__(kEngineThreads, 2) engine_kernel(EngineParams 
             if (e == my_rank)
 #pragma unroll
               for (int c = 0; c < 3; ++c) Ev[c] = Es[e][c];
-          const double n = sqrt(Ev[0] * Ev[0] + Ev[1] * Ev[1] + Ev[2] * Ev[2]);
-#pragma unroll
-          for (int c = 0; c < 3; ++c) nx[c] = sl.pos[c] + my.step * Ev[c] / n;
+          euler_step(Ev, sl.pos, my.step, nx);
         }
       }
     }
@@ -1108,22 +618,16 @@ size_t topo_smem_bytes(int S, int max_resident_pad, bool dip = false) {
          static_cast<size_t>(max_resident_pad) * (dip ? 24 : 16);
 }
 
-template <int PREC, int RES, int S, bool DIP>
+template <int PREC, int S, bool DIP, int SRC>
 cudaError_t launch_topo_t(const TopoParams& p, const TopoFrame& f0, int total_lines, int num_sms,
                           cudaStream_t s) {
-  const size_t smem = topo_smem_bytes(S, RES != kResNone ? p.max_resident_pad : 0, DIP);
-  cudaError_t err = cudaFuncSetAttribute(topo_kernel<PREC, RES, S, DIP>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
+  const size_t smem = topo_smem_bytes(S, PREC == kFP32C ? p.max_resident_pad : 0, DIP);
+  const cudaError_t err = cudaFuncSetAttribute(
+      topo_kernel<PREC, S, DIP, SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (err != cudaSuccess) return err;
-  int per_sm = 1;
-  err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, topo_kernel<PREC, RES, S, DIP>,
-                                                      kTopoThreads, smem);
-  if (err != cudaSuccess) return err;
-  per_sm = std::max(per_sm, 1);
-  const int max_useful = (total_lines + kTopoWarps * S - 1) / (kTopoWarps * S);
-  const int grid = std::max(1, std::min(num_sms * per_sm, max_useful));
-  topo_kernel<PREC, RES, S, DIP><<<grid, kTopoThreads, smem, s>>>(p, f0);
+  // one CTA per SM: its 512 threads take more than half of an SM's registers
+  const int grid = std::max(1, std::min(num_sms, total_lines));
+  topo_kernel<PREC, S, DIP, SRC><<<grid, kTopoThreads, smem, s>>>(p, f0);
   return cudaGetLastError();
 }
 
@@ -1262,21 +766,19 @@ cudaError_t launch_pack_topo_frames(int prec, int n_frames, const TopoFrame* d_f
   return cudaGetLastError();
 }
 
-template <int PREC, int RES, bool DIP = false>
-cudaError_t launch_topo_s(const TopoParams& p, const TopoFrame& f0, int total_lines, int num_sms,
-                          cudaStream_t s, int slots) {
-  return slots == 2 ? launch_topo_t<PREC, RES, 2, DIP>(p, f0, total_lines, num_sms, s)
-                    : launch_topo_t<PREC, RES, 4, DIP>(p, f0, total_lines, num_sms, s);
+template <int PREC, bool DIP, int SRC>
+cudaError_t launch_topo_s(const TopoParams& p, const TopoFrame& f0, int num_sms, cudaStream_t s, int slots) {
+  return slots == 2 ? launch_topo_t<PREC, 2, DIP, SRC>(p, f0, p.n_lines, num_sms, s)
+                    : launch_topo_t<PREC, 4, DIP, SRC>(p, f0, p.n_lines, num_sms, s);
 }
 
-// FP32C launch by residency mode; FP64 frames are never resident.
+// whole: every frame of the launch fits shared memory.
 template <bool DIP>
-cudaError_t launch_topo_mode(int prec, int mode, const TopoParams& p, const TopoFrame& f0,
-                             int num_sms, cudaStream_t s, int slots) {
-  if (prec == kFP64) return launch_topo_s<kFP64, kResNone, DIP>(p, f0, p.n_lines, num_sms, s, slots);
-  if (mode == kResWhole) return launch_topo_s<kFP32C, kResWhole, DIP>(p, f0, p.n_lines, num_sms, s, slots);
-  if (mode == kResAny) return launch_topo_s<kFP32C, kResAny, DIP>(p, f0, p.n_lines, num_sms, s, slots);
-  return launch_topo_s<kFP32C, kResNone, DIP>(p, f0, p.n_lines, num_sms, s, slots);
+cudaError_t launch_topo_prec(int prec, bool whole, const TopoParams& p, const TopoFrame& f0, int num_sms,
+                             cudaStream_t s, int slots) {
+  if (prec == kFP64) return launch_topo_s<kFP64, DIP, kSrcSplit>(p, f0, num_sms, s, slots);
+  return whole ? launch_topo_s<kFP32C, DIP, kSrcShared>(p, f0, num_sms, s, slots)
+               : launch_topo_s<kFP32C, DIP, kSrcSplit>(p, f0, num_sms, s, slots);
 }
 
 // Single frame: p.packed holds round_up(n_charges, topo_charge_pad(prec)) charges
@@ -1291,25 +793,40 @@ cudaError_t launch_topo(int prec, const TopoParams& p_in, int num_sms, cudaStrea
   f0.n_pad = ((std::max(p.n_charges, 1) + pad - 1) / pad) * pad;
   f0.n_lines = p.n_lines;
   f0.resident = topo_resident_count(prec, p.source, f0.n_pad);
-  f0.pad_ = 0;
+  f0.team_resident = topo_team_resident(prec, p.source, f0.n_pad);
+  f0.left_off = 0;
+  f0.left_cap = p.left ? topo_left_capacity(num_sms, p.n_lines) : 0;
   f0.step = p.step;
   for (int k = 0; k < 3; ++k) f0.half[k] = p.half[k];
   p.frames = nullptr;
   p.n_frames = 1;
   p.max_resident_pad = f0.resident;
-  const int slots = tuned_topo_slots(prec, f0.resident == f0.n_pad, p.n_lines);
-  const int mode = f0.resident == 0 ? kResNone : (f0.resident == f0.n_pad ? kResWhole : kResAny);
-  if (p.source == kDipoles) return launch_topo_mode<true>(prec, mode, p, f0, num_sms, s, slots);
-  return launch_topo_mode<false>(prec, mode, p, f0, num_sms, s, slots);
+  p.max_team_resident = f0.team_resident;
+  if (p.n_lines <= int64_t(num_sms) * kTeamLinesPerSm)
+    return launch_topo_team(prec, p, f0, 1, num_sms, s);
+  const bool whole = f0.resident == f0.n_pad;
+  const int slots = tuned_topo_slots(prec, whole, p.n_lines);
+  const cudaError_t e = p.source == kDipoles
+                            ? launch_topo_prec<true>(prec, whole, p, f0, num_sms, s, slots)
+                            : launch_topo_prec<false>(prec, whole, p, f0, num_sms, s, slots);
+  if (e != cudaSuccess || f0.left_cap == 0) return e;
+  return launch_topo_team(prec, p, f0, 0, num_sms, s);
+}
+
+int topo_left_capacity(int num_sms, int64_t n_lines) {
+  // what the CTAs of one launch may hold when they hand over
+  return static_cast<int>(std::min(n_lines, int64_t(num_sms) * kTeamLinesPerSm));
 }
 
 cudaError_t launch_topo_frames(int prec, const TopoParams& p, int num_sms, cudaStream_t s) {
   if (p.n_frames <= 0 || p.n_lines <= 0) return cudaSuccess;
   TopoFrame dummy{};
+  if (p.sum_lines <= int64_t(num_sms) * kTeamLinesPerSm)
+    return launch_topo_team(prec, p, dummy, 1, num_sms, s);
   const int slots = tuned_topo_slots(prec, p.all_resident != 0, p.n_lines);
-  // kResWhole when no frame is partly resident (all_resident: every frame whole)
-  const int mode = p.max_resident_pad <= 0 ? kResNone : (p.all_resident ? kResWhole : kResAny);
-  return launch_topo_mode<false>(prec, mode, p, dummy, num_sms, s, slots);
+  const cudaError_t e = launch_topo_prec<false>(prec, p.all_resident != 0, p, dummy, num_sms, s, slots);
+  if (e != cudaSuccess || !p.left) return e;
+  return launch_topo_team(prec, p, dummy, 0, num_sms, s);
 }
 
 }  // namespace cpetgb
