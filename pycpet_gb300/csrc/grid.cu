@@ -68,8 +68,11 @@ struct GridCfg<kFP64> {
   static constexpr int kTile = 256;  // charges per stage (8 KiB)
 };
 
-__device__ __forceinline__ double rsqrt_f64(double x) { return rsqrt(x); }
-__device__ __forceinline__ double charge_q(const Charge64& c) { return c.q; }
+// FP64: q r^-3 (field) or q r^-1 (potential).
+template <int KIND>
+__device__ __forceinline__ double weight_f64(const Charge64& c, double r2) {
+  return KIND == kField ? weight_r3_f64(c.q, r2) : weight_r1_f64(c.q, r2);
+}
 // {v, v} as one packed 64-bit value.
 __device__ __forceinline__ uint64_t dup2(float v) {
   const uint64_t b = __float_as_uint(v);
@@ -340,14 +343,13 @@ __global__ void __launch_bounds__(kGridThreads, PREC == kFP32C && PPT == 4 ? 6 :
           const Real dz = pz[k] - ch.z;
           Real r2 = dx * dx + dy * dy + dz * dz;
           if (CLAMP && clamp_tile) r2 = fmax(r2, Real(1e-6));  // compute_looped_field's fmaxf
-          const Real ri = rsqrt_f64(r2);
           if constexpr (KIND == kField) {
-            const Real w = (charge_q(ch) * ri) * (ri * ri);
+            const Real w = weight_f64<KIND>(ch, r2);
             part[0][k] += w * dx;
             part[1][k] += w * dy;
             part[2][k] += w * dz;
           } else {
-            part[0][k] += charge_q(ch) * ri;
+            part[0][k] += weight_f64<KIND>(ch, r2);
           }
         }
       }

@@ -480,10 +480,10 @@ __device__ __forceinline__ void sweep_slots(int na, const float (&posf)[3], cons
   for (int c = 0; c < 3; ++c) E[c] = __shfl_sync(0xffffffffu, total, (3 * rk + c) << shift);
 }
 
-// FP64: every operation in double precision; r^-1 from the double rsqrt
-// (1 ulp), whose few FP64-pipe operations replace a correctly rounded sqrt and
-// division (GB300's FP64 pipe is 1/64 of its FP32 pipe).  A run is kLaneRun64
-// charges per lane, summed plainly; the runs are added in order.
+// FP64.  Bound: the FP64 pipe (64 cycles per warp instruction); a charge pair
+// takes 13 of its instructions (3 differences, 3 for r^2, 4 for q r^-3 with
+// common.cuh's seed, 3 sums) where rsqrt() and three products took 19.  A run
+// is kLaneRun64 charges per lane, summed plainly; the runs are added in order.
 template <int NA, int S>
 __device__ __forceinline__ void run_f64(const Charge64* __restrict__ g, int base, int cnt,
                                         const double (&ex)[S][3], double (&part)[NA][3]) {
@@ -496,8 +496,7 @@ __device__ __forceinline__ void run_f64(const Charge64* __restrict__ g, int base
       const double dy = __dsub_rn(ex[e][1], ch.y);
       const double dz = __dsub_rn(ex[e][2], ch.z);
       const double r2 = __fma_rn(dx, dx, __fma_rn(dy, dy, __dmul_rn(dz, dz)));
-      const double ri = rsqrt(r2);  // double-precision reciprocal square root (1 ulp)
-      const double w = __dmul_rn(ch.q, __dmul_rn(ri, __dmul_rn(ri, ri)));
+      const double w = weight_r3_f64(ch.q, r2);
       part[e][0] = __fma_rn(w, dx, part[e][0]);
       part[e][1] = __fma_rn(w, dy, part[e][1]);
       part[e][2] = __fma_rn(w, dz, part[e][2]);
@@ -505,8 +504,8 @@ __device__ __forceinline__ void run_f64(const Charge64* __restrict__ g, int base
   }
 }
 
-// FP64 dipoles: same term as dipole_run, in double precision (r^-1 from the
-// double rsqrt, as run_f64).
+// FP64 dipoles: the term of dipole_terms, r^-5 dot R - r^-3 mu (22 FP64-pipe
+// instructions, 29 with rsqrt()).
 template <int NA, int S>
 __device__ __forceinline__ void run_f64(const Dipole64* __restrict__ g, int base, int cnt,
                                         const double (&ex)[S][3], double (&part)[NA][3]) {
@@ -519,13 +518,13 @@ __device__ __forceinline__ void run_f64(const Dipole64* __restrict__ g, int base
       const double dy = __dsub_rn(ex[e][1], d.y);
       const double dz = __dsub_rn(ex[e][2], d.z);
       const double r2 = __fma_rn(dx, dx, __fma_rn(dy, dy, __dmul_rn(dz, dz)));
-      const double ri = rsqrt(r2);  // double-precision reciprocal square root (1 ulp)
-      const double ri2 = __dmul_rn(ri, ri);
-      const double r5 = __dmul_rn(__dmul_rn(ri2, ri2), ri);
+      double r3, r5;
+      inv_r3_r5_f64(r2, r3, r5);
       const double dot = __fma_rn(3.0 * d.mx, dx, __fma_rn(d.my, dy, __dmul_rn(d.mz, dz)));
-      part[e][0] = __fma_rn(r5, __fma_rn(dot, dx, -__dmul_rn(d.mx, r2)), part[e][0]);
-      part[e][1] = __fma_rn(r5, __fma_rn(dot, dy, -__dmul_rn(d.my, r2)), part[e][1]);
-      part[e][2] = __fma_rn(r5, __fma_rn(dot, dz, -__dmul_rn(d.mz, r2)), part[e][2]);
+      const double w = __dmul_rn(r5, dot);
+      part[e][0] = __fma_rn(w, dx, __fma_rn(-r3, d.mx, part[e][0]));
+      part[e][1] = __fma_rn(w, dy, __fma_rn(-r3, d.my, part[e][1]));
+      part[e][2] = __fma_rn(w, dz, __fma_rn(-r3, d.mz, part[e][2]));
     }
   }
 }
