@@ -156,15 +156,6 @@ size_t packed_size(int prec) { return prec == CPETGB_FP32C ? 16 : 32; }  // stre
 constexpr size_t kGridRecord = 32;  // grid layouts: Charge64 or the duplicated FP32C record
 
 // ---------------------------------------------------------------------------
-// Grid work decomposition.
-// ---------------------------------------------------------------------------
-struct GridPlan {
-  std::vector<GridItem> items;
-  std::vector<GridFinal> finals;
-  int n_slots = 0;
-};
-
-// ---------------------------------------------------------------------------
 // Autotuner table: (operation, precision, class, size bucket) -> variant.
 // Filled by pycpet_gb300.autotune (timed candidates), read at every launch.
 // ---------------------------------------------------------------------------
@@ -212,55 +203,85 @@ int tune_choose(int key) {
   return -1;
 }
 
-void plan_grid(int n_frames, const int64_t* desc, int sms, GridPlan& plan, int ppt,
-               int items_per_sm) {
-  const int tile = kGridThreads * ppt;
-  // A CTA's time is proportional to its charge count alone: every thread
-  // evaluates all of its point slots, valid or not.  Each frame's points are
-  // cut into equal tiles, and charge ranges are split so that about
-  // items_per_sm items of equal cost fall on each SM.
-  auto n_tiles = [&](int64_t P) { return (P + tile - 1) / tile; };
+double grid_pair_evals(int n_frames, const int64_t* desc) {
+  double total = 0.0;
+  for (int f = 0; f < n_frames; ++f) total += double(desc[4 * f + 1]) * double(desc[4 * f + 3]);
+  return total;
+}
+
+// ---------------------------------------------------------------------------
+// Grid work decomposition: the frame table of a launch (kernels.cuh).
+// ---------------------------------------------------------------------------
+struct GridTable {
+  std::vector<GridFrame> frames;
+  int64_t n_items = 0, n_tiles = 0, n_prep = 0, few_items = 0, n_slots = 0;
+  int n_few = 0;
+};
+
+int plan_grid(int prec, int n_frames, const int64_t* desc, int sms, int ppt, int items_per_sm, GridTable& t) {
+  const int64_t tile = int64_t(kGridThreads) * ppt;
+  // A CTA's time is proportional to its charge count: each frame's charges are
+  // split so that about items_per_sm items of equal cost fall on each SM.  The
+  // chunks decide how the sums are grouped, so they depend on the frame sizes
+  // alone.
+  auto full_tiles = [&](int64_t P) { return (P + tile - 1) / tile; };
   double total = 0.0;
   for (int f = 0; f < n_frames; ++f)
-    total += double(n_tiles(desc[4 * f + 3])) * tile * double(desc[4 * f + 1]);
+    total += double(full_tiles(desc[4 * f + 3])) * double(tile) * double(desc[4 * f + 1]);
   const double target = std::max(1.0, total / (double(std::max(sms, 1)) * items_per_sm));
+  const bool mesh =
+      grid_pair_evals(n_frames, desc) >= (prec == CPETGB_FP64 ? kGridMeshPairsFp64 : kGridMeshPairsFp32);
+  t.frames.resize(size_t(n_frames));
   for (int f = 0; f < n_frames; ++f) {
-    const int64_t co = desc[4 * f + 0], n = desc[4 * f + 1];
-    const int64_t po = desc[4 * f + 2], P = desc[4 * f + 3];
-    const int64_t nt = n_tiles(P);
-    for (int64_t ti = 0; ti < nt; ++ti) {
-      const int64_t pb = ti * (P / nt) + std::min<int64_t>(ti, P % nt);
-      const int pc = static_cast<int>(P / nt + (ti < P % nt ? 1 : 0));
-      int64_t split = 1;
-      if (n > 0) {
-        split = static_cast<int64_t>(std::ceil(double(tile) * double(n) / target));
-        split = std::max<int64_t>(1, std::min<int64_t>(split, std::max<int64_t>(1, n / 256)));
-      }
-      const int64_t chunk = n > 0 ? (n + split - 1) / split : 0;
-      if (n > 0) split = (n + chunk - 1) / chunk;
-      int slot_base = -1;
-      if (split > 1) {
-        slot_base = plan.n_slots;
-        plan.n_slots += static_cast<int>(split);
-        plan.finals.push_back(GridFinal{po + pb, pc, slot_base, static_cast<int32_t>(split), 0});
-      }
-      for (int64_t k = 0; k < split; ++k) {
-        GridItem it;
-        it.charge_off = co;
-        it.point_off = po;
-        it.p_begin = static_cast<int32_t>(pb);
-        it.p_count = pc;
-        it.n_begin = static_cast<int32_t>(k * chunk);
-        it.n_count = static_cast<int32_t>(std::min<int64_t>(chunk, n - k * chunk));
-        it.slot = split > 1 ? slot_base + static_cast<int32_t>(k) : -1;
-        it.pad = 0;
-        plan.items.push_back(it);
-      }
+    const int64_t n = desc[4 * f + 1], P = desc[4 * f + 3];
+    GridFrame& fr = t.frames[f];
+    fr = GridFrame{};
+    fr.charge_off = desc[4 * f];
+    fr.point_off = desc[4 * f + 2];
+    fr.n_charges = static_cast<int32_t>(n);
+    fr.n_points = static_cast<int32_t>(P);
+    fr.few = P > 0 && P <= (prec == CPETGB_FP64 ? kGridFewPoints : kGridFewPointsFp32);
+    int64_t split = 1;
+    if (n > 0) {
+      split = static_cast<int64_t>(std::ceil(double(tile) * double(n) / target));
+      // FP32C: at least 256 charges each.  FP64 is so much slower that an uneven
+      // number of items per SM costs more than short chunks: 9,261 points x 5,000
+      // charges, 361 items of 264 charges 1,390 us, 1,216 of 79 1,160.
+      const int64_t least = prec == CPETGB_FP64 && !fr.few ? 32 : 256;
+      split = std::max<int64_t>(1, std::min<int64_t>(split, std::max<int64_t>(1, n / least)));
     }
+    const int64_t chunk = n > 0 ? (n + split - 1) / split : 0;
+    if (n > 0) split = (n + chunk - 1) / chunk;
+    fr.chunk = static_cast<int32_t>(chunk);
+    fr.n_split = static_cast<int32_t>(split);
+    // mesh columns and the other points are rounded up to warps separately
+    const int64_t threads = (P + ppt - 1) / ppt + 64;
+    fr.n_tiles = P == 0 ? 0 : (fr.few ? 1 : static_cast<int32_t>((threads + kGridThreads - 1) / kGridThreads));
   }
-  // longest first, so the last wave holds the shortest items
-  std::stable_sort(plan.items.begin(), plan.items.end(),
-                   [](const GridItem& a, const GridItem& b) { return a.n_count > b.n_count; });
+  // few-points frames first; the others longest chunk first, so the last wave
+  // holds the shortest items
+  std::stable_sort(t.frames.begin(), t.frames.end(), [](const GridFrame& a, const GridFrame& b) {
+    return a.few != b.few ? a.few > b.few : a.chunk > b.chunk;
+  });
+  for (GridFrame& fr : t.frames) {
+    const int64_t items = int64_t(fr.n_tiles) * fr.n_split;
+    fr.item_base = static_cast<int32_t>(t.n_items);
+    fr.tile_base = static_cast<int32_t>(t.n_tiles);
+    fr.prep_base = static_cast<int32_t>(t.n_prep);
+    fr.slot_base = fr.n_split > 1 ? static_cast<int32_t>(t.n_slots) : -1;
+    t.n_items += items;
+    t.n_tiles += fr.n_tiles;
+    if (fr.n_split > 1) t.n_slots += items;
+    if (fr.few) {
+      ++t.n_few;
+      t.few_items += items;
+    } else if (mesh) {
+      t.n_prep += (int64_t(fr.n_points) + kGridPrepPoints - 1) / kGridPrepPoints;
+    }
+    if (t.n_items > INT_MAX || t.n_tiles * ppt > INT_MAX)
+      return fail(CPETGB_EINVAL, "launch too large (%lld work items)", (long long)t.n_items);
+  }
+  return CPETGB_OK;
 }
 
 // Entries the refinement list may need: every point of every frame (frames
@@ -277,10 +298,32 @@ int64_t max_frame_points(int n_frames, const int64_t* desc) {
   return m;
 }
 
-double grid_pair_evals(int n_frames, const int64_t* desc) {
-  double total = 0.0;
-  for (int f = 0; f < n_frames; ++f) total += double(desc[4 * f + 1]) * double(desc[4 * f + 3]);
-  return total;
+// Everything of a launch that does not depend on its buffers.
+GridLaunch grid_launch(int kind, int prec, int clamp, int ppt, int n_frames, const int64_t* desc,
+                       const GridTable& t, int64_t tot_ch, const Ctx* c) {
+  GridLaunch g{};
+  g.kind = kind;
+  g.prec = prec;
+  g.clamp = clamp ? 1 : 0;
+  g.ppt = ppt;
+  g.n_frames = n_frames;
+  if (n_frames == 1) g.one = t.frames[0];
+  g.n_items = static_cast<int>(t.n_items);
+  g.n_tiles = static_cast<int>(t.n_tiles);
+  g.n_prep = static_cast<int>(t.n_prep);
+  g.n_few = t.n_few;
+  g.few_items = static_cast<int>(t.few_items);
+  g.n_charges = tot_ch;
+  g.max_points = static_cast<int>(max_frame_points(n_frames, desc));
+  g.status = c->status;
+  g.num_sms = c->sms;
+  // A frame of one or two points never has a point below tau x its lower
+  // median, so launches of such frames only (point fields) skip the pass.
+  const double tau = g_refine_tau.load();
+  const bool refine =
+      kind == CPETGB_FIELD && prec == CPETGB_FP32C && tau > 0.0 && tot_ch > 0 && g.max_points >= 3;
+  g.tau = refine ? tau : 0.0;
+  return g;
 }
 
 int grid_batch_impl(int kind, int prec, int mem, int clamp, int n_frames, const int64_t* desc,
@@ -308,10 +351,11 @@ int grid_batch_impl(int kind, int prec, int mem, int clamp, int n_frames, const 
   if (mem == CPETGB_HOST && !s) s = c->stream;
   const int NC = kind == CPETGB_FIELD ? 3 : 1;
 
-  GridPlan plan;
+  GridTable plan;
   int ppt = 4, ips = 8;
   tuned_grid_shape(prec, kind, grid_pair_evals(n_frames, desc), &ppt, &ips);
-  plan_grid(n_frames, desc, c->sms, plan, ppt, ips);
+  rc = plan_grid(prec, n_frames, desc, c->sms, ppt, ips, plan);
+  if (rc != CPETGB_OK) return rc;
 
   Scratch S(s);
   const double *dp = pts, *dx = x, *dq = q;
@@ -324,41 +368,32 @@ int grid_batch_impl(int kind, int prec, int mem, int clamp, int n_frames, const 
     }
     CK(S.get(&dout, size_t(tot_pts) * NC), "alloc output");
   }
-  unsigned char* packed = nullptr;
-  GridItem* d_items = nullptr;
-  GridFinal* d_fin = nullptr;
-  double* partial = nullptr;
-  CK(S.get(&packed, size_t(std::max<int64_t>(tot_ch, 1)) * kGridRecord), "alloc packed charges");
-  CK(h2d(&d_items, S, plan.items.data(), plan.items.size()), "copy work items");
-  if (!plan.finals.empty()) {
-    CK(h2d(&d_fin, S, plan.finals.data(), plan.finals.size()), "copy split table");
-    CK(S.get(&partial, size_t(plan.n_slots) * kGridSlotPts * 3), "alloc partial sums");
-  }
-  if (reinterpret_cast<uintptr_t>(packed) % 16 != 0)  // bulk async copies need 16-byte sources
-    return fail(CPETGB_ECUDA, "scratch allocation is not 16-byte aligned");
-  CK(launch_pack_charges(prec, tot_ch, tot_ch, dx, dq, packed, s), "pack charges");
-  CK(launch_grid(prec, kind, clamp ? 1 : 0, ppt, static_cast<int>(plan.items.size()), d_items,
-                 packed, dp, dout, partial, c->status, s),
-     "grid kernel launch");
-  CK(launch_grid_final(kind, static_cast<int>(plan.finals.size()), d_fin, partial, dout, s),
-     "grid reduction launch");
-  const double tau = g_refine_tau.load();
-  // A frame of one or two points never has a point below tau x its lower
-  // median, so launches of such frames only (point fields) skip the pass.
-  if (kind == CPETGB_FIELD && prec == CPETGB_FP32C && tau > 0.0 && tot_ch > 0 &&
-      max_frame_points(n_frames, desc) >= 3) {
-    int64_t *d_desc = nullptr, *list = nullptr;
-    int* count = nullptr;
-    unsigned char* dfq = nullptr;
-    int* hist = nullptr;
-    CK(h2d(&d_desc, S, desc, size_t(n_frames) * 4), "copy frame table");
-    CK(S.get(&list, size_t(refine_list_len(n_frames, desc)) * 2), "alloc refinement list");
-    CK(S.get(&count, 1), "alloc refinement count");
-    CK(S.get(&hist, size_t(grid_refine_hist_ints(n_frames))), "alloc magnitude histograms");
-    CK(S.get(&dfq, size_t(tot_ch) * 32), "alloc double-float charges");
-    CK(launch_grid_refine(n_frames, tot_ch, max_frame_points(n_frames, desc), d_desc, dp, dx, dq, dout,
-                          clamp ? 1 : 0, tau, list, count, hist, dfq, c->sms, s),
-       "field refinement launch");
+  GridLaunch g = grid_launch(kind, prec, clamp, ppt, n_frames, desc, plan, tot_ch, c);
+  g.points = dp;
+  g.x = dx;
+  g.q = dq;
+  g.out = dout;
+  if (grid_point_fits(g)) {
+    CK(launch_grid_point(g, s), "point kernel launch");
+  } else {
+    GridFrame* d_frames = nullptr;
+    unsigned char* packed = nullptr;
+    CK(S.get(&packed, size_t(std::max<int64_t>(tot_ch, 1)) * kGridRecord), "alloc packed charges");
+    if (reinterpret_cast<uintptr_t>(packed) % 16 != 0)  // bulk async copies need 16-byte sources
+      return fail(CPETGB_ECUDA, "scratch allocation is not 16-byte aligned");
+    g.packed = packed;
+    CK(h2d(&d_frames, S, plan.frames.data(), plan.frames.size()), "copy frame table");
+    g.frames = d_frames;
+    CK(S.get(&g.zeroed, grid_zero_ints(n_frames, g.tau > 0.0)), "alloc counters");
+    if (plan.n_slots)
+      CK(S.get(&g.partial, size_t(plan.n_slots) * grid_slot_doubles(kind, ppt)), "alloc partial sums");
+    if (g.tau > 0.0) {
+      unsigned char* dfq = nullptr;
+      CK(S.get(&g.list, size_t(refine_list_len(n_frames, desc)) * 2), "alloc refinement list");
+      CK(S.get(&dfq, size_t(tot_ch) * 32), "alloc double-float charges");
+      g.dfq = dfq;
+    }
+    CK(launch_grid(g, s), "grid launch");
   }
   if (mem == CPETGB_HOST) {
     CK(cudaMemcpyAsync(out, dout, size_t(tot_pts) * NC * sizeof(double), cudaMemcpyDeviceToHost, s),
@@ -919,68 +954,49 @@ int grid_plan_impl(cpetgb_plan** out_plan, int kind, int prec, int clamp, int n_
   int rc;
   Ctx* c = context(&rc);
   if (!c) return rc;
-  GridPlan gp;
+  GridTable gp;
   int ppt = 4, ips = 8;
   tuned_grid_shape(prec, kind, grid_pair_evals(n_frames, desc), &ppt, &ips);
-  plan_grid(n_frames, desc, c->sms, gp, ppt, ips);
+  rc = plan_grid(prec, n_frames, desc, c->sms, ppt, ips, gp);
+  if (rc != CPETGB_OK) return rc;
+  GridLaunch g = grid_launch(kind, prec, clamp, ppt, n_frames, desc, gp, tot_ch, c);
+  g.points = pts;
+  g.x = x;
+  g.q = q;
+  g.out = out;
   cpetgb_plan* pl = new cpetgb_plan();
   cudaGetDevice(&pl->device);
-  unsigned char* packed = nullptr;
-  GridItem* d_items = nullptr;
-  GridFinal* d_fin = nullptr;
-  double* partial = nullptr;
+  const bool point = grid_point_fits(g);
+  unsigned char *packed = nullptr, *dfq = nullptr;
+  GridFrame* d_frames = nullptr;
   cudaError_t e = plan_alloc(pl->bufs, &packed, size_t(std::max<int64_t>(tot_ch, 1)) * kGridRecord);
-  if (e == cudaSuccess) e = plan_alloc(pl->bufs, &d_items, gp.items.size());
-  if (e == cudaSuccess && !gp.items.empty())
-    e = cudaMemcpy(d_items, gp.items.data(), gp.items.size() * sizeof(GridItem), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && !gp.finals.empty()) {
-    e = plan_alloc(pl->bufs, &d_fin, gp.finals.size());
-    if (e == cudaSuccess)
-      e = cudaMemcpy(d_fin, gp.finals.data(), gp.finals.size() * sizeof(GridFinal),
-                     cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = plan_alloc(pl->bufs, &partial, size_t(gp.n_slots) * kGridSlotPts * 3);
+  if (e == cudaSuccess) e = plan_alloc(pl->bufs, &d_frames, gp.frames.size());
+  if (e == cudaSuccess && !gp.frames.empty())
+    e = cudaMemcpy(d_frames, gp.frames.data(), gp.frames.size() * sizeof(GridFrame), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = plan_alloc(pl->bufs, &g.zeroed, grid_zero_ints(n_frames, g.tau > 0.0));
+  if (e == cudaSuccess && gp.n_slots)
+    e = plan_alloc(pl->bufs, &g.partial, size_t(gp.n_slots) * grid_slot_doubles(kind, ppt));
+  if (e == cudaSuccess && g.tau > 0.0) {
+    e = plan_alloc(pl->bufs, &dfq, size_t(tot_ch) * 32);
+    if (e == cudaSuccess) e = plan_alloc(pl->bufs, &g.list, size_t(refine_list_len(n_frames, desc)) * 2);
   }
   if (e != cudaSuccess) {
     delete pl;
     return cuda_fail(e, "plan allocation");
   }
-  const double tau = g_refine_tau.load();
-  const bool refine = kind == CPETGB_FIELD && prec == CPETGB_FP32C && tau > 0.0 && tot_ch > 0 &&
-                      max_frame_points(n_frames, desc) >= 3;
-  int64_t *d_desc = nullptr, *list = nullptr;
-  int* count = nullptr;
-  unsigned char* dfq = nullptr;
-  int* hist = nullptr;
-  if (refine) {
-    e = plan_alloc(pl->bufs, &d_desc, size_t(n_frames) * 4);
-    if (e == cudaSuccess) e = plan_alloc(pl->bufs, &hist, size_t(grid_refine_hist_ints(n_frames)));
-    if (e == cudaSuccess) e = plan_alloc(pl->bufs, &dfq, size_t(tot_ch) * 32);
-    if (e == cudaSuccess)
-      e = cudaMemcpy(d_desc, desc, size_t(n_frames) * 4 * sizeof(int64_t), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = plan_alloc(pl->bufs, &list, size_t(refine_list_len(n_frames, desc)) * 2);
-    if (e == cudaSuccess) e = plan_alloc(pl->bufs, &count, 1);
-    if (e == cudaSuccess) e = preload_grid_refine();
-    if (e != cudaSuccess) {
-      delete pl;
-      return cuda_fail(e, "plan allocation");
-    }
-  }
-  const int n_items = static_cast<int>(gp.items.size()), n_fin = static_cast<int>(gp.finals.size());
+  g.packed = packed;
+  g.frames = d_frames;
+  g.dfq = dfq;
   e = preload_grid_kernels(prec, kind, clamp ? 1 : 0, ppt);
   if (e != cudaSuccess) {
     delete pl;
     return cuda_fail(e, "kernel load");
   }
   rc = capture_plan(pl, [&](cudaStream_t cs) -> int {
-    CK(launch_pack_charges(prec, tot_ch, tot_ch, x, q, packed, cs), "pack charges");
-    CK(launch_grid(prec, kind, clamp ? 1 : 0, ppt, n_items, d_items, packed, pts, out, partial,
-                   c->status, cs),
-       "grid kernel launch");
-    CK(launch_grid_final(kind, n_fin, d_fin, partial, out, cs), "grid reduction launch");
-    if (refine)
-      CK(launch_grid_refine(n_frames, tot_ch, max_frame_points(n_frames, desc), d_desc, pts, x, q, out,
-                            clamp ? 1 : 0, tau, list, count, hist, dfq, c->sms, cs),
-         "field refinement launch");
+    if (point)
+      CK(launch_grid_point(g, cs), "point kernel launch");
+    else
+      CK(launch_grid(g, cs), "grid launch");
     return CPETGB_OK;
   });
   if (rc != CPETGB_OK) {

@@ -5,12 +5,21 @@
 // a point) and calc_esp_base (math_module.c:453-486, potential), which the
 // reference evaluates one point at a time on one CPU core.
 //
-// Work decomposition: a CTA owns one GridItem = a tile of kGridSlotPts points
-// of one frame (PPT points per thread, kept in registers) and a contiguous
-// range of that frame's charges.  The charges stream through a ring of shared
-// memory stages filled by 1-D bulk async copies (cp.async.bulk) that complete
-// on mbarriers; every thread reads each staged charge as a broadcast and
-// applies it to its PPT points.
+// Work decomposition: a CTA owns a tile of a frame's points (kGridThreads
+// threads, PPT points each, kept in registers) and a contiguous chunk of that
+// frame's charges.  The charges stream through a ring of shared memory stages
+// filled by 1-D bulk async copies (cp.async.bulk) that complete on mbarriers;
+// every thread reads each staged charge as a broadcast and applies it to its
+// PPT points.
+//
+// Lattices: the points of a volume are a mesh, x slowest.  The preparation
+// kernel looks for the stride S after which (y, z) repeat, and for meshes a
+// thread takes PPT points of one (y, z) column: dy, dz and dy^2 + dz^2 are formed
+// once per charge instead of once per point and charge, in the same order of
+// operations, so the sums are the same bits.  That is 9 instead of 12 FP32-pipe
+// operations per pair (4 instead of 7 for the potential, which is then bound by
+// the MUFU alone), 9.25 FP64-pipe instructions instead of 13.  The points that do
+// not fill a column's last group are evaluated as points without a mesh.
 //
 // Precision forms:
 //   FP32C  pair terms in FP32 with the MUFU rsqrt; each stage's contribution is
@@ -19,7 +28,10 @@
 //          the CTA as a double.
 //   FP64   every operation in IEEE double (plain sums), the drop-in form.
 // A frame whose charges are split over several items writes per-split partial
-// sums (doubles) that grid_final_kernel adds in split order: deterministic.
+// sums (doubles) that grid_final_kernel adds in a fixed order: deterministic.
+// A frame of at most kGridFewPoints points (point fields) goes to
+// grid_few_kernel, whose threads take (point, run of charges) units instead of
+// points, with the same runs and order.
 //
 // The r^2 >= 1e-6 clamp of compute_looped_field only changes a pair term when
 // a point lies within 1e-3 A of a charge.  A CTA takes the bounding box of its
@@ -29,14 +41,18 @@
 //
 // FP32C field refinement: where the field nearly cancels, FP32 rounding of the
 // pair terms (about 1e-7 of each term) is a large fraction of |E|.  After the
-// FP32C pass, grid_mag_hist_kernel and grid_flag_kernel find, per frame, the
-// points whose |E| is below tau times the frame's median |E| (taken from a
-// histogram of |E|^2) and grid_refine_kernel recomputes those
+// FP32C pass, grid_final_kernel (which counts a histogram of |E|^2 and takes the
+// median from it) and grid_flag_kernel find, per frame, the points whose |E| is
+// below tau times the frame's median |E| and grid_refine_kernel recomputes those
 // points over all of the frame's charges in double-float arithmetic (pairs of
 // floats, about 48 significant bits, on the FP32 pipe: GB300's FP64 pipe is
 // 1/64 of its FP32 pipe).
 #include <algorithm>
+#include <climits>
+#include <cstddef>
 #include <type_traits>
+
+#include <cooperative_groups.h>
 
 #include "common.cuh"
 #include "kernels.cuh"
@@ -45,6 +61,15 @@ namespace cpetgb {
 namespace {
 
 constexpr int kStages = 4;
+
+// static_cast<Real>, FP32C without the FP64 pipe.
+template <typename Real>
+__device__ __forceinline__ Real to_real(double v) {
+  if constexpr (sizeof(Real) == 4)
+    return narrow(v);
+  else
+    return v;
+}
 
 template <int PREC>
 struct GridCfg;
@@ -148,11 +173,38 @@ __device__ __forceinline__ void pair_terms_f32x2(const ChargeDup& ch, const uint
   }
 }
 
+// One charge against G packed point pairs of one (y, z) column: the same
+// operations as pair_terms_f32x2, those of y and z once.
+template <int KIND, int G>
+__device__ __forceinline__ void column_terms_f32x2(const ChargeDup& ch, const uint64_t (&px)[G], float py,
+                                                   float pz, uint64_t (&part)[(KIND == kField) ? 3 : 1][G]) {
+  const ulonglong2 xy = ch.xy;
+  const ulonglong2 zq = ch.zq;
+  const float dy = __fsub_rn(py, __uint_as_float(static_cast<uint32_t>(xy.y)));
+  const float dz = __fsub_rn(pz, __uint_as_float(static_cast<uint32_t>(zq.x)));
+  const float t = __fmaf_rn(dy, dy, __fmul_rn(dz, dz));
+  const uint64_t t2 = pk2(t, t), dy2 = pk2(dy, dy), dz2 = pk2(dz, dz);
+#pragma unroll
+  for (int g = 0; g < G; ++g) {
+    const uint64_t dx = sub2(px[g], xy.x);
+    const uint64_t ri = rsqrt2(fma2(dx, dx, t2));
+    if constexpr (KIND == kField) {
+      const uint64_t w = mul2(mul2(zq.y, ri), mul2(ri, ri));
+      part[0][g] = fma2(w, dx, part[0][g]);
+      part[1][g] = fma2(w, dy2, part[1][g]);
+      part[2][g] = fma2(w, dz2, part[2][g]);
+    } else {
+      part[0][g] = fma2(zq.y, ri, part[0][g]);
+    }
+  }
+}
+
 // FP32C body: this thread's points as G packed pairs (points k = 2g, 2g+1).
 // CLAMP = true is the rare path (a staged charge next to the point box): the
 // same arithmetic with the clamp, in a loop that is not unrolled, so it adds
 // few registers to the kernel.
-template <int KIND, bool CLAMP, int G>
+// COLUMN: the points are of one (y, z) column.
+template <int KIND, bool CLAMP, bool COLUMN, int G>
 __device__ __forceinline__ void grid_tile_f32x2(const ChargeDup* __restrict__ tl, int cnt,
                                                 const uint64_t (&px)[G], const uint64_t (&py)[G],
                                                 const uint64_t (&pz)[G], uint64_t (&acc)[3][G],
@@ -168,6 +220,11 @@ __device__ __forceinline__ void grid_tile_f32x2(const ChargeDup* __restrict__ tl
     if constexpr (CLAMP) {
 #pragma unroll 1
       for (int j = j0; j < j1; ++j) pair_terms_f32x2<KIND, true, G>(tl[j], px, py, pz, part);
+    } else if constexpr (COLUMN) {
+      const float y = __uint_as_float(static_cast<uint32_t>(py[0]));
+      const float z = __uint_as_float(static_cast<uint32_t>(pz[0]));
+#pragma unroll 8
+      for (int j = j0; j < j1; ++j) column_terms_f32x2<KIND, G>(tl[j], px, y, z, part);
     } else {
 #pragma unroll 4
       for (int j = j0; j < j1; ++j) pair_terms_f32x2<KIND, false, G>(tl[j], px, py, pz, part);
@@ -179,11 +236,81 @@ __device__ __forceinline__ void grid_tile_f32x2(const ChargeDup* __restrict__ tl
   }
 }
 
-// FP32C with 4 points per thread: at most 80 registers, so six CTAs (24
-// warps) share an SM.
+// The frame of item / tile / preparation block `i`: the last one whose base (the
+// int32 at byte offset OFF of the record) is <= i.  32 records per look, by a
+// whole warp.
+template <int OFF>
+__device__ __forceinline__ int find_frame(const GridFrame* frames, int n_frames, int i) {
+  const int lane = threadIdx.x & 31;
+  auto base = [&](int f) {
+    return *reinterpret_cast<const int32_t*>(reinterpret_cast<const char*>(frames + f) + OFF);
+  };
+  int lo = 0, span = n_frames;
+  while (span > 1) {  // narrow [lo, lo + span) to one of 32 parts
+    const int part = (span + 31) / 32;
+    const int f = lo + lane * part;
+    const unsigned below = __ballot_sync(0xffffffffu, lane * part < span && base(f) <= i);
+    const int k = 31 - __clz(below);
+    span = min(part, span - k * part);
+    lo += k * part;
+  }
+  return lo;
+}
+
+// A kernel's view of its frame: the launch's only one, from the kernel's
+// parameters, or the table's entry.
+template <int OFF>
+__device__ __forceinline__ GridFrame load_frame(const GridFrame* frames, int n_frames, const GridFrame& one,
+                                                int i, int* f) {
+  if (n_frames == 1) {
+    *f = 0;
+    return one;
+  }
+  *f = find_frame<OFF>(frames, n_frames, i);
+  return frames[*f];
+}
+
+// Which points a frame's threads take (u: thread of the frame, k: its k-th
+// point): -1 for none.  stride: the lattice stride S, or 0.
+struct PointMap {
+  int stride, lat_threads, lat_end, rest;  // columns x groups; rounded up to a warp; first other point
+  int n_points;
+
+  template <int PPT>
+  __device__ __forceinline__ void set(int s, int P) {
+    n_points = P;
+    stride = s;
+    const int groups = s > 0 ? P / s / PPT : 0;
+    lat_threads = s * groups;
+    lat_end = (lat_threads + 31) & ~31;
+    rest = lat_threads * PPT;
+  }
+  // Threads of the frame that have points, rounded up to a warp.
+  template <int PPT>
+  __device__ __forceinline__ int threads() const {
+    return lat_end + (n_points - rest + 32 * PPT - 1) / (32 * PPT) * 32;
+  }
+  __device__ __forceinline__ bool column(int u) const { return u < lat_end; }  // uniform across a warp
+  template <int PPT>
+  __device__ __forceinline__ int point(int u, int k) const {
+    if (u < lat_end) {
+      if (u >= lat_threads) return -1;
+      const int g = u / stride;
+      return (g * PPT + k) * stride + (u - g * stride);
+    }
+    const int v = u - lat_end;
+    const int p = rest + (v >> 5) * (32 * PPT) + 32 * k + (v & 31);
+    return p < n_points ? p : -1;
+  }
+};
+
+// FP32C with 4 points per thread: four CTAs (16 warps) per SM for the field,
+// whose column loop needs more than 80 registers to keep the FP32 pipe fed (24
+// frames: 2.09 ms, 2.20 with six CTAs), six for the potential.
 template <int PREC, int KIND, bool CLAMP, int PPT>
-__global__ void __launch_bounds__(kGridThreads, PREC == kFP32C && PPT == 4 ? 6 : 0)
-    grid_kernel(const GridItem* __restrict__ items, const void* __restrict__ packed,
+__global__ void __launch_bounds__(kGridThreads, PREC == kFP32C && PPT == 4 ? (KIND == kField ? 4 : 6) : 0)
+    grid_kernel(const GridFrame* __restrict__ frames, int n_frames, const GridFrame one, int item0,
+                const int* __restrict__ stride, const int* __restrict__ broken, const void* __restrict__ packed,
                 const double* __restrict__ points, double* __restrict__ out,
                 double* __restrict__ partial, int* __restrict__ status) {
   using Cfg = GridCfg<PREC>;
@@ -195,11 +322,20 @@ __global__ void __launch_bounds__(kGridThreads, PREC == kFP32C && PPT == 4 ? 6 :
   __shared__ alignas(128) ChargeT tile[kStages][TC];
   __shared__ alignas(8) uint64_t full[kStages];
 
-  const GridItem it = items[blockIdx.x];
-  const ChargeT* src = reinterpret_cast<const ChargeT*>(packed) + it.charge_off + it.n_begin;
-  const int n = it.n_count;
-  const int n_tiles = (n + TC - 1) / TC;
   const int tid = threadIdx.x;
+  const int item = item0 + static_cast<int>(blockIdx.x);
+  int f;
+  const GridFrame fr = load_frame<offsetof(GridFrame, item_base)>(frames, n_frames, one, item, &f);
+  const int n_tiles_pt = fr.n_tiles;
+  const int split = (item - fr.item_base) / n_tiles_pt;
+  const int tile_id = (item - fr.item_base) - split * n_tiles_pt;
+  const int n_begin = split * fr.chunk;
+  const int n = min(fr.chunk, fr.n_charges - n_begin);
+  const ChargeT* src = reinterpret_cast<const ChargeT*>(packed) + fr.charge_off + n_begin;
+  const int n_tiles = (n + TC - 1) / TC;
+  PointMap map;
+  map.set<PPT>(stride && !broken[f] ? stride[f] : 0, fr.n_points);
+  if (tile_id * kGridThreads >= map.threads<PPT>()) return;  // the table's last tile may be spare
 
   if (tid == 0) {
     for (int s = 0; s < kStages; ++s) mbar_init(&full[s], 1);
@@ -218,16 +354,21 @@ __global__ void __launch_bounds__(kGridThreads, PREC == kFP32C && PPT == 4 ? 6 :
     for (int t = 0; t < min(kStages, n_tiles); ++t) issue(t);
   }
 
+  const int u = tile_id * kGridThreads + tid;
+  const int64_t point_off = fr.point_off;
+  const bool column = map.column(u);
+  unsigned valid = 0;  // which of this thread's points exist
   // This thread's points, in registers (FP32C: packed in pairs).
   Real px[PPT], py[PPT], pz[PPT];
 #pragma unroll
   for (int k = 0; k < PPT; ++k) {
-    const int pl = tid + k * kGridThreads;
-    if (pl < it.p_count) {
-      const double* pp = points + 3 * (it.point_off + it.p_begin + pl);
-      px[k] = static_cast<Real>(pp[0]);
-      py[k] = static_cast<Real>(pp[1]);
-      pz[k] = static_cast<Real>(pp[2]);
+    const int pl = map.point<PPT>(u, k);
+    if (pl >= 0) {
+      valid |= 1u << k;
+      const double* pp = points + 3 * (point_off + pl);
+      px[k] = to_real<Real>(pp[0]);
+      py[k] = to_real<Real>(pp[1]);
+      pz[k] = to_real<Real>(pp[2]);
     } else {
       px[k] = py[k] = pz[k] = static_cast<Real>(1.0e4);  // far away, never written
     }
@@ -260,7 +401,7 @@ __global__ void __launch_bounds__(kGridThreads, PREC == kFP32C && PPT == 4 ? 6 :
     float v[6] = {3.0e38f, 3.0e38f, 3.0e38f, -3.0e38f, -3.0e38f, -3.0e38f};
 #pragma unroll
     for (int k = 0; k < PPT; ++k) {
-      if (tid + k * kGridThreads < it.p_count) {
+      if ((valid >> k) & 1u) {
         const float c3[3] = {static_cast<float>(px[k]), static_cast<float>(py[k]),
                              static_cast<float>(pz[k])};
 #pragma unroll
@@ -291,6 +432,7 @@ __global__ void __launch_bounds__(kGridThreads, PREC == kFP32C && PPT == 4 ? 6 :
     __syncthreads();
   }
 
+  const bool work = __any_sync(0xffffffffu, valid != 0);  // a warp without points only waits
   bool ok = true;
   for (int t = 0; t < n_tiles; ++t) {
     const int s = t % kStages;
@@ -322,34 +464,48 @@ __global__ void __launch_bounds__(kGridThreads, PREC == kFP32C && PPT == 4 ? 6 :
     if (!ok) break;
     if (tid == 0 && t >= 1 && (t - 1) + kStages < n_tiles) issue((t - 1) + kStages);
 
+    if (!work) continue;
     if constexpr (PREC == kFP32C) {
       if (CLAMP && clamp_tile)
-        grid_tile_f32x2<KIND, true, G>(tl, cnt, px2, py2, pz2, acc2, cmp2);
+        grid_tile_f32x2<KIND, true, false, G>(tl, cnt, px2, py2, pz2, acc2, cmp2);
+      else if (column)
+        grid_tile_f32x2<KIND, false, true, G>(tl, cnt, px2, py2, pz2, acc2, cmp2);
       else
-        grid_tile_f32x2<KIND, false, G>(tl, cnt, px2, py2, pz2, acc2, cmp2);
+        grid_tile_f32x2<KIND, false, false, G>(tl, cnt, px2, py2, pz2, acc2, cmp2);
     } else {
       Real part[NC][PPT];
 #pragma unroll
       for (int c = 0; c < NC; ++c)
 #pragma unroll
         for (int k = 0; k < PPT; ++k) part[c][k] = Real(0);
-#pragma unroll 4
-      for (int j = 0; j < cnt; ++j) {
-        const ChargeT ch = tl[j];
+      auto term = [&](const ChargeT& ch, int k, Real dy, Real dz, Real t) {
+        const Real dx = px[k] - ch.x;
+        Real r2 = __fma_rn(dx, dx, t);
+        if (CLAMP && clamp_tile) r2 = fmax(r2, Real(1e-6));  // compute_looped_field's fmaxf
+        const Real w = weight_f64<KIND>(ch, r2);
+        if constexpr (KIND == kField) {
+          part[0][k] += w * dx;
+          part[1][k] += w * dy;
+          part[2][k] += w * dz;
+        } else {
+          part[0][k] += w;
+        }
+      };
+      if (column) {
+        for (int j = 0; j < cnt; ++j) {
+          const ChargeT ch = tl[j];
+          const Real dy = py[0] - ch.y, dz = pz[0] - ch.z;
+          const Real t = __fma_rn(dy, dy, __dmul_rn(dz, dz));
 #pragma unroll
-        for (int k = 0; k < PPT; ++k) {
-          const Real dx = px[k] - ch.x;
-          const Real dy = py[k] - ch.y;
-          const Real dz = pz[k] - ch.z;
-          Real r2 = dx * dx + dy * dy + dz * dz;
-          if (CLAMP && clamp_tile) r2 = fmax(r2, Real(1e-6));  // compute_looped_field's fmaxf
-          if constexpr (KIND == kField) {
-            const Real w = weight_f64<KIND>(ch, r2);
-            part[0][k] += w * dx;
-            part[1][k] += w * dy;
-            part[2][k] += w * dz;
-          } else {
-            part[0][k] += weight_f64<KIND>(ch, r2);
+          for (int k = 0; k < PPT; ++k) term(ch, k, dy, dz, t);
+        }
+      } else {
+        for (int j = 0; j < cnt; ++j) {
+          const ChargeT ch = tl[j];
+#pragma unroll
+          for (int k = 0; k < PPT; ++k) {
+            const Real dy = py[k] - ch.y, dz = pz[k] - ch.z;
+            term(ch, k, dy, dz, __fma_rn(dy, dy, __dmul_rn(dz, dz)));
           }
         }
       }
@@ -361,10 +517,11 @@ __global__ void __launch_bounds__(kGridThreads, PREC == kFP32C && PPT == 4 ? 6 :
   }
   if (!ok) return;
 
+  constexpr int kTilePts = kGridThreads * PPT;
+  const int slot = fr.slot_base < 0 ? -1 : fr.slot_base + (item - fr.item_base);
 #pragma unroll
   for (int k = 0; k < PPT; ++k) {
-    const int pl = tid + k * kGridThreads;
-    if (pl >= it.p_count) continue;
+    if (!((valid >> k) & 1u)) continue;
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       double v;
@@ -373,43 +530,145 @@ __global__ void __launch_bounds__(kGridThreads, PREC == kFP32C && PPT == 4 ? 6 :
         upk2(acc2[c][k / 2], sl, sh);
         upk2(cmp2[c][k / 2], cl, ch);
         const float sv = (k & 1) ? sh : sl, cv = (k & 1) ? ch : cl;
-        v = (static_cast<double>(sv) - static_cast<double>(cv)) * kCoulomb;
+        v = __dmul_rn(__dsub_rn(widen(sv), widen(cv)), kCoulomb);
       } else {
         v = static_cast<double>(acc[c][k]) * kCoulomb;
       }
-      if (it.slot < 0) {
-        out[NC * (it.point_off + it.p_begin + pl) + c] = v;
-      } else {
-        partial[(static_cast<int64_t>(it.slot) * kGridSlotPts + pl) * 3 + c] = v;
-      }
+      if (slot < 0)
+        out[NC * (point_off + map.point<PPT>(u, k)) + c] = v;
+      else
+        partial[(static_cast<int64_t>(slot) * NC + c) * kTilePts + k * kGridThreads + tid] = v;
     }
   }
 }
 
-template <int KIND>
-__global__ void grid_final_kernel(const GridFinal* __restrict__ fin,
-                                  const double* __restrict__ partial, double* __restrict__ out) {
-  constexpr int NC = (KIND == kField) ? 3 : 1;
-  const GridFinal f = fin[blockIdx.x];
-  for (int i = threadIdx.x; i < f.p_count * NC; i += blockDim.x) {
-    const int pl = i / NC, c = i % NC;
-    double v = 0.0;
-    for (int s = 0; s < f.n_split; ++s)
-      v += partial[(static_cast<int64_t>(f.slot_base + s) * kGridSlotPts + pl) * 3 + c];
-    out[NC * (f.out_row + pl) + c] = v;
-  }
+// Sum over a frame's splits, in one order everywhere: eight partial sums (splits
+// l, l + 8, ...), then ((v0 + v4) + (v2 + v6)) + ((v1 + v5) + (v3 + v7)).  By one
+// thread, or by eight neighbouring lanes (l = lane & 7): an FP64 addition holds a
+// scheduler's pipe for 64 cycles, so a few points with hundreds of splits would
+// otherwise wait for one long chain.
+constexpr int kSumLanes = 8;
+__device__ __forceinline__ double sum_lanes(double v) {
+#pragma unroll
+  for (int o = kSumLanes / 2; o >= 1; o >>= 1) v = __dadd_rn(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+__device__ __forceinline__ double sum_thread(const double (&v)[kSumLanes]) {
+  return __dadd_rn(__dadd_rn(__dadd_rn(v[0], v[4]), __dadd_rn(v[2], v[6])),
+                   __dadd_rn(__dadd_rn(v[1], v[5]), __dadd_rn(v[3], v[7])));
 }
 
-// ---------------------------------------------------------------------------
-// FP32C field refinement (see the header comment).
-// ---------------------------------------------------------------------------
-constexpr int kFlagThreads = 512;
-constexpr int kFlagChunk = kFlagThreads * 8;  // points of a frame per flagging CTA
-constexpr int kMagBins = 4096;  // bits 30..19 of the float |E|^2: exponent + 4 mantissa bits
-constexpr int kBinsPerThread = kMagBins / kFlagThreads;
-// 256 threads: the refinement CTAs must fit beside a serving engine launch
-// that holds half of every SM's registers (engine.cu), as the grid CTAs do.
-constexpr int kRefineThreads = 256;
+// Frames of few points (point fields): a CTA takes one chunk of a frame's
+// charges against all of its points.  Its threads take units of one point and
+// one run of kFewRun charges (the tile kernel's Kahan runs in FP32C: 32 charges
+// within stages of 256, so the sums are the same bits), and then add the runs of
+// each point and component in order.  With a thread per point instead, a
+// 1-point launch took 20 us (739 us in FP64) for the padding of its tile.
+template <int PREC, int KIND, bool CLAMP, int PPT>
+__global__ void __launch_bounds__(kGridThreads)
+    grid_few_kernel(const GridFrame* __restrict__ frames, int n_frames, const GridFrame one, const void* __restrict__ packed,
+                    const double* __restrict__ points, double* __restrict__ out,
+                    double* __restrict__ partial) {
+  using ChargeT = typename GridCfg<PREC>::ChargeT;
+  using Real = typename GridCfg<PREC>::Real;
+  constexpr int NC = (KIND == kField) ? 3 : 1;
+  constexpr int kFewRun = PREC == kFP32C ? kKahanRun : 8;
+  constexpr int kStage = GridCfg<PREC>::kTile;
+  constexpr int kUnits = 1024;  // (point, run) sums held at a time
+  __shared__ Real sums[NC][kUnits];
+  __shared__ Real acc_s[NC * kGridFewPoints], cmp_s[NC * kGridFewPoints];
+  const int tid = threadIdx.x;
+  const int item = static_cast<int>(blockIdx.x);
+  int f;
+  const GridFrame fr = load_frame<offsetof(GridFrame, item_base)>(frames, n_frames, one, item, &f);
+  const int P = fr.n_points;
+  const int split = item - fr.item_base;  // one tile
+  const int n_begin = split * fr.chunk;
+  const int n = min(fr.chunk, fr.n_charges - n_begin);
+  const ChargeT* src = reinterpret_cast<const ChargeT*>(packed) + fr.charge_off + n_begin;
+  const double* pts = points + 3 * fr.point_off;
+  for (int i = tid; i < NC * P; i += kGridThreads) acc_s[i] = cmp_s[i] = Real(0);
+  // runs: kStage / kFewRun per full stage, the last stage's last one shorter
+  const int runs = (n / kStage) * (kStage / kFewRun) + (n % kStage + kFewRun - 1) / kFewRun;
+  const int rb = kUnits / P;  // runs per pass
+  for (int r0 = 0; r0 < runs; r0 += rb) {
+    const int nr = min(rb, runs - r0);
+    __syncthreads();
+    for (int i = tid; i < nr * P; i += kGridThreads) {
+      const int r = i / P, p = i - r * P;
+      const Real x = to_real<Real>(pts[3 * p]), y = to_real<Real>(pts[3 * p + 1]),
+                 z = to_real<Real>(pts[3 * p + 2]);
+      const int j0 = (r0 + r) * kFewRun, cnt = min(kFewRun, n - j0);
+      Real part[NC];
+#pragma unroll
+      for (int c = 0; c < NC; ++c) part[c] = Real(0);
+#pragma unroll 8
+      for (int j = 0; j < cnt; ++j) {
+        const ChargeT ch = src[j0 + j];
+        if constexpr (PREC == kFP32C) {
+          const float dx = __fsub_rn(x, __uint_as_float(static_cast<uint32_t>(ch.xy.x)));
+          const float dy = __fsub_rn(y, __uint_as_float(static_cast<uint32_t>(ch.xy.y)));
+          const float dz = __fsub_rn(z, __uint_as_float(static_cast<uint32_t>(ch.zq.x)));
+          const float q = __uint_as_float(static_cast<uint32_t>(ch.zq.y));
+          float r2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
+          if (CLAMP && r2 < 1e-6f) r2 = 1e-6f;
+          const float ri = rsqrt_mufu(r2);
+          if constexpr (KIND == kField) {
+            const float w = __fmul_rn(__fmul_rn(q, ri), __fmul_rn(ri, ri));
+            part[0] = __fmaf_rn(w, dx, part[0]);
+            part[1] = __fmaf_rn(w, dy, part[1]);
+            part[2] = __fmaf_rn(w, dz, part[2]);
+          } else {
+            part[0] = __fmaf_rn(q, ri, part[0]);
+          }
+        } else {
+          const double dx = x - ch.x, dy = y - ch.y, dz = z - ch.z;
+          double r2 = __fma_rn(dx, dx, __fma_rn(dy, dy, __dmul_rn(dz, dz)));
+          if (CLAMP && r2 < 1e-6) r2 = 1e-6;
+          const double w = weight_f64<KIND>(ch, r2);
+          if constexpr (KIND == kField) {
+            part[0] = __fma_rn(w, dx, part[0]);
+            part[1] = __fma_rn(w, dy, part[1]);
+            part[2] = __fma_rn(w, dz, part[2]);
+          } else {
+            part[0] = __dadd_rn(part[0], w);
+          }
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < NC; ++c) sums[c][i] = part[c];
+    }
+    __syncthreads();
+    for (int i = tid; i < NC * P; i += kGridThreads) {
+      const int c = i / P, p = i - c * P;
+      Real acc = acc_s[i];
+      [[maybe_unused]] Real cmp = cmp_s[i];
+#pragma unroll 4
+      for (int r = 0; r < nr; ++r) {
+        if constexpr (PREC == kFP32C)
+          kahan_add(acc, cmp, sums[c][r * P + p]);
+        else
+          acc = __dadd_rn(acc, sums[c][r * P + p]);
+      }
+      acc_s[i] = acc;
+      if constexpr (PREC == kFP32C) cmp_s[i] = cmp;
+    }
+  }
+  __syncthreads();
+  constexpr int kTilePts = kGridThreads * PPT;
+  for (int i = tid; i < NC * P; i += kGridThreads) {
+    const int c = i / P, p = i - c * P;
+    double v;
+    if constexpr (PREC == kFP32C)
+      v = __dmul_rn(__dsub_rn(widen(acc_s[i]), widen(cmp_s[i])), kCoulomb);
+    else
+      v = acc_s[i] * kCoulomb;
+    if (fr.slot_base < 0)
+      out[NC * (fr.point_off + p) + c] = v;
+    else
+      partial[(static_cast<int64_t>(fr.slot_base + split) * NC + c) * kTilePts + p] = v;
+  }
+}
 
 // Integer-only reads of doubles.  GB300's FP64 pipe is 1/64 of its FP32 pipe
 // and conversions from double run on it, so the refinement's helpers take a
@@ -464,125 +723,292 @@ __device__ __forceinline__ float field_norm2(const double* e) {
   return __fmaf_rn(x, x, __fmaf_rn(y, y, __fmul_rn(z, z)));
 }
 
-// Histogram of |E|^2 over the frames' points in 1/16-octave bins (of |E|^2;
-// 1/32 octave of |E|): grid (frame, chunk of kFlagChunk points); each CTA
-// counts its chunk in shared memory and adds its non-empty bins to the frame's
-// row of hist[n_frames][kMagBins] (zeroed by the caller).
-__global__ void __launch_bounds__(kFlagThreads)
-    grid_mag_hist_kernel(const int64_t* __restrict__ desc, const double* __restrict__ out,
-                         int* __restrict__ hist) {
-  __shared__ int h[kMagBins];
-  const int64_t po = desc[4 * blockIdx.x + 2], P = desc[4 * blockIdx.x + 3];
-  const int64_t i0 = static_cast<int64_t>(blockIdx.y) * kFlagChunk;
-  if (i0 >= P) return;
-  const int64_t i1 = min(P, i0 + kFlagChunk);
-  for (int b = threadIdx.x; b < kMagBins; b += kFlagThreads) h[b] = 0;
-  __syncthreads();
-  for (int64_t i = i0 + threadIdx.x; i < i1; i += kFlagThreads) {
-    const float m2 = field_norm2(out + 3 * (po + i));
-    if (m2 <= 3.0e38f)  // finite (NaN compares false)
-      atomicAdd(&h[__float_as_uint(m2) >> 19], 1);
+// One frame of few points, FP32C, in one launch: as grid_few_kernel and the sum
+// over the splits, by one cluster of CTAs that read the caller's arrays.  CTA r
+// takes the splits r, r + kPointCtas, ...; the splits' results go to CTA 0's shared
+// memory, which adds them in split order.  The smallest calls are a chain of
+// launches (27 us of GPU time for packing, sums and the sum over the splits of one
+// point and 8,000 charges); one CTA alone took 37 us for reading the charges.
+constexpr int kPointCtas = 8;
+constexpr int kPointThreads = 256;
+constexpr int kPointUnits = 2048;       // (point, run) units per CTA at most
+constexpr int kPointResults = 2048;     // results of all splits at most
+constexpr int kPointCharges = 4096;     // charges per CTA at most
+
+template <int KIND, bool CLAMP>
+__global__ void __cluster_dims__(kPointCtas, 1, 1) __launch_bounds__(kPointThreads)
+    grid_point_kernel(const GridFrame fr, const double* __restrict__ points, const double* __restrict__ x,
+                      const double* __restrict__ q, double* __restrict__ out) {
+  constexpr int NC = (KIND == kField) ? 3 : 1;
+  extern __shared__ __align__(16) unsigned char point_smem[];
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int rank = static_cast<int>(cluster.block_rank());
+  const int tid = threadIdx.x;
+  const int P = fr.n_points, ns = fr.n_split, chunk = fr.chunk, n_all = fr.n_charges;
+  const int rps = (chunk + kKahanRun - 1) / kKahanRun;  // runs per split
+  const int mine = (ns - rank + kPointCtas - 1) / kPointCtas;
+  const int most = (ns + kPointCtas - 1) / kPointCtas;
+  const int units = P * most * rps;
+  float4* ch_s = reinterpret_cast<float4*>(point_smem);                  // [most][chunk]
+  double* v_s = reinterpret_cast<double*>(ch_s + most * chunk);          // [ns][NC * P], CTA 0's used
+  float* sums = reinterpret_cast<float*>(v_s + ns * NC * P);             // [NC][units]
+  const double* pts = points + 3 * fr.point_off;
+  const double* xs = x + 3 * fr.charge_off;
+  const double* qs = q + fr.charge_off;
+#pragma unroll 4
+  for (int i = tid; i < mine * chunk; i += kPointThreads) {
+    const int k = i / chunk, j = (rank + k * kPointCtas) * chunk + (i - k * chunk);
+    if (j < n_all) {
+      const double* xj = xs + 3 * static_cast<int64_t>(j);
+      ch_s[i] = make_float4(narrow(xj[0]), narrow(xj[1]), narrow(xj[2]), narrow(qs[j]));
+    }
   }
   __syncthreads();
-  int* row = hist + static_cast<int64_t>(blockIdx.x) * kMagBins;
-  for (int b = threadIdx.x; b < kMagBins; b += kFlagThreads)
-    if (h[b]) atomicAdd(&row[b], h[b]);
+  for (int i = tid; i < mine * rps * P; i += kPointThreads) {
+    const int p = i % P, kr = i / P, k = kr / rps, r = kr - k * rps;
+    const float px = narrow(pts[3 * p]), py = narrow(pts[3 * p + 1]), pz = narrow(pts[3 * p + 2]);
+    const int n = min(chunk, n_all - (rank + k * kPointCtas) * chunk);
+    const int cnt = max(0, min(kKahanRun, n - r * kKahanRun));
+    const float4* src = ch_s + k * chunk + r * kKahanRun;
+    float part[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) part[c] = 0.f;
+#pragma unroll 8
+    for (int j = 0; j < cnt; ++j) {
+      const float4 ch = src[j];
+      const float dx = __fsub_rn(px, ch.x);
+      const float dy = __fsub_rn(py, ch.y);
+      const float dz = __fsub_rn(pz, ch.z);
+      float r2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
+      if (CLAMP && r2 < 1e-6f) r2 = 1e-6f;
+      const float ri = rsqrt_mufu(r2);
+      if constexpr (KIND == kField) {
+        const float w = __fmul_rn(__fmul_rn(ch.w, ri), __fmul_rn(ri, ri));
+        part[0] = __fmaf_rn(w, dx, part[0]);
+        part[1] = __fmaf_rn(w, dy, part[1]);
+        part[2] = __fmaf_rn(w, dz, part[2]);
+      } else {
+        part[0] = __fmaf_rn(ch.w, ri, part[0]);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < NC; ++c) sums[c * units + i] = part[c];
+  }
+  __syncthreads();
+  double* v_0 = cluster.map_shared_rank(v_s, 0);
+  for (int i = tid; i < mine * NC * P; i += kPointThreads) {
+    const int k = i / (NC * P), cp = i - k * (NC * P), c = cp / P, p = cp - c * P;
+    const int split = rank + k * kPointCtas;
+    const int n = min(chunk, n_all - split * chunk);
+    const int nr = (n + kKahanRun - 1) / kKahanRun;
+    const float* in = sums + c * units + (k * rps) * P + p;
+    float acc = 0.f, cmp = 0.f;
+#pragma unroll 4
+    for (int r = 0; r < nr; ++r) kahan_add(acc, cmp, in[r * P]);
+    v_0[split * NC * P + cp] = __dmul_rn(__dsub_rn(widen(acc), widen(cmp)), kCoulomb);
+  }
+  cluster.sync();
+  if (rank != 0) return;
+  const int l = tid % kSumLanes;
+  for (int i0 = 0; i0 < NC * P; i0 += kPointThreads / kSumLanes) {
+    const int i = min(i0 + tid / kSumLanes, NC * P - 1);
+    double v = l < ns ? v_s[l * NC * P + i] : 0.0;
+#pragma unroll 4
+    for (int split = l + kSumLanes; split < ns; split += kSumLanes) v = __dadd_rn(v, v_s[split * NC * P + i]);
+    if (ns > 1) v = sum_lanes(v);
+    const int c = i / P, p = i - c * P;
+    if (l == 0) out[NC * (fr.point_off + p) + c] = v;
+  }
 }
 
-// Grid (frame, chunk) as grid_mag_hist_kernel.  Every CTA finds its frame's
-// scale -- the lower edge of the histogram bin holding the lower median of
-// |E|^2 -- and appends each point of its chunk with |E|^2 below tau^2 times
-// that scale to list[] as {output row, frame}.  The counts are exact
-// integers, so the threshold and the set of points are deterministic.
-__global__ void __launch_bounds__(kFlagThreads)
-    grid_flag_kernel(const int64_t* __restrict__ desc, const double* __restrict__ out,
-                     const int* __restrict__ hist, float tau2, int64_t* __restrict__ list,
-                     int* __restrict__ count) {
-  __shared__ int hs[kMagBins];
-  __shared__ int part[kFlagThreads];
-  __shared__ float scale_s;
-  const int64_t po = desc[4 * blockIdx.x + 2], P = desc[4 * blockIdx.x + 3];
-  const int64_t i0 = static_cast<int64_t>(blockIdx.y) * kFlagChunk;
-  if (i0 >= P) return;
-  const int64_t i1 = min(P, i0 + kFlagChunk);
-  const int* row = hist + static_cast<int64_t>(blockIdx.x) * kMagBins;
-  int own = 0;
-#pragma unroll
-  for (int k = 0; k < kBinsPerThread; ++k) {
-    const int v = row[threadIdx.x * kBinsPerThread + k];
-    hs[threadIdx.x * kBinsPerThread + k] = v;
-    own += v;
+constexpr int kMagBins = 4096;  // bits 30..19 of the float |E|^2: exponent + 4 mantissa bits
+
+// Sums of the splits.  LANES = 1: block (tile, k), a thread takes the k-th point of
+// a tile's thread; LANES = 8: eight lanes per point and eight blocks.  HIST
+// (FP32C field refinement): also counts |E|^2 in 1/16-octave bins (of |E|^2; 1/32
+// octave of |E|) per frame, exact integers, and a frame's last block takes the
+// scale from them: the lower edge of the bin that holds the lower median.
+template <int PREC, int KIND, int PPT, bool HIST, int LANES>
+__global__ void __launch_bounds__(kGridThreads)
+    grid_final_kernel(const GridFrame* __restrict__ frames, int n_frames, const GridFrame one,
+                      const int* __restrict__ stride, const int* __restrict__ broken,
+                      const double* __restrict__ partial, double* __restrict__ out, int* __restrict__ hist,
+                      int* __restrict__ done, float* __restrict__ scale) {
+  constexpr int NC = (KIND == kField) ? 3 : 1;
+  constexpr int kTilePts = kGridThreads * PPT;
+  constexpr int kBlocks = PPT * LANES;  // per tile
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int tile = static_cast<int>(blockIdx.x) / kBlocks, part = static_cast<int>(blockIdx.x) % kBlocks;
+  const int k = part / LANES;
+  const int th = ((part % LANES) * kGridThreads + tid) / LANES;  // thread of the tile
+  const int l = tid % LANES;
+  int f;
+  const GridFrame fr = load_frame<offsetof(GridFrame, tile_base)>(frames, n_frames, one, tile, &f);
+  const int t = tile - fr.tile_base;
+  int pl;
+  if (fr.few) {
+    pl = k * kGridThreads + th < fr.n_points ? k * kGridThreads + th : -1;
+  } else {
+    PointMap map;
+    map.set<PPT>(stride && !broken[f] ? stride[f] : 0, fr.n_points);
+    pl = map.point<PPT>(t * kGridThreads + th, k);
   }
-  part[threadIdx.x] = own;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    constexpr int kPerLane = kFlagThreads / 32;
-    const int lane = threadIdx.x;
-    int mine = 0;
+  double v[NC];
 #pragma unroll
-    for (int k = 0; k < kPerLane; ++k) mine += part[lane * kPerLane + k];
+  for (int c = 0; c < NC; ++c) v[c] = 0.0;
+  double* o = out + NC * (fr.point_off + max(pl, 0));
+  if (fr.slot_base >= 0) {
+    const double* in = partial + (static_cast<int64_t>(fr.slot_base + t) * NC) * kTilePts + k * kGridThreads + th;
+    const int64_t step = static_cast<int64_t>(fr.n_tiles) * NC * kTilePts;
+    const int ns = pl >= 0 ? fr.n_split : 0;
+    if constexpr (LANES == 1) {
+      double w[NC][kSumLanes];
+#pragma unroll
+      for (int c = 0; c < NC; ++c)
+#pragma unroll
+        for (int s = 0; s < kSumLanes; ++s) w[c][s] = s < ns ? in[s * step + c * kTilePts] : 0.0;
+      for (int s0 = kSumLanes; s0 < ns; s0 += kSumLanes) {
+#pragma unroll
+        for (int s = 0; s < kSumLanes; ++s)
+          if (s0 + s < ns) {
+#pragma unroll
+            for (int c = 0; c < NC; ++c) w[c][s] = __dadd_rn(w[c][s], in[(s0 + s) * step + c * kTilePts]);
+          }
+      }
+#pragma unroll
+      for (int c = 0; c < NC; ++c) v[c] = sum_thread(w[c]);
+    } else {
+#pragma unroll
+      for (int c = 0; c < NC; ++c) v[c] = l < ns ? in[l * step + c * kTilePts] : 0.0;
+#pragma unroll 4
+      for (int s = l + LANES; s < ns; s += LANES)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) v[c] = __dadd_rn(v[c], in[s * step + c * kTilePts]);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) v[c] = sum_lanes(v[c]);
+    }
+    if (pl >= 0 && l == 0)
+#pragma unroll
+      for (int c = 0; c < NC; ++c) o[c] = v[c];
+  } else if (HIST && pl >= 0) {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) v[c] = o[c];
+  }
+  if constexpr (HIST) {
+    int* row = hist + static_cast<int64_t>(f) * kMagBins;
+    const float m2 = pl >= 0 && l == 0 ? field_norm2(v) : 4.0e38f;
+    const int bin = m2 <= 3.0e38f ? static_cast<int>(__float_as_uint(m2) >> 19) : -1;  // finite (NaN compares false)
+    const unsigned same = __match_any_sync(0xffffffffu, bin);
+    if (bin >= 0 && lane == __ffs(same) - 1) atomicAdd(&row[bin], __popc(same));
+    __shared__ int s_last;
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(&done[f], 1) == fr.n_tiles * kBlocks - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    // 32 consecutive bins per thread
+    constexpr int kPer = kMagBins / kGridThreads;
+    __shared__ int warp_sum[kGridThreads / 32];
+    int own[kPer], mine = 0;
+#pragma unroll
+    for (int b = 0; b < kPer; b += 4) {
+      const int4 h = __ldcg(reinterpret_cast<const int4*>(row + tid * kPer + b));
+      own[b] = h.x;
+      own[b + 1] = h.y;
+      own[b + 2] = h.z;
+      own[b + 3] = h.w;
+      mine += h.x + h.y + h.z + h.w;
+    }
+    int incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int w = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += w;
+    }
+    if (lane == 31) warp_sum[tid >> 5] = incl;
+    __syncthreads();
+    int total = 0;
+#pragma unroll
+    for (int w = 0; w < kGridThreads / 32; ++w) {
+      if (w < (tid >> 5)) incl += warp_sum[w];
+      total += warp_sum[w];
+    }
+    const int rank = (total - 1) / 2;
+    if (total > 0 && incl > rank && incl - mine <= rank) {
+      int cum = incl - mine, bin_of_rank = tid * kPer;
+#pragma unroll
+      for (int b = 0; b < kPer; ++b) {
+        if (cum <= rank && cum + own[b] > rank) bin_of_rank = tid * kPer + b;
+        cum += own[b];
+      }
+      scale[f] = __uint_as_float(static_cast<uint32_t>(bin_of_rank) << 19);
+    }  // no finite value: the scale stays 0 and nothing is refined
+  }
+}
+
+// ---------------------------------------------------------------------------
+// FP32C field refinement (see the header comment).
+// ---------------------------------------------------------------------------
+constexpr int kFlagThreads = 256;
+constexpr int kFlagChunk = kFlagThreads * 4;  // points of a frame per flagging CTA
+// 512 threads of at most 64 registers: the refinement CTAs must fit beside a
+// serving engine launch that holds half of every SM's registers (engine.cu), as
+// the grid CTAs do.
+constexpr int kRefineThreads = 512;
+
+// Grid (frame, chunk of kFlagChunk points): appends each point of the chunk with
+// |E|^2 below tau^2 times the frame's scale to list[] as {output row, frame}.
+// The counts behind the scale are exact integers, so the threshold and the set
+// of points are deterministic.
+__global__ void __launch_bounds__(kFlagThreads)
+    grid_flag_kernel(const GridFrame* __restrict__ frames, const double* __restrict__ out,
+                     const float* __restrict__ scale, float tau2, int64_t* __restrict__ list,
+                     int* __restrict__ count) {
+  __shared__ int part[kFlagThreads / 32 + 1];
+  const int64_t po = frames[blockIdx.x].point_off, P = frames[blockIdx.x].n_points;
+  const float thr = __fmul_rn(tau2, scale[blockIdx.x]);
+  constexpr int kPer = kFlagChunk / kFlagThreads;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int64_t i0 = static_cast<int64_t>(blockIdx.y) * kFlagChunk; i0 < P;
+       i0 += static_cast<int64_t>(gridDim.y) * kFlagChunk) {
+    const int64_t i1 = min(P, i0 + kFlagChunk);
+    // the chunk's points below the threshold, in thread order (point i0 + t +
+    // kFlagThreads * k belongs to thread t), appended as one contiguous block
+    unsigned mask = 0;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const int64_t i = i0 + threadIdx.x + int64_t(k) * kFlagThreads;
+      if (i < i1 && field_norm2(out + 3 * (po + i)) < thr) mask |= 1u << k;
+    }
+    if (!__syncthreads_or(mask != 0)) continue;
+    const int mine = __popc(mask);
     int incl = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int v = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += v;
     }
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
-    if (total == 0) {
-      if (lane == 0) scale_s = 0.f;  // no finite value: nothing to refine
-    } else {
-      const int rank = (total - 1) / 2;
-      const unsigned passed = __ballot_sync(0xffffffffu, incl > rank);
-      if (lane == __ffs(passed) - 1) {
-        int cum = incl - mine, t = lane * kPerLane;
-        while (cum + part[t] <= rank) cum += part[t++];
-        int b = t * kBinsPerThread;
-        while (cum + hs[b] <= rank) cum += hs[b++];
-        scale_s = __uint_as_float(static_cast<uint32_t>(b) << 19);
+    if (lane == 31) part[warp] = incl;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int run = 0;
+      for (int w = 0; w < kFlagThreads / 32; ++w) {
+        const int c = part[w];
+        part[w] = run;
+        run += c;
       }
+      part[kFlagThreads / 32] = atomicAdd(count, run);
     }
-  }
-  __syncthreads();
-  // This CTA's points below the threshold, in thread order (point i0 + t +
-  // kFlagThreads * k belongs to thread t), appended as one contiguous block.
-  const float thr = __fmul_rn(tau2, scale_s);
-  constexpr int kPer = kFlagChunk / kFlagThreads;
-  unsigned mask = 0;
-  int mine = 0;
+    __syncthreads();
+    int k_out = part[kFlagThreads / 32] + part[warp] + incl - mine;
 #pragma unroll
-  for (int k = 0; k < kPer; ++k) {
-    const int64_t i = i0 + threadIdx.x + int64_t(k) * kFlagThreads;
-    if (i < i1 && field_norm2(out + 3 * (po + i)) < thr) {
-      mask |= 1u << k;
-      ++mine;
-    }
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int incl = mine;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += v;
-  }
-  if (lane == 31) part[warp] = incl;  // part[] is free again: the scale is known
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int run = 0;
-    for (int w = 0; w < kFlagThreads / 32; ++w) {
-      const int c = part[w];
-      part[w] = run;
-      run += c;
-    }
-    part[kFlagThreads / 32] = run ? atomicAdd(count, run) : 0;
-  }
-  __syncthreads();
-  int k_out = part[kFlagThreads / 32] + part[warp] + incl - mine;
-#pragma unroll
-  for (int k = 0; k < kPer; ++k) {
-    if (mask & (1u << k)) {
-      list[2 * k_out] = po + i0 + threadIdx.x + int64_t(k) * kFlagThreads;
-      list[2 * k_out + 1] = blockIdx.x;
-      ++k_out;
+    for (int k = 0; k < kPer; ++k) {
+      if (mask & (1u << k)) {
+        list[2 * static_cast<int64_t>(k_out)] = po + i0 + threadIdx.x + int64_t(k) * kFlagThreads;
+        list[2 * static_cast<int64_t>(k_out) + 1] = blockIdx.x;
+        ++k_out;
+      }
     }
   }
 }
@@ -678,13 +1104,14 @@ __device__ __forceinline__ void df_add(float& h, float& l, float bh, float bl) {
 }
 
 // Recomputes the listed points in double-float arithmetic: one CTA per point
-// at a time, the frame's charges (double-float records, pack_df_kernel) split
-// over the threads.  Each thread keeps two independent sums (its even and odd
-// charges), so two dependent double-float chains are in flight; the two are
-// added at the end and the threads' sums combined by a fixed tree.
+// at a time, the frame's charges (double-float records of prep_kernel) split
+// over the threads.  A launch has few points, so what counts is one point's
+// latency: a thread loads the next two charges while it evaluates two, into
+// independent sums, which are added at the end; the threads' sums are combined
+// by a fixed tree.
 template <bool CLAMP>
-__global__ void __launch_bounds__(kRefineThreads)
-    grid_refine_kernel(const int64_t* __restrict__ desc, const int64_t* __restrict__ list,
+__global__ void __launch_bounds__(kRefineThreads, 2)
+    grid_refine_kernel(const GridFrame* __restrict__ frames, const int64_t* __restrict__ list,
                        const int* __restrict__ count, const double* __restrict__ points,
                        const float4* __restrict__ dfq, double* __restrict__ out) {
   __shared__ float red[kRefineThreads / 32][6];
@@ -693,7 +1120,9 @@ __global__ void __launch_bounds__(kRefineThreads)
   for (int e = blockIdx.x; e < n_list; e += gridDim.x) {
     const int64_t row = list[2 * e];
     const int64_t f = list[2 * e + 1];
-    const int64_t co = desc[4 * f], n = desc[4 * f + 1];
+    const int64_t co = frames[f].charge_off;
+    const int n = frames[f].n_charges;
+    const float4* src = dfq + 2 * co;
     float ph[3], pl[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -702,16 +1131,27 @@ __global__ void __launch_bounds__(kRefineThreads)
     }
     float sh[3] = {0.f, 0.f, 0.f}, sl[3] = {0.f, 0.f, 0.f};
     float th[3] = {0.f, 0.f, 0.f}, tl[3] = {0.f, 0.f, 0.f};
-    int64_t j = threadIdx.x;
-    for (; j + kRefineThreads < n; j += 2 * kRefineThreads) {
-      const float4 hi0 = dfq[2 * (co + j)], lo0 = dfq[2 * (co + j) + 1];
-      const float4 hi1 = dfq[2 * (co + j + kRefineThreads)], lo1 = dfq[2 * (co + j + kRefineThreads) + 1];
-      df_field_term<CLAMP>(ph, pl, hi0, lo0, sh, sl);
-      df_field_term<CLAMP>(ph, pl, hi1, lo1, th, tl);
-    }
-    if (j < n) {
-      const float4 hi0 = dfq[2 * (co + j)], lo0 = dfq[2 * (co + j) + 1];
-      df_field_term<CLAMP>(ph, pl, hi0, lo0, sh, sl);
+    // a charge past the end: zero charge 1 A from the point (its term is exactly 0)
+    auto load = [&](int j, float4& hi, float4& lo) {
+      if (j < n) {
+        hi = src[2 * static_cast<int64_t>(j)];
+        lo = src[2 * static_cast<int64_t>(j) + 1];
+      } else {
+        hi = make_float4(__fadd_rn(ph[0], 1.f), ph[1], ph[2], 0.f);
+        lo = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    };
+    int j = threadIdx.x;
+    float4 h0, l0, h1, l1;
+    load(j, h0, l0);
+    load(j + kRefineThreads, h1, l1);
+    while (j < n) {
+      const float4 a0 = h0, b0 = l0, a1 = h1, b1 = l1;
+      j += 2 * kRefineThreads;
+      load(j, h0, l0);
+      load(j + kRefineThreads, h1, l1);
+      df_field_term<CLAMP>(ph, pl, a0, b0, sh, sl);
+      df_field_term<CLAMP>(ph, pl, a1, b1, th, tl);
     }
 #pragma unroll
     for (int k = 0; k < 3; ++k) df_add(sh[k], sl[k], th[k], tl[k]);
@@ -741,35 +1181,87 @@ __global__ void __launch_bounds__(kRefineThreads)
   }
 }
 
-// Charges as double-float records {xh, yh, zh, qh} {xl, yl, zl, ql}.
-__global__ void pack_df_kernel(int64_t n, const double* __restrict__ x, const double* __restrict__ q,
-                               float4* __restrict__ out) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const double v[4] = {x[3 * i], x[3 * i + 1], x[3 * i + 2], q[i]};
-    out[2 * i] = make_float4(dbl_hi_float(v[0]), dbl_hi_float(v[1]), dbl_hi_float(v[2]),
-                             dbl_hi_float(v[3]));
-    out[2 * i + 1] = make_float4(dbl_lo_float(v[0]), dbl_lo_float(v[1]), dbl_lo_float(v[2]),
-                                 dbl_lo_float(v[3]));
-  }
+constexpr int kPrepThreads = 256;
+constexpr int kPrepCharges = 1024;   // charges per preparation block
+constexpr int kMaxStride = 16384;    // longest lattice stride looked for
+
+__device__ __forceinline__ bool same_yz(const double* a, const double* b, bool f32) {
+  if (f32)  // the FP32C kernels see the FP32 images
+    return __float_as_uint(narrow(a[1])) == __float_as_uint(narrow(b[1])) &&
+           __float_as_uint(narrow(a[2])) == __float_as_uint(narrow(b[2]));
+  return __double_as_longlong(a[1]) == __double_as_longlong(b[1]) &&
+         __double_as_longlong(a[2]) == __double_as_longlong(b[2]);
 }
 
-__global__ void pack_dup_f32_kernel(int64_t n, int64_t n_pad, const double* __restrict__ x,
-                                    const double* __restrict__ q, ChargeDup* __restrict__ out) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_pad;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    float v[4] = {1.0e4f, 1.0e4f, 1.0e4f, 0.f};  // zero charge far outside any box
-    if (i < n) {
-      v[0] = static_cast<float>(x[3 * i]);
-      v[1] = static_cast<float>(x[3 * i + 1]);
-      v[2] = static_cast<float>(x[3 * i + 2]);
-      v[3] = static_cast<float>(q[i]);
+// Preparation, one launch: blocks [0, n_charge_blocks) pack the charges (FP32C:
+// every component duplicated; FP64: Charge64) and, for the refinement, their
+// double-float records {xh, yh, zh, qh} {xl, yl, zl, ql}; the others look for the
+// frames' lattice strides, kGridPrepPoints points each.  A frame's stride is the
+// first index whose (y, z) equal those of point 0; it holds if every point's
+// (y, z) equal those one stride earlier.  stride[f] is written by the frame's
+// first block, broken[f] (zeroed by the caller) by any block that finds a
+// difference.
+template <int PREC, bool DF>
+__global__ void __launch_bounds__(kPrepThreads)
+    prep_kernel(int64_t n, const double* __restrict__ x, const double* __restrict__ q,
+                void* __restrict__ packed, float4* __restrict__ dfq, int n_charge_blocks,
+                const GridFrame* __restrict__ frames, int n_frames, const GridFrame one,
+                const double* __restrict__ points, int min_rows, int* __restrict__ stride, int* __restrict__ broken) {
+  if (static_cast<int>(blockIdx.x) < n_charge_blocks) {
+    const int64_t i0 = static_cast<int64_t>(blockIdx.x) * kPrepCharges;
+    const int64_t i1 = min(n, i0 + kPrepCharges);
+    for (int64_t i = i0 + threadIdx.x; i < i1; i += kPrepThreads) {
+      const double v[4] = {x[3 * i], x[3 * i + 1], x[3 * i + 2], q[i]};
+      if constexpr (PREC == kFP32C) {
+        ChargeDup c;
+        c.xy = make_ulonglong2(dup2(narrow(v[0])), dup2(narrow(v[1])));
+        c.zq = make_ulonglong2(dup2(narrow(v[2])), dup2(narrow(v[3])));
+        static_cast<ChargeDup*>(packed)[i] = c;
+        if constexpr (DF) {
+          dfq[2 * i] = make_float4(dbl_hi_float(v[0]), dbl_hi_float(v[1]), dbl_hi_float(v[2]),
+                                   dbl_hi_float(v[3]));
+          dfq[2 * i + 1] = make_float4(dbl_lo_float(v[0]), dbl_lo_float(v[1]), dbl_lo_float(v[2]),
+                                       dbl_lo_float(v[3]));
+        }
+      } else {
+        static_cast<Charge64*>(packed)[i] = Charge64{v[0], v[1], v[2], v[3]};
+      }
     }
-    ChargeDup c;
-    c.xy = make_ulonglong2(dup2(v[0]), dup2(v[1]));
-    c.zq = make_ulonglong2(dup2(v[2]), dup2(v[3]));
-    out[i] = c;
+    return;
   }
+  const int b = static_cast<int>(blockIdx.x) - n_charge_blocks;
+  int f;
+  const GridFrame fr = load_frame<offsetof(GridFrame, prep_base)>(frames, n_frames, one, b, &f);
+  const int part = b - fr.prep_base;
+  const int P = fr.n_points;
+  const double* pts = points + 3 * fr.point_off;
+  constexpr bool kF32 = PREC == kFP32C;
+  __shared__ int s_stride;
+  if (threadIdx.x == 0) s_stride = INT_MAX;
+  __syncthreads();
+  const int limit = min(P / min_rows, kMaxStride);  // at least min_rows rows
+  constexpr int kLook = kPrepThreads * 4;
+  for (int i0 = 1; i0 <= limit; i0 += kLook) {
+    int hit = INT_MAX;
+#pragma unroll
+    for (int k = 3; k >= 0; --k) {
+      const int i = i0 + k * kPrepThreads + static_cast<int>(threadIdx.x);
+      if (i <= limit && i < P && same_yz(pts, pts + 3 * static_cast<int64_t>(i), kF32)) hit = i;
+    }
+    if (hit != INT_MAX) atomicMin(&s_stride, hit);
+    if (__syncthreads_or(hit != INT_MAX)) break;
+  }
+  const int S = s_stride;
+  const bool mesh = S != INT_MAX && P % S == 0;
+  if (part == 0 && threadIdx.x == 0) stride[f] = mesh ? S : 0;
+  if (!mesh) return;
+  const int64_t j0 = max(static_cast<int64_t>(part) * kGridPrepPoints, static_cast<int64_t>(S));
+  const int64_t j1 = min(static_cast<int64_t>(P), static_cast<int64_t>(part + 1) * kGridPrepPoints);
+  bool bad = false;
+#pragma unroll 4
+  for (int64_t j = j0 + threadIdx.x; j < j1; j += kPrepThreads)
+    bad |= !same_yz(pts + 3 * j, pts + 3 * (j - S), kF32);
+  if (__syncthreads_or(bad) && threadIdx.x == 0) broken[f] = 1;
 }
 
 __global__ void pack_f64_kernel(int64_t n, int64_t n_pad, const double* __restrict__ x,
@@ -790,136 +1282,179 @@ __global__ void pack_f64_kernel(int64_t n, int64_t n_pad, const double* __restri
   }
 }
 
-template <int PREC, int KIND, int PPT>
-cudaError_t launch_grid_t(int clamp, int n_items, const GridItem* items, const void* packed,
-                          const double* points, double* out, double* partial, int* status,
-                          cudaStream_t s) {
-  // same carveout as the streamline engine, so both fit on one SM
-  cudaFuncSetAttribute(grid_kernel<PREC, KIND, true, PPT>,
-                       cudaFuncAttributePreferredSharedMemoryCarveout,
-                       cudaSharedmemCarveoutMaxShared);
-  cudaFuncSetAttribute(grid_kernel<PREC, KIND, false, PPT>,
-                       cudaFuncAttributePreferredSharedMemoryCarveout,
-                       cudaSharedmemCarveoutMaxShared);
-  if (clamp)
-    grid_kernel<PREC, KIND, true, PPT>
-        <<<n_items, kGridThreads, 0, s>>>(items, packed, points, out, partial, status);
-  else
-    grid_kernel<PREC, KIND, false, PPT>
-        <<<n_items, kGridThreads, 0, s>>>(items, packed, points, out, partial, status);
+// Layout of GridLaunch::zeroed.
+struct Zeroed {
+  int *stride, *broken, *done, *count, *hist;
+  float* scale;
+  Zeroed(int* base, int n_frames)
+      : stride(base), broken(base + n_frames), done(base + 2 * n_frames), count(base + 4 * n_frames),
+        hist(base + ((4 * n_frames + 1 + 3) & ~3)), scale(reinterpret_cast<float*>(base + 3 * n_frames)) {}
+};
+
+template <int PREC, int KIND, bool CLAMP, int PPT>
+cudaError_t launch_grid_c(const GridLaunch& g, cudaStream_t s) {
+  const Zeroed z(g.zeroed, g.n_frames);
+  const bool refine = g.tau > 0.0;
+  const int charge_blocks = static_cast<int>((g.n_charges + kPrepCharges - 1) / kPrepCharges);
+  float4* dfq = static_cast<float4*>(g.dfq);
+  const int* stride = g.n_prep > 0 ? z.stride : nullptr;  // null: no frame is looked at for a mesh
+  if (charge_blocks + g.n_prep > 0) {
+    if (refine && PREC == kFP32C)
+      prep_kernel<PREC, PREC == kFP32C><<<charge_blocks + g.n_prep, kPrepThreads, 0, s>>>(
+          g.n_charges, g.x, g.q, g.packed, dfq, charge_blocks, g.frames, g.n_frames, g.one, g.points, PPT, z.stride,
+          z.broken);
+    else
+      prep_kernel<PREC, false><<<charge_blocks + g.n_prep, kPrepThreads, 0, s>>>(
+          g.n_charges, g.x, g.q, g.packed, dfq, charge_blocks, g.frames, g.n_frames, g.one, g.points, PPT, z.stride,
+          z.broken);
+  }
+  if (g.few_items > 0)
+    grid_few_kernel<PREC, KIND, CLAMP, PPT>
+        <<<g.few_items, kGridThreads, 0, s>>>(g.frames, g.n_frames, g.one, g.packed, g.points, g.out, g.partial);
+  if (g.n_items > g.few_items) {
+    // same carveout as the streamline engine, so both fit on one SM
+    cudaFuncSetAttribute(grid_kernel<PREC, KIND, CLAMP, PPT>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                         cudaSharedmemCarveoutMaxShared);
+    grid_kernel<PREC, KIND, CLAMP, PPT><<<g.n_items - g.few_items, kGridThreads, 0, s>>>(
+        g.frames, g.n_frames, g.one, g.few_items, stride, z.broken, g.packed, g.points, g.out, g.partial, g.status);
+  }
+  // Eight lanes per point where that is shorter: FP64 additions per scheduler with
+  // one thread per point against eight.
+  const double splits = double(g.n_items) / std::max(g.n_tiles, 1);
+  const double warps = double(g.n_tiles) * PPT * (kGridThreads / 32) / (4.0 * std::max(g.num_sms, 1));
+  const bool lanes = std::max(1.0, 8.0 * warps) * (splits / 8.0 + 3.0) < std::max(1.0, warps) * splits;
+  auto final = [&](auto hist, auto ln) {
+    constexpr int L = decltype(ln)::value;
+    grid_final_kernel<PREC, KIND, PPT, decltype(hist)::value, L><<<g.n_tiles * PPT * L, kGridThreads, 0, s>>>(
+        g.frames, g.n_frames, g.one, stride, z.broken, g.partial, g.out, z.hist, z.done, z.scale);
+  };
+  auto final_lanes = [&](auto hist) {
+    if (lanes)
+      final(hist, std::integral_constant<int, kSumLanes>{});
+    else
+      final(hist, std::integral_constant<int, 1>{});
+  };
+  if (refine) {
+    if constexpr (KIND == kField && PREC == kFP32C) {
+      final_lanes(std::true_type{});
+      const dim3 fgrid(g.n_frames, std::min((g.max_points - 1) / kFlagChunk + 1, 65535));
+      grid_flag_kernel<<<fgrid, kFlagThreads, 0, s>>>(g.frames, g.out, z.scale,
+                                                      static_cast<float>(g.tau * g.tau), g.list, z.count);
+      grid_refine_kernel<CLAMP><<<std::max(g.num_sms, 1) * 4, kRefineThreads, 0, s>>>(
+          g.frames, g.list, z.count, g.points, dfq, g.out);
+    }
+  } else if (g.partial) {
+    final_lanes(std::false_type{});
+  }
   return cudaGetLastError();
 }
 
-template <int PREC, int KIND>
-cudaError_t launch_grid_p(int clamp, int ppt, int n_items, const GridItem* items,
-                          const void* packed, const double* points, double* out, double* partial,
-                          int* status, cudaStream_t s) {
-  return ppt == 8 ? launch_grid_t<PREC, KIND, 8>(clamp, n_items, items, packed, points, out,
-                                                 partial, status, s)
-                  : launch_grid_t<PREC, KIND, 4>(clamp, n_items, items, packed, points, out,
-                                                 partial, status, s);
+template <int PREC, int KIND, int PPT>
+cudaError_t launch_grid_k(const GridLaunch& g, cudaStream_t s) {
+  if constexpr (KIND == kField)
+    if (g.clamp) return launch_grid_c<PREC, KIND, true, PPT>(g, s);
+  return launch_grid_c<PREC, KIND, false, PPT>(g, s);
 }
 
-template <int PREC, int KIND, int PPT>
-cudaError_t preload_t(int clamp) {
+template <int PREC, int KIND, bool CLAMP, int PPT>
+cudaError_t preload_c() {
   cudaFuncAttributes a;
-  return clamp ? cudaFuncGetAttributes(&a, grid_kernel<PREC, KIND, true, PPT>)
-               : cudaFuncGetAttributes(&a, grid_kernel<PREC, KIND, false, PPT>);
+  cudaError_t e = cudaFuncGetAttributes(&a, grid_kernel<PREC, KIND, CLAMP, PPT>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, grid_few_kernel<PREC, KIND, CLAMP, PPT>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, prep_kernel<PREC, false>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, grid_final_kernel<PREC, KIND, PPT, false, 1>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, grid_final_kernel<PREC, KIND, PPT, false, kSumLanes>);
+  if constexpr (KIND == kField && PREC == kFP32C) {
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, prep_kernel<PREC, true>);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, grid_final_kernel<PREC, KIND, PPT, true, 1>);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, grid_final_kernel<PREC, KIND, PPT, true, kSumLanes>);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, grid_flag_kernel);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, grid_refine_kernel<CLAMP>);
+  }
+  return e;
+}
+
+// Calls f with the launch's (precision, kind, points per thread) as constants.
+template <typename F>
+cudaError_t with_form(int prec, int kind, int ppt, F f) {
+  auto by_ppt = [&](auto p, auto k) {
+    return ppt == 8 ? f(p, k, std::integral_constant<int, 8>{}) : f(p, k, std::integral_constant<int, 4>{});
+  };
+  auto by_kind = [&](auto p) {
+    return kind == kField ? by_ppt(p, std::integral_constant<int, kField>{})
+                          : by_ppt(p, std::integral_constant<int, kEsp>{});
+  };
+  return prec == kFP32C ? by_kind(std::integral_constant<int, kFP32C>{})
+                        : by_kind(std::integral_constant<int, kFP64>{});
 }
 
 }  // namespace
 
-cudaError_t launch_pack_charges(int prec, int64_t n, int64_t n_pad, const double* x,
-                                const double* q, void* packed, cudaStream_t s) {
-  if (n_pad <= 0) return cudaSuccess;
-  const int blocks = static_cast<int>(std::min<int64_t>((n_pad + 255) / 256, 4096));
-  if (prec == kFP32C)
-    pack_dup_f32_kernel<<<blocks, 256, 0, s>>>(n, n_pad, x, q, static_cast<ChargeDup*>(packed));
-  else
-    pack_f64_kernel<<<blocks, 256, 0, s>>>(n, n_pad, x, q, static_cast<Charge64*>(packed));
-  return cudaGetLastError();
+namespace {
+struct PointSizes {
+  int64_t charges, units, results;
+  explicit PointSizes(const GridLaunch& g) {
+    const int64_t most = (g.one.n_split + kPointCtas - 1) / kPointCtas;
+    charges = most * g.one.chunk;
+    units = most * g.one.n_points * ((int64_t(g.one.chunk) + kKahanRun - 1) / kKahanRun);
+    results = int64_t(g.one.n_split) * g.one.n_points * (g.kind == kField ? 3 : 1);
+  }
+};
+}  // namespace
+
+bool grid_point_fits(const GridLaunch& g) {
+  if (g.n_frames != 1 || g.prec != kFP32C || !g.one.few || g.tau > 0.0) return false;
+  const PointSizes n(g);
+  return n.charges <= kPointCharges && n.units <= kPointUnits && n.results <= kPointResults;
 }
 
-cudaError_t launch_grid(int prec, int kind, int clamp, int ppt, int n_items, const GridItem* items,
-                        const void* packed, const double* points, double* out, double* partial,
-                        int* status, cudaStream_t s) {
-  if (n_items <= 0) return cudaSuccess;
-  if (prec == kFP32C) {
-    return kind == kField ? launch_grid_p<kFP32C, kField>(clamp, ppt, n_items, items, packed, points,
-                                                         out, partial, status, s)
-                          : launch_grid_p<kFP32C, kEsp>(0, ppt, n_items, items, packed, points, out,
-                                                       partial, status, s);
+cudaError_t launch_grid_point(const GridLaunch& g, cudaStream_t s) {
+  const PointSizes n(g);
+  const size_t smem = size_t(n.charges) * sizeof(float4) + size_t(n.results) * sizeof(double) +
+                      size_t(n.units) * (g.kind == kField ? 3 : 1) * sizeof(float);
+  auto run = [&](auto kernel) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
+    kernel<<<kPointCtas, kPointThreads, smem, s>>>(g.one, g.points, g.x, g.q, g.out);
+    return cudaGetLastError();
+  };
+  if (g.kind != kField) return run(grid_point_kernel<kEsp, false>);
+  return g.clamp ? run(grid_point_kernel<kField, true>) : run(grid_point_kernel<kField, false>);
+}
+
+size_t grid_slot_doubles(int kind, int ppt) { return size_t(kGridThreads) * ppt * (kind == kField ? 3 : 1); }
+
+size_t grid_zero_ints(int n_frames, bool refine) {
+  return size_t((4 * n_frames + 1 + 3) & ~3) + (refine ? size_t(n_frames) * kMagBins : 0);
+}
+
+cudaError_t launch_grid(const GridLaunch& g, cudaStream_t s) {
+  if (g.n_items <= 0) return cudaSuccess;
+  if (g.n_prep > 0 || g.tau > 0.0) {
+    const cudaError_t e =
+        cudaMemsetAsync(g.zeroed, 0, grid_zero_ints(g.n_frames, g.tau > 0.0) * sizeof(int), s);
+    if (e != cudaSuccess) return e;
   }
-  return kind == kField ? launch_grid_p<kFP64, kField>(clamp, ppt, n_items, items, packed, points,
-                                                      out, partial, status, s)
-                        : launch_grid_p<kFP64, kEsp>(0, ppt, n_items, items, packed, points, out,
-                                                    partial, status, s);
+  return with_form(g.prec, g.kind, g.ppt, [&](auto p, auto k, auto t) {
+    return launch_grid_k<decltype(p)::value, decltype(k)::value, decltype(t)::value>(g, s);
+  });
 }
 
 cudaError_t preload_grid_kernels(int prec, int kind, int clamp, int ppt) {
-  cudaError_t e;
-  if (prec == kFP32C) {
-    if (kind == kField)
-      e = ppt == 8 ? preload_t<kFP32C, kField, 8>(clamp) : preload_t<kFP32C, kField, 4>(clamp);
-    else
-      e = ppt == 8 ? preload_t<kFP32C, kEsp, 8>(0) : preload_t<kFP32C, kEsp, 4>(0);
-  } else {
-    if (kind == kField)
-      e = ppt == 8 ? preload_t<kFP64, kField, 8>(clamp) : preload_t<kFP64, kField, 4>(clamp);
-    else
-      e = ppt == 8 ? preload_t<kFP64, kEsp, 8>(0) : preload_t<kFP64, kEsp, 4>(0);
-  }
-  if (e != cudaSuccess) return e;
-  cudaFuncAttributes a;
-  e = kind == kField ? cudaFuncGetAttributes(&a, grid_final_kernel<kField>)
-                     : cudaFuncGetAttributes(&a, grid_final_kernel<kEsp>);
-  if (e != cudaSuccess) return e;
-  return prec == kFP32C ? cudaFuncGetAttributes(&a, pack_dup_f32_kernel)
-                        : cudaFuncGetAttributes(&a, pack_f64_kernel);
+  return with_form(prec, kind, ppt, [&](auto p, auto k, auto t) {
+    constexpr int P = decltype(p)::value, K = decltype(k)::value, T = decltype(t)::value;
+    if constexpr (K == kField)
+      if (clamp) return preload_c<P, K, true, T>();
+    return preload_c<P, K, false, T>();
+  });
 }
 
-cudaError_t launch_grid_refine(int n_frames, int64_t n_charges, int64_t max_points,
-                               const int64_t* desc, const double* points, const double* x,
-                               const double* q, double* out, int clamp, double tau, int64_t* list,
-                               int* count, int* hist, void* df_charges, int num_sms, cudaStream_t s) {
-  if (n_frames <= 0 || n_charges <= 0 || max_points <= 0 || !(tau > 0.0)) return cudaSuccess;
-  cudaError_t e = cudaMemsetAsync(count, 0, sizeof(int), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(hist, 0, size_t(n_frames) * kMagBins * sizeof(int), s);
-  if (e != cudaSuccess) return e;
-  float4* dfq = static_cast<float4*>(df_charges);
-  const int pack_blocks = static_cast<int>(std::min<int64_t>((n_charges + 255) / 256, 4096));
-  pack_df_kernel<<<pack_blocks, 256, 0, s>>>(n_charges, x, q, dfq);
-  const dim3 fgrid(n_frames, static_cast<unsigned>((max_points + kFlagChunk - 1) / kFlagChunk));
-  grid_mag_hist_kernel<<<fgrid, kFlagThreads, 0, s>>>(desc, out, hist);
-  const float tau2 = static_cast<float>(tau * tau);
-  grid_flag_kernel<<<fgrid, kFlagThreads, 0, s>>>(desc, out, hist, tau2, list, count);
-  const int ctas = std::max(num_sms, 1) * 8;
-  if (clamp)
-    grid_refine_kernel<true><<<ctas, kRefineThreads, 0, s>>>(desc, list, count, points, dfq, out);
-  else
-    grid_refine_kernel<false><<<ctas, kRefineThreads, 0, s>>>(desc, list, count, points, dfq, out);
-  return cudaGetLastError();
-}
-
-int64_t grid_refine_hist_ints(int n_frames) { return int64_t(std::max(n_frames, 1)) * kMagBins; }
-
-cudaError_t preload_grid_refine() {
-  cudaFuncAttributes a;
-  cudaError_t e = cudaFuncGetAttributes(&a, grid_flag_kernel);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, grid_mag_hist_kernel);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, grid_refine_kernel<true>);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, grid_refine_kernel<false>);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, pack_df_kernel);
-  return e;
-}
-
-cudaError_t launch_grid_final(int kind, int n_final, const GridFinal* fin, const double* partial,
-                              double* out, cudaStream_t s) {
-  if (n_final <= 0) return cudaSuccess;
-  if (kind == kField)
-    grid_final_kernel<kField><<<n_final, 256, 0, s>>>(fin, partial, out);
-  else
-    grid_final_kernel<kEsp><<<n_final, 256, 0, s>>>(fin, partial, out);
+cudaError_t launch_pack_f64(int64_t n, int64_t n_pad, const double* x, const double* q, void* packed,
+                            cudaStream_t s) {
+  if (n_pad <= 0) return cudaSuccess;
+  const int blocks = static_cast<int>(std::min<int64_t>((n_pad + 255) / 256, 4096));
+  pack_f64_kernel<<<blocks, 256, 0, s>>>(n, n_pad, x, q, static_cast<Charge64*>(packed));
   return cudaGetLastError();
 }
 

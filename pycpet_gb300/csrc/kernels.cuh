@@ -33,61 +33,82 @@ static_assert(sizeof(Dipole64) == 48, "Dipole64 layout");
 enum Source : int { kCharges = 0, kDipoles = 1 };
 // FP32C uses float4 {x, y, z, q}.
 
-// One CTA of the grid kernel: a tile of up to kGridTilePts points of one frame
-// against a contiguous range of that frame's charges.
-struct GridItem {
-  int64_t charge_off;  // first packed charge of the frame
-  int64_t point_off;   // first point of the frame (points / output rows)
-  int32_t p_begin;     // first point of this tile inside the frame
-  int32_t p_count;     // points in this tile (<= kGridThreads * points per thread)
-  int32_t n_begin;     // first charge of this item inside the frame
-  int32_t n_count;     // charges of this item
-  int32_t slot;        // partial-sum slot (>= 0), or -1 to write the final value
-  int32_t pad;
-};
-static_assert(sizeof(GridItem) == 40, "GridItem layout");
-
-// Reduction of the partial sums of one point tile over its charge splits.
-struct GridFinal {
-  int64_t out_row;     // first output row (frame point_off + p_begin)
-  int32_t p_count;
-  int32_t slot_base;   // partial slots slot_base .. slot_base + n_split - 1
-  int32_t n_split;
-  int32_t pad;
-};
-static_assert(sizeof(GridFinal) == 24, "GridFinal layout");
-
 constexpr int kGridThreads = 128;
-constexpr int kGridMaxPPT = 8;                              // points per thread: 4 or 8
-constexpr int kGridSlotPts = kGridThreads * kGridMaxPPT;    // stride of a partial-sum slot
+// A frame of at most this many points goes to the few-points kernel.  FP32C: 30
+// points x 50 frames 476 -> 206 us, but 200 points x 20,000 charges 27 -> 52 us
+// (potential; its charges come from L2 there); FP64, where a thread per point
+// leaves most of the slow pipe to padding, 200 points 481 -> 236 us.
+constexpr int kGridFewPoints = 256;
+constexpr int kGridFewPointsFp32 = 32;
+// Launches with fewer pairs than this don't look for meshes: the look costs about
+// 5 us, a quarter of so small a launch's kernel less.
+constexpr double kGridMeshPairsFp32 = 2.0e7, kGridMeshPairsFp64 = 1.0e6;
+
+// One frame of a grid launch (device table, sorted by charge chunk, longest
+// first).  Its points are cut into tiles of kGridThreads threads with 4 or 8
+// points each, its charges into n_split chunks; a CTA takes one tile and one
+// chunk (item = split * n_tiles + tile within the frame).
+struct GridFrame {
+  int64_t charge_off;   // first charge of the frame in x / q / packed
+  int64_t point_off;    // first point of the frame (points / output rows)
+  int32_t n_charges;
+  int32_t n_points;
+  int32_t n_tiles;
+  int32_t n_split;
+  int32_t chunk;        // charges per split (the last may have fewer)
+  int32_t slot_base;    // partial sums of (split, tile): slot_base + item; -1: n_split == 1, none
+  int32_t item_base;    // items, tiles and preparation blocks of the frames before this one
+  int32_t tile_base;
+  int32_t prep_base;
+  int32_t few;          // 1: few-points kernel (one tile)
+  int32_t pad[2];
+};
+static_assert(sizeof(GridFrame) == 64, "GridFrame layout");
+
+// A grid launch.  Scratch (device): packed 32 bytes per charge; partial
+// n_slots * grid_slot_doubles(kind, ppt); lattice and, for the refinement, list
+// (2 int64 per point) and dfq (32 bytes per charge); zeroed: grid_zero_ints()
+// ints, cleared by launch_grid.
+struct GridLaunch {
+  int prec, kind, clamp, ppt;
+  int n_frames;
+  const GridFrame* frames;    // device
+  GridFrame one;              // the frame itself when n_frames == 1 (saves its kernels the table's loads)
+  int n_items;                // items of all frames
+  int n_tiles;
+  int n_prep;                 // preparation blocks of all frames (0: no look for meshes)
+  int n_few;                  // frames with few != 0 (they come first: their items precede the others)
+  int few_items;              // items of those frames
+  int64_t n_charges;          // extent of x / q
+  int max_points;             // largest frame
+  const double *points, *x, *q;
+  double* out;
+  void* packed;
+  double* partial;
+  int* zeroed;
+  int* status;
+  double tau;                 // refinement threshold; 0: no refinement
+  int64_t* list;
+  void* dfq;
+  int num_sms;
+};
+constexpr int kGridPrepPoints = 1024;  // points per preparation block of a frame
+size_t grid_slot_doubles(int kind, int ppt);
+size_t grid_zero_ints(int n_frames, bool refine);
 
 // grid.cu
-// Packs x[n][3], q[n] for the grid kernels (32-byte records: Charge64, or the
-// FP32C record with every component duplicated) and fills [n, n_pad) with zero
-// charges placed far outside any box (they contribute exactly zero).
-cudaError_t launch_pack_charges(int prec, int64_t n, int64_t n_pad, const double* x,
-                                const double* q, void* packed, cudaStream_t s);
-cudaError_t launch_grid(int prec, int kind, int clamp, int ppt, int n_items, const GridItem* items,
-                        const void* packed, const double* points, double* out,
-                        double* partial, int* status, cudaStream_t s);
+// A launch of one frame of so few (point, run) units that one CTA does all of it
+// in one kernel, without scratch (g.one, points, x, q, out set).
+bool grid_point_fits(const GridLaunch& g);
+cudaError_t launch_grid_point(const GridLaunch& g, cudaStream_t s);
+cudaError_t launch_grid(const GridLaunch& g, cudaStream_t s);
 // Loads the module code of the grid kernels (before a graph capture).
 cudaError_t preload_grid_kernels(int prec, int kind, int clamp, int ppt);
-cudaError_t launch_grid_final(int kind, int n_final, const GridFinal* fin,
-                              const double* partial, double* out, cudaStream_t s);
-
-// FP32C field refinement after the grid pass: points of each frame (desc rows
-// {charge_off, n, point_off, P}, device memory; max_points = the largest P)
-// whose |E| is below tau times the frame's median |E| are recomputed in
-// double-float arithmetic from x/q (n_charges of them in all).  Scratch: list
-// 2 int64 per point of the launch, count one int, hist
-// grid_refine_hist_ints(n_frames) ints (both zeroed here), df_charges 32 bytes
-// per charge.  tau <= 0: no-op.
-cudaError_t launch_grid_refine(int n_frames, int64_t n_charges, int64_t max_points,
-                               const int64_t* desc, const double* points, const double* x,
-                               const double* q, double* out, int clamp, double tau, int64_t* list,
-                               int* count, int* hist, void* df_charges, int num_sms, cudaStream_t s);
-int64_t grid_refine_hist_ints(int n_frames);
-cudaError_t preload_grid_refine();
+// Packs x[n][3], q[n] as Charge64 (the FP64 streamline layout) and fills [n,
+// n_pad) with zero charges placed far outside any box (they contribute exactly
+// zero).
+cudaError_t launch_pack_f64(int64_t n, int64_t n_pad, const double* x, const double* q, void* packed,
+                            cudaStream_t s);
 
 // topo.cu
 // One frame of a streamline launch (device table for multi-frame launches).

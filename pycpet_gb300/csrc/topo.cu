@@ -750,7 +750,7 @@ size_t topo_source_bytes(int prec, int source) {
 
 cudaError_t launch_pack_topo(int prec, int64_t n, int64_t n_pad, const double* x, const double* q,
                              void* packed, cudaStream_t s) {
-  if (prec != kFP32C) return launch_pack_charges(prec, n, n_pad, x, q, packed, s);
+  if (prec != kFP32C) return launch_pack_f64(n, n_pad, x, q, packed, s);
   if (n_pad <= 0) return cudaSuccess;
   const int blocks = static_cast<int>(std::min<int64_t>((n_pad / 2 + 255) / 256, 4096));
   pack_pairs_kernel<<<blocks, 256, 0, s>>>(n, n_pad, x, q, static_cast<float4*>(packed));
