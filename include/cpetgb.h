@@ -151,6 +151,16 @@ int cpetgb_thread_operation_batch_p(int precision, int n_lines, int n_charges,
 int cpetgb_compute_esp_grid_p(int precision, int total_points, int n_charges, const float* x_0,
                               const float* x, const float* Q, float* ESP);
 
+/* The output rows of compute_box and compute_box_ESP
+ * (CPET/source/calculator.py:489-528, CPET/utils/calculator.py:430-475) in one
+ * call, from and to float32 / float16 HOST arrays: points[P][3], x[N][3], q[N].
+ * rows[P][6] = {x, y, z, Ex, Ey, Ez} (the r^2-clamped field); rows[P][4] =
+ * {x, y, z, phi} as IEEE binary16 bits.  Every value rounded once. */
+int cpetgb_box_field_rows(int precision, int n_points, int n_charges, const float* points,
+                          const float* x, const float* q, float* rows);
+int cpetgb_box_esp_rows(int precision, int n_points, int n_charges, const float* points,
+                        const float* x, const float* q, uint16_t* rows);
+
 /* ---- general entry points (double buffers, host or device) --------------- */
 /* Field at n_points points: points[P][3], x[N][3], q[N] -> field[P][3].
  * clamp != 0 applies compute_looped_field's r^2 >= 1e-6; clamp == 0 is calc_field. */

@@ -65,6 +65,71 @@ int cuda_fail(cudaError_t e, const char* what) {
     if (e_ != cudaSuccess) return cuda_fail(e_, what); \
   } while (0)
 
+// Pinned staging buffers of the float32 host calls: at most kStagingBytes in all per
+// process, of which kStagingIdle stay for the next calls; a call that gets none copies
+// from and to the caller's pageable arrays.  A buffer belongs to one call at a time
+// (any thread, any stream) and goes back after the call has waited for its copies.
+constexpr size_t kStagingBytes = size_t(64) << 20;
+constexpr size_t kStagingIdle = size_t(16) << 20;
+struct StagingPool {
+  std::mutex mu;
+  std::vector<std::pair<void*, size_t>> idle;
+  size_t total = 0, idle_bytes = 0;
+  void drop(size_t i) {
+    cudaFreeHost(idle[i].first);
+    total -= idle[i].second;
+    idle_bytes -= idle[i].second;
+    idle.erase(idle.begin() + static_cast<std::ptrdiff_t>(i));
+  }
+};
+StagingPool& staging_pool() {
+  static StagingPool* pool = new StagingPool();  // never destroyed: calls may outlive static destruction
+  return *pool;
+}
+
+struct Staging {
+  void* p = nullptr;
+  size_t size = size_t(1) << 18;
+  cudaStream_t stream;
+  bool waited = false;  // set once no copy to or from the buffer is in flight
+  Staging(size_t need, cudaStream_t s) : stream(s) {
+    if (need > kStagingBytes) return;
+    while (size < need) size *= 2;
+    StagingPool& pool = staging_pool();
+    std::lock_guard<std::mutex> lock(pool.mu);
+    size_t best = pool.idle.size();
+    for (size_t i = 0; i < pool.idle.size(); ++i)
+      if (pool.idle[i].second >= need && (best == pool.idle.size() || pool.idle[i].second < pool.idle[best].second))
+        best = i;
+    if (best < pool.idle.size()) {
+      p = pool.idle[best].first;
+      size = pool.idle[best].second;
+      pool.idle_bytes -= size;
+      pool.idle.erase(pool.idle.begin() + static_cast<std::ptrdiff_t>(best));
+      return;
+    }
+    while (pool.total + size > kStagingBytes && !pool.idle.empty()) pool.drop(pool.idle.size() - 1);
+    if (pool.total + size > kStagingBytes) return;
+    if (cudaHostAlloc(&p, size, cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+      return;
+    }
+    pool.total += size;
+  }
+  ~Staging() {
+    if (!p) return;
+    if (!waited) cudaStreamSynchronize(stream);
+    StagingPool& pool = staging_pool();
+    std::lock_guard<std::mutex> lock(pool.mu);
+    pool.idle.emplace_back(p, size);
+    pool.idle_bytes += size;
+    if (pool.idle_bytes > kStagingIdle) pool.drop(pool.idle.size() - 1);
+  }
+  Staging(const Staging&) = delete;
+  Staging& operator=(const Staging&) = delete;
+};
+
 Ctx* context(int* rc) {
   int dev = -1, count = 0;
   if (cudaGetDeviceCount(&count) != cudaSuccess || count <= 0) {
@@ -132,11 +197,8 @@ cudaError_t h2d(T** dst, Scratch& S, const T* src, size_t count) {
   return e;
 }
 
-// Waits for the stream and converts the device status word into a return code.
-int finish(Ctx* c, cudaStream_t s) {
-  CK(cudaStreamSynchronize(s), "stream synchronize");
-  int st = 0;
-  CK(cudaMemcpy(&st, c->status, sizeof(int), cudaMemcpyDeviceToHost), "status read");
+// Converts a status word read from the device into a return code (and clears it there).
+int status_code(Ctx* c, int st) {
   if (st != kDevOk) {
     cudaMemset(c->status, 0, sizeof(int));
     if (st == kDevWaitTimeout)
@@ -148,6 +210,14 @@ int finish(Ctx* c, cudaStream_t s) {
     return fail(CPETGB_ECUDA, "device status %d", st);
   }
   return CPETGB_OK;
+}
+
+// Waits for the stream and converts the device status word into a return code.
+int finish(Ctx* c, cudaStream_t s) {
+  CK(cudaStreamSynchronize(s), "stream synchronize");
+  int st = 0;
+  CK(cudaMemcpy(&st, c->status, sizeof(int), cudaMemcpyDeviceToHost), "status read");
+  return status_code(c, st);
 }
 
 bool valid_prec(int p) { return p == CPETGB_FP64 || p == CPETGB_FP32C; }
@@ -326,6 +396,44 @@ GridLaunch grid_launch(int kind, int prec, int clamp, int ppt, int n_frames, con
   return g;
 }
 
+// A grid launch on device arrays, its scratch from S (released after it on the stream).
+int grid_device(int kind, int prec, int clamp, int n_frames, const int64_t* desc, int64_t tot_ch,
+                const double* pts, const double* x, const double* q, double* out, const Ctx* c, Scratch& S) {
+  GridTable plan;
+  int ppt = 4, ips = 8;
+  tuned_grid_shape(prec, kind, grid_pair_evals(n_frames, desc), &ppt, &ips);
+  const int rc = plan_grid(prec, n_frames, desc, c->sms, ppt, ips, plan);
+  if (rc != CPETGB_OK) return rc;
+  GridLaunch g = grid_launch(kind, prec, clamp, ppt, n_frames, desc, plan, tot_ch, c);
+  g.points = pts;
+  g.x = x;
+  g.q = q;
+  g.out = out;
+  if (grid_point_fits(g)) {
+    CK(launch_grid_point(g, S.s), "point kernel launch");
+  } else {
+    GridFrame* d_frames = nullptr;
+    unsigned char* packed = nullptr;
+    CK(S.get(&packed, size_t(std::max<int64_t>(tot_ch, 1)) * kGridRecord), "alloc packed charges");
+    if (reinterpret_cast<uintptr_t>(packed) % 16 != 0)  // bulk async copies need 16-byte sources
+      return fail(CPETGB_ECUDA, "scratch allocation is not 16-byte aligned");
+    g.packed = packed;
+    CK(h2d(&d_frames, S, plan.frames.data(), plan.frames.size()), "copy frame table");
+    g.frames = d_frames;
+    CK(S.get(&g.zeroed, grid_zero_ints(n_frames, g.tau > 0.0)), "alloc counters");
+    if (plan.n_slots)
+      CK(S.get(&g.partial, size_t(plan.n_slots) * grid_slot_doubles(kind, ppt)), "alloc partial sums");
+    if (g.tau > 0.0) {
+      unsigned char* dfq = nullptr;
+      CK(S.get(&g.list, size_t(refine_list_len(n_frames, desc)) * 2), "alloc refinement list");
+      CK(S.get(&dfq, size_t(tot_ch) * 32), "alloc double-float charges");
+      g.dfq = dfq;
+    }
+    CK(launch_grid(g, S.s), "grid launch");
+  }
+  return CPETGB_OK;
+}
+
 int grid_batch_impl(int kind, int prec, int mem, int clamp, int n_frames, const int64_t* desc,
                     const double* pts, const double* x, const double* q, double* out,
                     void* stream) {
@@ -351,12 +459,6 @@ int grid_batch_impl(int kind, int prec, int mem, int clamp, int n_frames, const 
   if (mem == CPETGB_HOST && !s) s = c->stream;
   const int NC = kind == CPETGB_FIELD ? 3 : 1;
 
-  GridTable plan;
-  int ppt = 4, ips = 8;
-  tuned_grid_shape(prec, kind, grid_pair_evals(n_frames, desc), &ppt, &ips);
-  rc = plan_grid(prec, n_frames, desc, c->sms, ppt, ips, plan);
-  if (rc != CPETGB_OK) return rc;
-
   Scratch S(s);
   const double *dp = pts, *dx = x, *dq = q;
   double* dout = out;
@@ -368,39 +470,79 @@ int grid_batch_impl(int kind, int prec, int mem, int clamp, int n_frames, const 
     }
     CK(S.get(&dout, size_t(tot_pts) * NC), "alloc output");
   }
-  GridLaunch g = grid_launch(kind, prec, clamp, ppt, n_frames, desc, plan, tot_ch, c);
-  g.points = dp;
-  g.x = dx;
-  g.q = dq;
-  g.out = dout;
-  if (grid_point_fits(g)) {
-    CK(launch_grid_point(g, s), "point kernel launch");
-  } else {
-    GridFrame* d_frames = nullptr;
-    unsigned char* packed = nullptr;
-    CK(S.get(&packed, size_t(std::max<int64_t>(tot_ch, 1)) * kGridRecord), "alloc packed charges");
-    if (reinterpret_cast<uintptr_t>(packed) % 16 != 0)  // bulk async copies need 16-byte sources
-      return fail(CPETGB_ECUDA, "scratch allocation is not 16-byte aligned");
-    g.packed = packed;
-    CK(h2d(&d_frames, S, plan.frames.data(), plan.frames.size()), "copy frame table");
-    g.frames = d_frames;
-    CK(S.get(&g.zeroed, grid_zero_ints(n_frames, g.tau > 0.0)), "alloc counters");
-    if (plan.n_slots)
-      CK(S.get(&g.partial, size_t(plan.n_slots) * grid_slot_doubles(kind, ppt)), "alloc partial sums");
-    if (g.tau > 0.0) {
-      unsigned char* dfq = nullptr;
-      CK(S.get(&g.list, size_t(refine_list_len(n_frames, desc)) * 2), "alloc refinement list");
-      CK(S.get(&dfq, size_t(tot_ch) * 32), "alloc double-float charges");
-      g.dfq = dfq;
-    }
-    CK(launch_grid(g, s), "grid launch");
-  }
+  rc = grid_device(kind, prec, clamp, n_frames, desc, tot_ch, dp, dx, dq, dout, c, S);
+  if (rc != CPETGB_OK) return rc;
   if (mem == CPETGB_HOST) {
     CK(cudaMemcpyAsync(out, dout, size_t(tot_pts) * NC * sizeof(double), cudaMemcpyDeviceToHost, s),
        "copy output");
     return finish(c, s);
   }
   return CPETGB_OK;
+}
+
+// Field or potential from float32 host arrays to float32 / float16 host rows
+// (RowFormat): one copy in, one out, the conversions on the device.
+int grid_f32_impl(int kind, int prec, int clamp, int P, int N, const float* pts, const float* x,
+                  const float* q, int fmt, void* rows) {
+  if (P < 0 || N < 0) return fail(CPETGB_EINVAL, "negative size");
+  if (P == 0) return CPETGB_OK;
+  if (!valid_prec(prec)) return fail(CPETGB_EINVAL, "bad precision %d", prec);
+  if (!pts || !rows || (N && (!x || !q))) return fail(CPETGB_EINVAL, "NULL pointer");
+  int rc;
+  Ctx* c = context(&rc);
+  if (!c) return rc;
+  cudaStream_t s = c->stream;
+  const size_t np = size_t(P) * 3, nx = size_t(N) * 3, nq = size_t(N), n_in = np + nx + nq;
+  const size_t n_val = size_t(P) * (kind == CPETGB_FIELD ? 3 : 1);
+  const size_t row_bytes =
+      fmt == kRowsField ? size_t(P) * 24 : (fmt == kRowsEspHalf ? size_t(P) * 8 : n_val * sizeof(float));
+  const size_t out_bytes = ((row_bytes + 15) & ~size_t(15)) + 16;  // the status word behind the rows
+  const size_t in_bytes = (n_in * sizeof(float) + 255) & ~size_t(255);
+  Staging host(in_bytes + out_bytes, s);
+  Scratch S(s);
+  float* d_in = nullptr;
+  double *d64 = nullptr, *d_val = nullptr;
+  unsigned char* d_rows = nullptr;
+  CK(S.get(&d_in, n_in), "alloc inputs");
+  CK(S.get(&d64, n_in), "alloc inputs");
+  CK(S.get(&d_val, n_val), "alloc output");
+  CK(S.get(&d_rows, out_bytes), "alloc rows");
+  if (host.p) {
+    float* h = static_cast<float*>(host.p);
+    std::memcpy(h, pts, np * sizeof(float));
+    if (N) {
+      std::memcpy(h + np, x, nx * sizeof(float));
+      std::memcpy(h + np + nx, q, nq * sizeof(float));
+    }
+    CK(cudaMemcpyAsync(d_in, h, n_in * sizeof(float), cudaMemcpyHostToDevice, s), "copy inputs");
+  } else {
+    CK(cudaMemcpyAsync(d_in, pts, np * sizeof(float), cudaMemcpyHostToDevice, s), "copy points");
+    if (N) {
+      CK(cudaMemcpyAsync(d_in + np, x, nx * sizeof(float), cudaMemcpyHostToDevice, s), "copy charge positions");
+      CK(cudaMemcpyAsync(d_in + np + nx, q, nq * sizeof(float), cudaMemcpyHostToDevice, s), "copy charges");
+    }
+  }
+  CK(launch_widen(static_cast<int64_t>(n_in), d_in, d64, s), "widen inputs");
+  const int64_t desc[4] = {0, N, 0, P};
+  rc = grid_device(kind, prec, clamp, 1, desc, N, d64, d64 + np, d64 + np + nx, d_val, c, S);
+  if (rc != CPETGB_OK) return rc;
+  int* tail = reinterpret_cast<int*>(d_rows + out_bytes - 16);
+  CK(launch_rows(fmt, fmt == kRowsPlain ? static_cast<int64_t>(n_val) : P, d_in, d_val, d_rows, c->status, tail, s),
+     "row conversion");
+  int st = 0;
+  if (host.p) {
+    unsigned char* h = static_cast<unsigned char*>(host.p) + in_bytes;
+    CK(cudaMemcpyAsync(h, d_rows, out_bytes, cudaMemcpyDeviceToHost, s), "copy rows");
+    CK(cudaStreamSynchronize(s), "stream synchronize");
+    host.waited = true;
+    std::memcpy(rows, h, row_bytes);
+    std::memcpy(&st, h + out_bytes - 16, sizeof(int));
+  } else {
+    CK(cudaMemcpyAsync(rows, d_rows, row_bytes, cudaMemcpyDeviceToHost, s), "copy rows");
+    CK(cudaMemcpyAsync(&st, tail, sizeof(int), cudaMemcpyDeviceToHost, s), "status read");
+    CK(cudaStreamSynchronize(s), "stream synchronize");
+  }
+  return status_code(c, st);
 }
 
 // source = kCharges: q[N] charges; kDipoles: q is mu[N][3], the dipole moments.
@@ -1307,34 +1449,22 @@ int cpetgb_field_distance_matrix(int precision, int mem, int n, int n_points,
 
 int cpetgb_compute_looped_field_p(int precision, int total_points, int n_charges,
                                   const float* x_0, const float* x, const float* Q, float* E) {
-  if (total_points < 0 || n_charges < 0) return fail(CPETGB_EINVAL, "negative size");
-  if (total_points == 0) return CPETGB_OK;
-  if (!x_0 || !E || (n_charges && (!x || !Q))) return fail(CPETGB_EINVAL, "NULL pointer");
-  auto p = widen(x_0, size_t(total_points) * 3);
-  auto xx = widen(x, size_t(n_charges) * 3);
-  auto qq = widen(Q, size_t(n_charges));
-  std::vector<double> out(size_t(total_points) * 3);
-  const int rc = cpetgb_field_grid(precision, CPETGB_HOST, total_points, n_charges,
-                                   p.data(), xx.data(), qq.data(), 1, out.data(), nullptr);
-  if (rc != CPETGB_OK) return rc;
-  for (size_t i = 0; i < out.size(); ++i) E[i] = static_cast<float>(out[i]);
-  return CPETGB_OK;
+  return grid_f32_impl(CPETGB_FIELD, precision, 1, total_points, n_charges, x_0, x, Q, kRowsPlain, E);
 }
 
 int cpetgb_compute_esp_grid_p(int precision, int total_points, int n_charges, const float* x_0,
                               const float* x, const float* Q, float* ESP) {
-  if (total_points < 0 || n_charges < 0) return fail(CPETGB_EINVAL, "negative size");
-  if (total_points == 0) return CPETGB_OK;
-  if (!x_0 || !ESP || (n_charges && (!x || !Q))) return fail(CPETGB_EINVAL, "NULL pointer");
-  auto p = widen(x_0, size_t(total_points) * 3);
-  auto xx = widen(x, size_t(n_charges) * 3);
-  auto qq = widen(Q, size_t(n_charges));
-  std::vector<double> out(static_cast<size_t>(total_points));
-  const int rc = cpetgb_esp_grid(precision, CPETGB_HOST, total_points, n_charges,
-                                 p.data(), xx.data(), qq.data(), out.data(), nullptr);
-  if (rc != CPETGB_OK) return rc;
-  for (size_t i = 0; i < out.size(); ++i) ESP[i] = static_cast<float>(out[i]);
-  return CPETGB_OK;
+  return grid_f32_impl(CPETGB_ESP, precision, 0, total_points, n_charges, x_0, x, Q, kRowsPlain, ESP);
+}
+
+int cpetgb_box_field_rows(int precision, int n_points, int n_charges, const float* points,
+                          const float* x, const float* q, float* rows) {
+  return grid_f32_impl(CPETGB_FIELD, precision, 1, n_points, n_charges, points, x, q, kRowsField, rows);
+}
+
+int cpetgb_box_esp_rows(int precision, int n_points, int n_charges, const float* points,
+                        const float* x, const float* q, uint16_t* rows) {
+  return grid_f32_impl(CPETGB_ESP, precision, 0, n_points, n_charges, points, x, q, kRowsEspHalf, rows);
 }
 
 int cpetgb_calc_esp_base_p(int precision, float* ESP, const float* x_init, int n_charges,
@@ -1350,15 +1480,7 @@ int cpetgb_calc_esp_base_p(int precision, float* ESP, const float* x_init, int n
 int cpetgb_calc_field_p(int precision, float* E, const float* x_init, int n_charges,
                         const float* x, const float* Q) {
   if (!E || !x_init) return fail(CPETGB_EINVAL, "NULL pointer");
-  if (n_charges < 0) return fail(CPETGB_EINVAL, "negative size");
-  double p[3] = {x_init[0], x_init[1], x_init[2]}, out[3];
-  auto xx = widen(x, size_t(n_charges) * 3);
-  auto qq = widen(Q, size_t(n_charges));
-  const int rc = cpetgb_field_grid(precision, CPETGB_HOST, 1, n_charges, p, xx.data(),
-                                   qq.data(), 0, out, nullptr);
-  if (rc != CPETGB_OK) return rc;
-  for (int k = 0; k < 3; ++k) E[k] = static_cast<float>(out[k]);
-  return CPETGB_OK;
+  return grid_f32_impl(CPETGB_FIELD, precision, 0, 1, n_charges, x_init, x, Q, kRowsPlain, E);
 }
 
 int cpetgb_thread_operation_batch_p(int precision, int n_lines, int n_charges,

@@ -204,6 +204,13 @@ cudaError_t launch_pack_topo(int prec, int64_t n, int64_t n_pad, const double* x
 // out after limit_ns and records kDevWaitTimeout in *status.
 cudaError_t launch_wait_limit_check(int* status, unsigned long long limit_ns, cudaStream_t s);
 
+// rows.cu: conversions of the float32 host calls.  launch_rows writes n float32
+// values (kRowsPlain) or n points' rows, and copies the status word to *tail.
+enum RowFormat : int { kRowsPlain = 0, kRowsField = 1, kRowsEspHalf = 2 };
+cudaError_t launch_widen(int64_t n, const float* in, double* out, cudaStream_t s);
+cudaError_t launch_rows(int fmt, int64_t n, const float* pts, const double* val, void* rows, const int* status,
+                        int* tail, cudaStream_t s);
+
 // api.cu: records `msg` as the calling thread's last error and returns `code`.
 int set_error(int code, const char* msg);
 

@@ -29,9 +29,12 @@ import numpy as np
 
 from .calculator import (box_transformation, initialize_box_points_random, initialize_box_points_uniform,
                          volume_grid_counts)
-from .core import esp_grid, field_grid, prepare_frame, topo_dipole_lines, topo_lines
+from ._lib import check, lib
+from .core import esp_grid, field_grid, precision_code, prepare_frame, topo_dipole_lines, topo_lines
 
 log = logging.getLogger(__name__)
+
+_ORIGIN = np.zeros(3, np.float32)
 
 HOT_METHODS = ("compute_point_field", "compute_box", "compute_box_ESP", "compute_topo_complete_c_shared",
                "compute_topo_GPU_batch_filter", "compute_topo_complete_c_shared_dipole")
@@ -41,14 +44,47 @@ def _prec(self):
     return getattr(self, "precision", None) or "fp32c"
 
 
+def _f32_inputs(self):
+    """(x, q) as contiguous float32 arrays when that is what the calculator
+    holds (its default dtype), else None: the float32 calls convert on the GPU."""
+    x, q = self.x, self.Q
+    if not (isinstance(x, np.ndarray) and isinstance(q, np.ndarray) and x.dtype == np.float32
+            and q.dtype == np.float32 and x.size == 3 * q.size):
+        return None
+    return np.ascontiguousarray(x), np.ascontiguousarray(q)
+
+
 def compute_point_field(self):
     """Field at the box centre (the origin of the rotated frame)."""
+    f32 = _f32_inputs(self)
+    if f32 is not None:
+        x, q = f32
+        E = np.empty(3, np.float32)
+        check(lib().cpetgb_calc_field_p(precision_code(_prec(self)), E.ctypes.data, _ORIGIN.ctypes.data, q.size,
+                                        x.ctypes.data, q.ctypes.data))
+        return E
     E = field_grid(np.zeros((1, 3)), np.asarray(self.x, np.float64), np.asarray(self.Q, np.float64),
                    precision=_prec(self), clamp=False)
     return E[0].astype(np.float32)
 
 
+def _box_rows(self, fn, columns, dtype):
+    """The whole output array from one float32 call, or None for other dtypes."""
+    f32 = _f32_inputs(self)
+    if f32 is None or not isinstance(self.mesh, np.ndarray) or self.mesh.dtype != np.float32:
+        return None
+    x, q = f32
+    pts = np.ascontiguousarray(self.mesh).reshape(-1, 3)
+    rows = np.empty((len(pts), columns), dtype)
+    check(fn(precision_code(_prec(self)), len(pts), q.size, pts.ctypes.data, x.ctypes.data, q.ctypes.data,
+             rows.ctypes.data))
+    return rows
+
+
 def compute_box(self):
+    rows = _box_rows(self, lib().cpetgb_box_field_rows, 6, np.float32)
+    if rows is not None:
+        return rows, self.mesh.shape
     x_0 = self.mesh.reshape(-1, 3)
     E = field_grid(x_0, np.asarray(self.x, np.float64), np.asarray(self.Q, np.float64),
                    precision=_prec(self), clamp=True)
@@ -56,6 +92,9 @@ def compute_box(self):
 
 
 def compute_box_ESP(self):
+    rows = _box_rows(self, lib().cpetgb_box_esp_rows, 4, np.half)
+    if rows is not None:
+        return rows, self.mesh.shape
     x_0 = self.mesh.reshape(-1, 3)
     phi = esp_grid(x_0, np.asarray(self.x, np.float64), np.asarray(self.Q, np.float64), precision=_prec(self))
     return np.concatenate((x_0, phi.reshape(-1, 1)), axis=1).astype(np.half), self.mesh.shape
