@@ -1000,12 +1000,13 @@ int distance_impl(int kind, int prec, int mem, int n, int feat, const double* sr
     CK(S.get(&dout, size_t(n) * n), "alloc matrix");
   }
   const int splits = distance_splits(n, feat, c->sms);
-  double* partial = nullptr;
-  if (splits > 1) CK(S.get(&partial, size_t(splits) * n * n), "alloc partial sums");
-  unsigned char* f32_rows = nullptr;
+  unsigned char *partial = nullptr, *f32_rows = nullptr;
+  if (splits > 1) CK(S.get(&partial, distance_partial_bytes(prec, kind, n, splits)), "alloc partial sums");
   if (prec != CPETGB_FP64 && feat > 0)
     CK(S.get(&f32_rows, distance_f32_bytes(kind, n, feat)), "alloc float rows");
-  CK(launch_distance_matrix(prec, kind, n, feat, dsrc, dout, splits, partial, f32_rows, s),
+  if (reinterpret_cast<uintptr_t>(f32_rows) % 16 != 0)  // bulk async copies need 16-byte sources
+    return fail(CPETGB_ECUDA, "scratch allocation is not 16-byte aligned");
+  CK(launch_distance_matrix(prec, kind, n, feat, dsrc, dout, splits, partial, f32_rows, c->status, s),
      "distance launch");
   if (mem == CPETGB_HOST) {
     CK(cudaMemcpyAsync(out, dout, size_t(n) * n * sizeof(double), cudaMemcpyDeviceToHost, s),

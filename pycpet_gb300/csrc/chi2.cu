@@ -1,0 +1,266 @@
+// chi2.cu -- the FP32C chi-square matrix over histograms (distance.cu has the
+// other distance matrices and the definition).
+//
+// Three launches:
+//   pack     every value rounded to FP32 once and laid out tile-major,
+//            [64-row block][bin][64 rows], rows past the end zero, so that a
+//            chunk of 32 bins of a block is 8 KB in one piece;
+//   tiles    one CTA per 64 x 64 tile of the upper triangle and bin split:
+//            chunks of both row blocks come by bulk async copy into a two-stage
+//            ring, a thread owns 4 x 4 entries and reads its rows and its
+//            column pairs with one 16-byte load each per bin; two terms per
+//            packed f32x2 instruction, one MUFU reciprocal per term.  Each chunk
+//            is summed plainly and Kahan-added (Kahan 1965) into a running
+//            (sum, compensation) pair per entry;
+//   merge    the splits' pairs added in split order (TwoSum, the rounding errors
+//            beside the compensations: 48 bits), halved, and written to the entry
+//            and its mirror image through shared memory.
+//            With one split the tile kernel writes the matrix itself.
+// Sums stay in FP32 pairs until the single double subtraction at the end: an FP64
+// warp instruction holds a scheduler's FP64 pipe for 64 cycles, and 48 of them per
+// thread (conversions included) were a quarter of the time.
+// Bound: the MUFU reciprocals, one per term: a warp's takes a scheduler's unit 8
+// cycles, and a loop of this body on registers alone 16.9 cycles per pair of terms
+// (10.3 without the reciprocals); two terms can't share one, 1 / (s t) rounds
+// differently.  1,024 histograms of 400 bins: pack 3, tiles 59 (51 at 16.9 cycles),
+// merge 9 us; 96 us per call before, with row-major staging, a
+// select around each reciprocal, and the splits summed in double.  3 CTAs per SM: 59.4 us,
+// against 63.5 with the 2 that unlimited registers leave and 60.3 with 4; 2 x 4 and
+// 4 x 2 entries per thread 59.4 to 65.5; 32 x 16 tiles in one pass without splits 65.6.
+#include <algorithm>
+#include <cfloat>
+#include <cstdint>
+
+#include "common.cuh"
+#include "kernels.cuh"
+
+namespace cpetgb {
+namespace {
+
+constexpr int kTile = 64;
+constexpr int kThreads = 256;  // 16 x 16 threads, 4 x 4 entries each
+constexpr int kChunk = 32;     // bins per Kahan-added sum and per stage
+constexpr int kStages = 2;
+constexpr int kEntries = kTile * kTile;
+
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
+// MUFU reciprocal, +infinity (of a zero sum) made finite: such a term is
+// 0 * 0 * FLT_MAX = 0, as the definition has it.
+__device__ __forceinline__ float rcp_finite(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return fminf(y, FLT_MAX);
+}
+
+__device__ __forceinline__ double pair_value(float s, float c) { return __dsub_rn(widen(s), widen(c)); }
+
+// Upper-triangle tile t, column by column: t = jb (jb + 1) / 2 + ib, ib <= jb.
+__device__ __forceinline__ void tile_of(uint32_t t, int& ib, int& jb) {
+  uint32_t j = static_cast<uint32_t>(0.5f * (sqrtf(8.f * static_cast<float>(t) + 1.f) - 1.f));
+  while (uint64_t(j) * (j + 1) / 2 > t) --j;
+  while (uint64_t(j + 1) * (j + 2) / 2 <= t) ++j;
+  jb = static_cast<int>(j);
+  ib = static_cast<int>(t - uint64_t(j) * (j + 1) / 2);
+}
+
+// One row block x 32 bins per step, all of a thread's loads in flight at once.
+__global__ void __launch_bounds__(kThreads)
+    chi2_pack_kernel(int n, int bins, const double* __restrict__ in, float* __restrict__ out) {
+  constexpr int kBins = 32, kLoads = kTile * kBins / kThreads;
+  __shared__ float t[kBins][kTile + 1];
+  const int tid = threadIdx.x, rb = blockIdx.x;
+  for (int64_t k0 = int64_t(blockIdx.y) * kBins; k0 < bins; k0 += int64_t(gridDim.y) * kBins) {
+    const int64_t k = k0 + tid % kBins;
+    double v[kLoads];
+#pragma unroll
+    for (int u = 0; u < kLoads; ++u) {
+      const int64_t row = int64_t(rb) * kTile + tid / kBins + u * (kThreads / kBins);
+      v[u] = row < n && k < bins ? in[row * bins + k] : 0.0;
+    }
+    __syncthreads();  // the previous step's reads
+#pragma unroll
+    for (int u = 0; u < kLoads; ++u)  // + 0: a sum of two zeros is +0 whatever their signs
+      t[tid % kBins][tid / kBins + u * (kThreads / kBins)] = __fadd_rn(narrow(v[u]), 0.f);
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kLoads; ++u) {
+      const int e = tid + u * kThreads;
+      if (k0 + e / kTile < bins) out[(int64_t(rb) * bins + k0) * kTile + e] = t[e / kTile][e % kTile];
+    }
+  }
+}
+
+// part: [tile][split][16 entries][256 threads] pairs, or null (one split).
+__global__ void __launch_bounds__(kThreads, 3)
+    chi2_tile_kernel(int n, int bins, int per, const float* __restrict__ rows, double* __restrict__ out,
+                     float2* __restrict__ part, int* __restrict__ status) {
+  __shared__ alignas(16) float sA[kStages][kChunk][kTile];
+  __shared__ alignas(16) float sB[kStages][kChunk][kTile];
+  __shared__ uint64_t full[kStages];
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  int ib, jb;
+  tile_of(blockIdx.x, ib, jb);
+  const int kb = blockIdx.y * per, ke = min(bins, kb + per);
+  const int n_chunks = ke > kb ? (ke - kb + kChunk - 1) / kChunk : 0;
+  const float* rows_a = rows + (int64_t(ib) * bins + kb) * kTile;
+  const float* rows_b = rows + (int64_t(jb) * bins + kb) * kTile;
+
+  if (tid == 0) {
+    for (int s = 0; s < kStages; ++s) mbar_init(&full[s], 1);
+    fence_mbar_init();
+  }
+  __syncthreads();
+  auto issue = [&](int t) {
+    const int s = t % kStages;
+    const uint32_t bytes = static_cast<uint32_t>(min(kChunk, ke - kb - t * kChunk)) * kTile * sizeof(float);
+    mbar_arrive_expect_tx(&full[s], 2 * bytes);
+    bulk_g2s(&sA[s][0][0], rows_a + int64_t(t) * kChunk * kTile, bytes, &full[s]);
+    bulk_g2s(&sB[s][0][0], rows_b + int64_t(t) * kChunk * kTile, bytes, &full[s]);
+  };
+  if (tid == 0)
+    for (int t = 0; t < min(kStages, n_chunks); ++t) issue(t);
+
+  float sum[4][4], cmp[4][4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) sum[r][c] = cmp[r][c] = 0.f;
+
+  for (int t = 0; t < n_chunks; ++t) {
+    const int s = t % kStages;
+    const bool mine = mbar_wait(&full[s], static_cast<uint32_t>((t / kStages) & 1), status);
+    // also: every thread is done with chunk t - 1, whose stage takes the next copy
+    if (!__syncthreads_and(mine)) {
+      // a copy that never came: wait (with the same limit) for what else is in flight
+      if (tid == 0)
+        for (int u = t; u < min(t - 1 + kStages, n_chunks); ++u)
+          mbar_wait(&full[u % kStages], static_cast<uint32_t>((u / kStages) & 1), status);
+      return;
+    }
+    if (tid == 0 && t >= 1 && t - 1 + kStages < n_chunks) issue(t - 1 + kStages);
+    const int kn = min(kChunk, ke - kb - t * kChunk);
+    const float4* a4 = reinterpret_cast<const float4*>(&sA[s][0][0]) + ty;
+    const ulonglong2* b4 = reinterpret_cast<const ulonglong2*>(&sB[s][0][0]) + tx;
+    uint64_t p[4][2];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) p[r][0] = p[r][1] = 0ull;
+#pragma unroll 2
+    for (int k = 0; k < kn; ++k) {
+      const float4 av = a4[k * (kTile / 4)];
+      const ulonglong2 bv = b4[k * (kTile / 4)];
+      const float a[4] = {av.x, av.y, av.z, av.w};
+      const uint64_t b[2] = {bv.x, bv.y};
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const uint64_t aa = pk2(a[r], a[r]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint64_t d = sub2(aa, b[h]);
+          float s0, s1;
+          upk2(add2(aa, b[h]), s0, s1);
+          p[r][h] = fma2(mul2(d, d), pk2(rcp_finite(s0), rcp_finite(s1)), p[r][h]);
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float lo, hi;
+        upk2(p[r][h], lo, hi);
+        kahan_add(sum[r][2 * h], cmp[r][2 * h], lo);
+        kahan_add(sum[r][2 * h + 1], cmp[r][2 * h + 1], hi);
+      }
+  }
+
+  if (part) {
+    float2* dst = part + (int64_t(blockIdx.x) * gridDim.y + blockIdx.y) * kEntries + tid;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) dst[(4 * r + c) * kThreads] = make_float2(sum[r][c], cmp[r][c]);
+    return;
+  }
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int64_t i = int64_t(ib) * kTile + 4 * ty + r, j = int64_t(jb) * kTile + 4 * tx + c;
+      if (i >= n || j >= n) continue;
+      const double v = i == j ? 0.0 : 0.5 * pair_value(sum[r][c], cmp[r][c]);
+      out[i * n + j] = v;
+      if (ib != jb) out[j * n + i] = v;
+    }
+}
+
+// blockIdx.y = quarter g of the tile: its rows 16 g .. 16 g + 15, so that both the
+// rows and their mirror columns are written in runs of 128 bytes or more.
+__global__ void __launch_bounds__(kThreads)
+    chi2_merge_kernel(int n, int splits, const float2* __restrict__ part, double* __restrict__ out) {
+  constexpr int kRows = kTile / 4;
+  __shared__ double t[kRows][kTile + 1];
+  const int tid = threadIdx.x, g = blockIdx.y, owner = tid & 63, r = tid >> 6;
+  int ib, jb;
+  tile_of(blockIdx.x, ib, jb);
+  const float2* src = part + int64_t(blockIdx.x) * splits * kEntries + 4 * r * kThreads + 64 * g + owner;
+  float s[4] = {}, c[4] = {};
+#pragma unroll 4
+  for (int z = 0; z < splits; ++z)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float2 v = src[int64_t(z) * kEntries + k * kThreads];
+      float e;
+      two_sum(s[k], v.x, s[k], e);
+      c[k] = __fadd_rn(c[k], __fsub_rn(v.y, e));
+    }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) t[4 * (owner >> 4) + r][4 * (owner & 15) + k] = 0.5 * pair_value(s[k], c[k]);
+  __syncthreads();
+  const int64_t i0 = int64_t(ib) * kTile + kRows * g, j0 = int64_t(jb) * kTile;
+  for (int e = tid; e < kRows * kTile; e += kThreads) {
+    const int64_t i = i0 + e / kTile, j = j0 + e % kTile;
+    if (i < n && j < n) out[i * n + j] = i == j ? 0.0 : t[e / kTile][e % kTile];
+  }
+  if (ib == jb) return;
+  for (int e = tid; e < kRows * kTile; e += kThreads) {
+    const int64_t i = i0 + e % kRows, j = j0 + e / kRows;
+    if (i < n && j < n) out[j * n + i] = t[e % kRows][e / kRows];
+  }
+}
+
+}  // namespace
+
+int64_t chi2_row_blocks(int n) { return (int64_t(n) + kTile - 1) / kTile; }
+size_t chi2_rows_bytes(int n, int bins) { return size_t(chi2_row_blocks(n)) * kTile * size_t(bins) * sizeof(float); }
+size_t chi2_partial_bytes(int n, int splits) {
+  const int64_t nb = chi2_row_blocks(n);
+  return size_t(nb * (nb + 1) / 2) * size_t(splits) * kEntries * sizeof(float2);
+}
+
+cudaError_t launch_chi2_f32(int n, int bins, const double* hists, double* out, int splits, void* partial,
+                            void* rows, int* status, cudaStream_t s) {
+  const int64_t nb = chi2_row_blocks(n);
+  float* fr = static_cast<float*>(rows);
+  if (bins > 0) {
+    const int by = static_cast<int>(std::min<int64_t>((int64_t(bins) + 31) / 32, 65535));
+    chi2_pack_kernel<<<dim3(static_cast<unsigned>(nb), by), kThreads, 0, s>>>(n, bins, hists, fr);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  if (splits < 1 || bins == 0) splits = 1;
+  const int per = (bins + splits - 1) / splits;
+  float2* pairs = splits > 1 ? static_cast<float2*>(partial) : nullptr;
+  const unsigned tiles = static_cast<unsigned>(nb * (nb + 1) / 2);
+  chi2_tile_kernel<<<dim3(tiles, splits), kThreads, 0, s>>>(n, bins, per, fr, out, pairs, status);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess || splits == 1) return e;
+  chi2_merge_kernel<<<dim3(tiles, 4), kThreads, 0, s>>>(n, splits, pairs, out);
+  return cudaGetLastError();
+}
+
+}  // namespace cpetgb

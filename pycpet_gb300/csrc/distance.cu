@@ -24,11 +24,10 @@
 //   FP64   every operation in IEEE double; the per-point norm is formed as
 //          numpy forms it, (dx*dx + dy*dy) + dz*dz then sqrt, with no fused
 //          multiply-add, so only the order of the final sum differs.
-//   FP32C  values rounded to FP32 once before the launch; chi2 terms use the
-//          MUFU reciprocal (two columns per packed f32x2 instruction), field
-//          terms the MUFU reciprocal square root; each staged chunk is summed
-//          plainly and Kahan-added (Kahan 1965) into a running (sum,
-//          compensation) pair.
+//   FP32C  values rounded to FP32 once before the launch; field terms use the
+//          MUFU reciprocal square root; each staged chunk is summed plainly and
+//          Kahan-added (Kahan 1965) into a running (sum, compensation) pair.
+//          The chi2 matrix has kernels of its own (chi2.cu).
 // The term of (i, j) equals the term of (j, i) bit for bit in both forms, so
 // a tile on the diagonal writes an exactly symmetric block.
 #include <algorithm>
@@ -48,18 +47,6 @@ constexpr int kThreads = 256;  // 16 x 16 threads, 4 x 4 entries each
 template <typename Real, int NC>
 constexpr int chunk_of() {
   return NC == 1 ? 32 : (sizeof(Real) == 4 ? 16 : 8);
-}
-
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-
-__device__ __forceinline__ float rcp_mufu(float x) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
 }
 
 template <typename Real>
@@ -96,15 +83,7 @@ __device__ __forceinline__ double chi2_term(double a, double b) {
   const double d = __dsub_rn(a, b);
   return s != 0.0 ? __ddiv_rn(__dmul_rn(d, d), s) : 0.0;
 }
-__device__ __forceinline__ float chi2_term(float a, float b) {
-  const float s = __fadd_rn(a, b);
-  const float d = __fsub_rn(a, b);
-  const float r = s != 0.f ? rcp_mufu(s) : 0.f;
-  return __fmul_rn(__fmul_rn(d, d), r);
-}
-
-template <typename Real>
-__device__ __forceinline__ Real term(const Feat<Real, 1>& a, const Feat<Real, 1>& b) {
+__device__ __forceinline__ double term(const Feat<double, 1>& a, const Feat<double, 1>& b) {
   return chi2_term(a.v, b.v);
 }
 __device__ __forceinline__ double term(const Feat<double, 3>& a, const Feat<double, 3>& b) {
@@ -175,43 +154,6 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
       for (int c = 0; c < 4; ++c) part[r][c] = Real(0);
     const int kn = min(kChunk, ke - k0);
-    if constexpr (KIND == 0 && sizeof(Real) == 4) {
-      // chi2 in packed pairs of columns: one f32x2 instruction for two terms
-      uint64_t p2[4][2];
-#pragma unroll
-      for (int r = 0; r < 4; ++r) p2[r][0] = p2[r][1] = 0ull;
-#pragma unroll 4
-      for (int k = 0; k < kn; ++k) {
-        float a[4];
-        uint64_t b2[2];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) a[r] = reinterpret_cast<const float&>(sA[k][ty + 16 * r]);
-        b2[0] = pk2(reinterpret_cast<const float&>(sB[k][tx]), reinterpret_cast<const float&>(sB[k][tx + 16]));
-        b2[1] = pk2(reinterpret_cast<const float&>(sB[k][tx + 32]), reinterpret_cast<const float&>(sB[k][tx + 48]));
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const uint64_t aa = pk2(a[r], a[r]);
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const uint64_t s2 = add2(aa, b2[h]);
-            const uint64_t d2 = sub2(aa, b2[h]);
-            float s0, s1;
-            upk2(s2, s0, s1);
-            const uint64_t rr = pk2(s0 != 0.f ? rcp_mufu(s0) : 0.f, s1 != 0.f ? rcp_mufu(s1) : 0.f);
-            p2[r][h] = fma2(mul2(d2, d2), rr, p2[r][h]);
-          }
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          float lo, hi;
-          upk2(p2[r][h], lo, hi);
-          part[r][2 * h] = reinterpret_cast<Real&>(lo);
-          part[r][2 * h + 1] = reinterpret_cast<Real&>(hi);
-        }
-    } else {
 #pragma unroll 4
     for (int k = 0; k < kn; ++k) {
       F a[4], b[4];
@@ -230,7 +172,6 @@ __global__ void __launch_bounds__(kThreads)
           else
             part[r][c] = __fadd_rn(part[r][c], t);
         }
-    }
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r)
@@ -255,14 +196,12 @@ __global__ void __launch_bounds__(kThreads)
     }
 }
 
-// FP32C staging source: every value rounded to float once (a field point
-// padded to 4 components), instead of in every CTA that stages the row.
-template <int NC>
-__global__ void to_f32_kernel(int64_t n_feat, const double* __restrict__ in,
-                              Feat<float, NC>* __restrict__ out) {
+// FP32C staging source of the field form: every value rounded to float once (a
+// point padded to 4 components), instead of in every CTA that stages the row.
+__global__ void to_f32_kernel(int64_t n_feat, const double* __restrict__ in, Feat<float, 3>* __restrict__ out) {
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n_feat;
        i += int64_t(gridDim.x) * blockDim.x)
-    load_feat<float, NC>(out[i], in + i * NC, true);
+    load_feat<float, 3>(out[i], in + i * 3, true);
 }
 
 // Sum of the feature splits in split order (deterministic); chi2 halved;
@@ -292,20 +231,24 @@ int distance_splits(int n, int feat, int num_sms) {
 }
 
 size_t distance_f32_bytes(int kind, int n, int feat) {
-  return size_t(n) * size_t(feat) * (kind == 0 ? sizeof(float) : sizeof(Feat<float, 3>));
+  return kind == 0 ? chi2_rows_bytes(n, feat) : size_t(n) * size_t(feat) * sizeof(Feat<float, 3>);
+}
+
+size_t distance_partial_bytes(int prec, int kind, int n, int splits) {
+  return prec != kFP64 && kind == 0 ? chi2_partial_bytes(n, splits) : size_t(splits) * n * n * sizeof(double);
 }
 
 cudaError_t launch_distance_matrix(int prec, int kind, int n, int feat, const double* src,
-                                   double* out, int splits, double* partial, void* f32_rows,
-                                   cudaStream_t s) {
+                                   double* out, int splits, void* partial_raw, void* f32_rows,
+                                   int* status, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
+  if (prec != kFP64 && kind == 0)
+    return launch_chi2_f32(n, feat, src, out, splits, partial_raw, f32_rows, status, s);
+  double* partial = static_cast<double*>(partial_raw);
   if (prec != kFP64 && int64_t(n) * feat > 0) {
     const int64_t nf = int64_t(n) * feat;
     const int blocks = static_cast<int>(std::min<int64_t>((nf + 255) / 256, 8192));
-    if (kind == 0)
-      to_f32_kernel<1><<<blocks, 256, 0, s>>>(nf, src, static_cast<Feat<float, 1>*>(f32_rows));
-    else
-      to_f32_kernel<3><<<blocks, 256, 0, s>>>(nf, src, static_cast<Feat<float, 3>*>(f32_rows));
+    to_f32_kernel<<<blocks, 256, 0, s>>>(nf, src, static_cast<Feat<float, 3>*>(f32_rows));
     cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return err;
   }
@@ -320,10 +263,7 @@ cudaError_t launch_distance_matrix(int prec, int kind, int n, int feat, const do
     else
       distance_kernel<double, 1><<<grid, kThreads, 0, s>>>(n, feat, per, src, out, pout);
   } else {
-    if (kind == 0)
-      distance_kernel<float, 0><<<grid, kThreads, 0, s>>>(n, feat, per, f32_rows, out, pout);
-    else
-      distance_kernel<float, 1><<<grid, kThreads, 0, s>>>(n, feat, per, f32_rows, out, pout);
+    distance_kernel<float, 1><<<grid, kThreads, 0, s>>>(n, feat, per, f32_rows, out, pout);
   }
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess || splits == 1) return err;

@@ -254,8 +254,6 @@ cudaError_t launch_hist2d_sets(int n_sets, const int64_t* d_off, int64_t max_set
                                double* edges, unsigned long long* counts, double* hists,
                                int* status, cudaStream_t s);
 
-// distance.cu: kind 0 = chi-square over histogram rows [n][feat]; kind 1 =
-// summed Euclidean norms over field rows [n][feat][3]; out [n][n].
 // prep.cu: residue radius filter, rotation, box filter, shift, compaction of one
 // frame (device pointers; center/inv/half/shift on the host, inv/half/shift may
 // be null); the survivor count lands in d_count (device int64).
@@ -278,12 +276,20 @@ cudaError_t launch_text_offsets(int fmt, int64_t n_rows, int n_cols, const float
 cudaError_t launch_text_write(int fmt, int64_t n_rows, int n_cols, const float* v,
                               const int64_t* offsets, char* out, cudaStream_t s);
 
-// splits > 1 (distance_splits) needs partial scratch of splits * n * n doubles.
+// distance.cu: kind 0 = chi-square over histogram rows [n][feat]; kind 1 =
+// summed Euclidean norms over field rows [n][feat][3]; out [n][n].
+// splits > 1 (distance_splits) needs partial scratch of distance_partial_bytes;
 // FP32C also needs f32_rows scratch of distance_f32_bytes(kind, n, feat) bytes.
 int distance_splits(int n, int feat, int num_sms);
 size_t distance_f32_bytes(int kind, int n, int feat);
+size_t distance_partial_bytes(int prec, int kind, int n, int splits);
 cudaError_t launch_distance_matrix(int prec, int kind, int n, int feat, const double* src,
-                                   double* out, int splits, double* partial, void* f32_rows,
-                                   cudaStream_t s);
+                                   double* out, int splits, void* partial, void* f32_rows,
+                                   int* status, cudaStream_t s);
+// chi2.cu: kind 0 in FP32C.  Scratch 16-byte aligned.
+size_t chi2_rows_bytes(int n, int bins);
+size_t chi2_partial_bytes(int n, int splits);
+cudaError_t launch_chi2_f32(int n, int bins, const double* hists, double* out, int splits, void* partial,
+                            void* rows, int* status, cudaStream_t s);
 
 }  // namespace cpetgb
