@@ -192,10 +192,19 @@ __device__ __forceinline__ void run_frame(const TopoParams& p, const FrameCtx& f
   }
 }
 
-// Frames are visited in table order; a CTA stays on a frame while its line
-// queue lasts, then moves on (after its own warps are done or have handed their
-// lines over, so the shared copy of the charges can be replaced).  Frames thus
-// overlap only at their tails.
+// One frame's share of a launch's work.
+__device__ __forceinline__ double frame_work(const TopoFrame& fr) {
+  return static_cast<double>(fr.n_lines) * fr.n_pad;
+}
+
+// The CTAs start spread over the frames by their work and visit them in table
+// order from there.  With all CTAs starting at the first frame, a frame of 3,000
+// lines fills the slots of 94 CTAs at once and leaves them nothing to refill
+// with, and half of the launch's lines are handed over (6 frames x 3,000 lines of
+// 5,000 to 20,000 charges: 93 ms here and 72 ms of rounds; spread, 123 and 38).
+// A CTA stays on a frame while its line queue lasts, then moves on (after its
+// own warps are done or have handed their lines over, so the shared copy of the
+// charges can be replaced).
 // DIP: the sources are point dipoles (FP32C: three 16-byte pair blocks per
 // frame; FP64: Dipole64 records) instead of point charges.  SRC: kSrcShared when
 // every frame of the launch fits shared memory, kSrcSplit otherwise (FP64:
@@ -203,7 +212,7 @@ __device__ __forceinline__ void run_frame(const TopoParams& p, const FrameCtx& f
 template <int PREC, int S, bool DIP, int SRC>
 __global__ void __launch_bounds__(kTopoThreads, 1) topo_kernel(TopoParams p, TopoFrame frame0) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ int s_skip;
+  __shared__ int s_skip, s_first;
   __shared__ int s_idle;  // line slots of this CTA that found the frame's queue empty
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -219,7 +228,34 @@ __global__ void __launch_bounds__(kTopoThreads, 1) topo_kernel(TopoParams p, Top
     fence_mbar_init();
   }
 
-  for (int f = 0; f < n_frames; ++f) {
+  if (p.frames && warp == 0) {
+    // work (lines x sources) before this CTA's share, and the frame it lies in
+    double total = 0.0;
+    for (int f = lane; f < n_frames; f += 32) total += frame_work(p.frames[f]);
+    for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+    const double mine = total * (blockIdx.x + 0.5) / gridDim.x;
+    double base = 0.0;
+    int first = 0;
+    for (int f0 = 0; f0 < n_frames; f0 += 32) {
+      double incl = f0 + lane < n_frames ? frame_work(p.frames[f0 + lane]) : 0.0;
+      for (int o = 1; o < 32; o <<= 1) {
+        const double v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      const unsigned past = __ballot_sync(0xffffffffu, f0 + lane < n_frames && base + incl > mine);
+      if (past) {
+        first = f0 + __ffs(past) - 1;
+        break;
+      }
+      base += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) s_first = first;
+  }
+  __syncthreads();
+  const int first_frame = p.frames ? s_first : 0;
+
+  for (int i = 0; i < n_frames; ++i) {
+    const int f = first_frame + i < n_frames ? first_frame + i : first_frame + i - n_frames;
     const TopoFrame fr = p.frames ? p.frames[f] : frame0;
     int* queue = p.queue + f;
     __syncthreads();  // the CTA's warps are done with the previous frame
