@@ -589,8 +589,10 @@ int topo_impl(int prec, int mem, int L, int N, const double* starts, const int32
   int* queue = nullptr;  // the queue counter and, per round, the count of lines handed over
   TopoState* left = nullptr;
   const int rounds = topo_team_rounds(c->sms, L, topo_diag_steps(half, step));
+  const bool fresh = topo_fresh(prec, topo_resident_count(prec, source, static_cast<int>(n_pad)) == n_pad, L,
+                                c->sms, true);
   const bool hand = rounds > 1 || L > int64_t(c->sms) * kTeamLinesPerSm;
-  const int left_cap = hand ? topo_left_capacity(c->sms, L) : 0;
+  const int left_cap = hand ? topo_left_capacity(c->sms, L, fresh) : 0;
   CK(S.get(&packed, size_t(n_pad) * topo_source_bytes(prec, source)), "alloc packed charges");
   CK(S.get(&queue, size_t(1 + rounds)), "alloc queue");
   CK(cudaMemsetAsync(queue, 0, (1 + rounds) * sizeof(int), s), "zero queue");
@@ -651,7 +653,6 @@ struct TopoTables {
 // Charge64), how many charges of each frame stay resident in shared memory, and
 // each frame's hand-over records (at most kMaxLeft in all; frames beyond that
 // have none and their lines end where they started).
-constexpr int64_t kMaxLeft = int64_t(1) << 18;  // two lists of 42 MB
 
 int build_topo_tables(int prec, int F, const int64_t* desc, const double* params, TopoTables& t) {
   if (!valid_prec(prec)) return fail(CPETGB_EINVAL, "bad precision %d", prec);
@@ -693,11 +694,12 @@ int build_topo_tables(int prec, int F, const int64_t* desc, const double* params
   return CPETGB_OK;
 }
 
-void plan_hand_over(int sms, TopoTables& t) {
+void plan_hand_over(int prec, int sms, TopoTables& t) {
   t.rounds = topo_team_rounds(sms, t.sum_lines, t.diag_steps);
+  const bool fresh = topo_fresh(prec, t.all_resident, t.sum_lines, sms, true);
   const bool hand = t.rounds > 1 || t.sum_lines > int64_t(sms) * kTeamLinesPerSm;
   for (TopoFrame& fr : t.frames) {
-    const int64_t cap = hand ? topo_left_capacity(sms, fr.n_lines) : 0;
+    const int64_t cap = hand ? topo_left_capacity(sms, fr.n_lines, fresh) : 0;
     fr.left_off = static_cast<int32_t>(t.left_records);
     fr.left_cap = t.left_records + cap <= kMaxLeft ? static_cast<int32_t>(cap) : 0;
     t.left_records += fr.left_cap;
@@ -722,7 +724,7 @@ int topo_batch_impl(int prec, int mem, int F, const int64_t* desc, const double*
   int rc;
   Ctx* c = context(&rc);
   if (!c) return rc;
-  plan_hand_over(c->sms, t);
+  plan_hand_over(prec, c->sms, t);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (mem == CPETGB_HOST && !s) s = c->stream;
   const size_t L = size_t(tot_lines);
@@ -1163,7 +1165,7 @@ int topo_plan_impl(cpetgb_plan** out_plan, int prec, int F, const int64_t* desc,
   if (t.tot_ch > 0 && (!x || !q)) return fail(CPETGB_EINVAL, "charge pointer is NULL");
   Ctx* c = context(&rc);
   if (!c) return rc;
-  plan_hand_over(c->sms, t);
+  plan_hand_over(prec, c->sms, t);
   cpetgb_plan* pl = new cpetgb_plan();
   cudaGetDevice(&pl->device);
   unsigned char* packed = nullptr;

@@ -169,7 +169,7 @@ cudaError_t launch_pack_topo_frames(int prec, int n_frames, const TopoFrame* d_f
                                     const int64_t* d_src, const double* x, const double* q,
                                     void* packed, int max_pairs, cudaStream_t s);
 // Hand-over records of a frame of n_lines in each list (TopoFrame::left_cap).
-int topo_left_capacity(int num_sms, int64_t n_lines);
+int topo_left_capacity(int num_sms, int64_t n_lines, bool fresh);
 
 // topo_team.cu: lines stepped by teams of warps, in p.rounds launches.  fresh !=
 // 0: the lines of the frames' tables from their start points; 0: the lines
@@ -181,9 +181,14 @@ int topo_team_resident(int prec, int source, int n_pad);
 // in diag_steps steps (the largest of the launch's frames).
 int topo_team_rounds(int num_sms, int64_t sum_lines, double diag_steps);
 double topo_diag_steps(const double* half, double step);
-// a launch of at most this many lines per SM goes to the team kernel at once, and a CTA
-// of the persistent kernel hands its last lines over once it holds no more than this many
+// the lines a CTA of the team kernel steps together; a CTA of the persistent kernel
+// hands its last lines over once it holds no more than this many
 constexpr int kTeamLinesPerSm = 16;
+constexpr int64_t kMaxLeft = int64_t(1) << 18;  // hand-over records of a launch: two lists of 42 MB
+// Whether a launch's lines go to the team kernel from their start points
+// (resident: every frame's sources fit shared memory; lists: hand-over records
+// can be had).
+bool topo_fresh(int prec, bool resident, int64_t sum_lines, int num_sms, bool lists);
 
 // max sources (charges or dipoles) held resident in shared memory
 size_t topo_resident_limit(int prec, int source = kCharges);

@@ -831,16 +831,16 @@ cudaError_t launch_topo(int prec, const TopoParams& p_in, int num_sms, cudaStrea
   f0.resident = topo_resident_count(prec, p.source, f0.n_pad);
   f0.team_resident = topo_team_resident(prec, p.source, f0.n_pad);
   f0.left_off = 0;
-  f0.left_cap = p.left ? topo_left_capacity(num_sms, p.n_lines) : 0;
   f0.step = p.step;
   for (int k = 0; k < 3; ++k) f0.half[k] = p.half[k];
   p.frames = nullptr;
   p.n_frames = 1;
   p.max_resident_pad = f0.resident;
   p.max_team_resident = f0.team_resident;
-  if (p.n_lines <= int64_t(num_sms) * kTeamLinesPerSm)
-    return launch_topo_team(prec, p, f0, 1, num_sms, s);
   const bool whole = f0.resident == f0.n_pad;
+  const bool fresh = topo_fresh(prec, whole, p.n_lines, num_sms, p.left != nullptr);
+  f0.left_cap = p.left ? topo_left_capacity(num_sms, p.n_lines, fresh) : 0;
+  if (fresh) return launch_topo_team(prec, p, f0, 1, num_sms, s);
   const int slots = tuned_topo_slots(prec, whole, p.n_lines);
   const cudaError_t e = p.source == kDipoles
                             ? launch_topo_prec<true>(prec, whole, p, f0, num_sms, s, slots)
@@ -849,15 +849,32 @@ cudaError_t launch_topo(int prec, const TopoParams& p_in, int num_sms, cudaStrea
   return launch_topo_team(prec, p, f0, 0, num_sms, s);
 }
 
-int topo_left_capacity(int num_sms, int64_t n_lines) {
-  // what the CTAs of one launch may hold when they hand over
-  return static_cast<int>(std::min(n_lines, int64_t(num_sms) * kTeamLinesPerSm));
+// Up to 16 lines per SM the persistent kernel has less than a line per warp.  Above
+// that, all lines kept in the rounds of teams, against the persistent kernel and
+// rounds for its last lines (GB300, lines per SM: ms, box of 3 A, ends at the box):
+//   FP64    1,000 charges  24: 21.6 against 27.7   64: 54.1 / 62.4   256: 198 / 213
+//           4,000 charges, 52 steps across the box  24: 7.3 / 7.8  128: 31.7 / 34.9
+//   FP32C   3,000 charges  17: 17.2 / 19.6  20: 18.9 / 20.6  24: 21.6 / 21.8  33: 26.3 / 24.5
+//           8,000 charges  17: 19.9 / 22.4  24: 25.4 / 27.9  48: 44.4 / 40.1
+//           40,000 charges 17: 49.5 / 63.4  24: 64.3 / 76.6  33: 87.9 / 96.6, larger
+//           steps  33: 19.6 / 20.4  40: 23.6 / 22.3
+// A team has the FP64 pipe busy with a line per warp; in FP32C the persistent kernel
+// reaches the pipe's rate from 32 lines per SM on, later where sources come from L2.
+bool topo_fresh(int prec, bool resident, int64_t sum_lines, int num_sms, bool lists) {
+  int64_t per_sm = kTeamLinesPerSm;
+  if (lists) per_sm = prec == kFP64 ? kMaxLeft : (resident ? 20 : 32);
+  return sum_lines <= std::min(per_sm * num_sms, std::max(kMaxLeft, int64_t(kTeamLinesPerSm) * num_sms));
+}
+
+int topo_left_capacity(int num_sms, int64_t n_lines, bool fresh) {
+  // every line, or what the CTAs of one launch may hold when they hand over
+  return static_cast<int>(fresh ? n_lines : std::min(n_lines, int64_t(num_sms) * kTeamLinesPerSm));
 }
 
 cudaError_t launch_topo_frames(int prec, const TopoParams& p, int num_sms, cudaStream_t s) {
   if (p.n_frames <= 0 || p.n_lines <= 0) return cudaSuccess;
   TopoFrame dummy{};
-  if (p.sum_lines <= int64_t(num_sms) * kTeamLinesPerSm)
+  if (topo_fresh(prec, p.all_resident != 0, p.sum_lines, num_sms, p.left != nullptr))
     return launch_topo_team(prec, p, dummy, 1, num_sms, s);
   const int slots = tuned_topo_slots(prec, p.all_resident != 0, p.n_lines);
   const cudaError_t e = launch_topo_prec<false>(prec, p.all_resident != 0, p, dummy, num_sms, s, slots);

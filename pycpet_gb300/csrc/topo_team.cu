@@ -404,8 +404,9 @@ __device__ __forceinline__ void team_lines(const TopoParams& p, const TopoFrame&
 }
 
 // Items are (frame, up to `chunk` lines); CTA b takes items b, b + gridDim.x, ...
-// chunk is the smallest line count per item for which all items fit one wave of
-// CTAs (at most kTeamLinesPerSm), so the lines are spread evenly over the SMs.
+// chunk is the smallest line count per item for which all items fit the waves of
+// CTAs that kTeamLinesPerSm lines each would need, so the lines are spread evenly
+// over the SMs.
 template <int PREC, bool DIP>
 __global__ void __launch_bounds__(kTeams* kTeamThreads, 1)
     team_kernel(TopoParams p, TopoFrame frame0, int fresh, int round) {
@@ -439,12 +440,14 @@ __global__ void __launch_bounds__(kTeams* kTeamThreads, 1)
     long long total = 0;
     for (int f = lane; f < n_frames; f += 32) total += count_of(f);
     for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-    int chunk = total > 0 ? static_cast<int>(min((total + G - 1) / G, (long long)kTeamLinesPerSm)) : 0;
+    const long long wave = static_cast<long long>(G) * kTeamLinesPerSm;
+    const long long slots = G * ((total + wave - 1) / wave);
+    int chunk = total > 0 ? static_cast<int>((total + slots - 1) / slots) : 0;
     while (chunk > 0 && chunk < kTeamLinesPerSm) {
       long long items = 0;
       for (int f = lane; f < n_frames; f += 32) items += (count_of(f) + chunk - 1) / chunk;
       for (int o = 16; o > 0; o >>= 1) items += __shfl_xor_sync(0xffffffffu, items, o);
-      if (items <= G) break;
+      if (items <= slots) break;
       ++chunk;
     }
     if (lane == 0) s_chunk = chunk;
