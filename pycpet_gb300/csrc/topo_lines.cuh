@@ -463,8 +463,11 @@ __device__ __forceinline__ void sweep_slots(int na, const float (&posf)[3], cons
     if constexpr (SRC == kSrcShared) {
       total = sweep_shared<NA, DIP>(pt, sm_off, g, n_pairs);
     } else {
-      // about eight independent pair chains in flight per lane: unroll 8 / NA
-      constexpr int kFull = NA >= 3 ? 2 : (NA == 2 ? 4 : 8);
+      // about eight independent pair chains in flight per lane: unroll 8 / NA; twice
+      // that for four lines on global memory alone (the serving engine, 48,000
+      // lines of 8,000 and 20,000 charges: 0.750 s against 0.785, two CTAs per SM
+      // 0.54 against 0.58; from shared and global memory both run alike)
+      constexpr int kFull = NA == 4 && SRC == kSrcGlobal ? 4 : (NA >= 3 ? 2 : (NA == 2 ? 4 : 8));
       total = sweep_frame<NA, DIP, SRC, kFull, 1>(pt, sm_off, res_pairs, g, n_pairs);
     }
   };
