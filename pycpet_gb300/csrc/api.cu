@@ -171,21 +171,40 @@ Ctx* context(int* rc) {
 struct Scratch {
   cudaStream_t s;
   std::vector<void*> ptrs;
+  unsigned char* block = nullptr;  // what is left of the last reserve()
+  size_t left = 0;
   explicit Scratch(cudaStream_t st) : s(st) {}
   ~Scratch() {
     for (void* p : ptrs) cudaFreeAsync(p, s);
   }
+  static size_t bytes_of(size_t bytes) { return (std::max<size_t>(bytes, 1) + 255) / 256 * 256; }
+  // One allocation for the get() calls that follow, up to `bytes` of bytes_of() sums
+  // (an allocation and its release cost a call about 1.5 us).
+  cudaError_t reserve(size_t bytes) {
+    void* v = nullptr;
+    const cudaError_t e = cudaMallocAsync(&v, bytes_of(bytes), s);
+    if (e != cudaSuccess) return e;
+    ptrs.push_back(v);
+    block = static_cast<unsigned char*>(v);
+    left = bytes_of(bytes);
+    return e;
+  }
   template <typename T>
   cudaError_t get(T** p, size_t count) {
     *p = nullptr;
-    if (count == 0) count = 1;
-    void* v = nullptr;
-    cudaError_t e = cudaMallocAsync(&v, ((count * sizeof(T) + 255) / 256) * 256, s);
-    if (e == cudaSuccess) {
+    const size_t need = bytes_of(count * sizeof(T));
+    if (need > left) {
+      void* v = nullptr;
+      const cudaError_t e = cudaMallocAsync(&v, need, s);
+      if (e != cudaSuccess) return e;
       ptrs.push_back(v);
       *p = static_cast<T*>(v);
+      return e;
     }
-    return e;
+    *p = reinterpret_cast<T*>(block);
+    block += need;
+    left -= need;
+    return cudaSuccess;
   }
 };
 
@@ -285,7 +304,6 @@ double grid_pair_evals(int n_frames, const int64_t* desc) {
 struct GridTable {
   std::vector<GridFrame> frames;
   int64_t n_items = 0, n_tiles = 0, n_prep = 0, few_items = 0, n_slots = 0;
-  int n_few = 0;
 };
 
 int plan_grid(int prec, int n_frames, const int64_t* desc, int sms, int ppt, int items_per_sm, GridTable& t) {
@@ -343,7 +361,6 @@ int plan_grid(int prec, int n_frames, const int64_t* desc, int sms, int ppt, int
     t.n_tiles += fr.n_tiles;
     if (fr.n_split > 1) t.n_slots += items;
     if (fr.few) {
-      ++t.n_few;
       t.few_items += items;
     } else if (mesh) {
       t.n_prep += (int64_t(fr.n_points) + kGridPrepPoints - 1) / kGridPrepPoints;
@@ -381,7 +398,6 @@ GridLaunch grid_launch(int kind, int prec, int clamp, int ppt, int n_frames, con
   g.n_items = static_cast<int>(t.n_items);
   g.n_tiles = static_cast<int>(t.n_tiles);
   g.n_prep = static_cast<int>(t.n_prep);
-  g.n_few = t.n_few;
   g.few_items = static_cast<int>(t.few_items);
   g.n_charges = tot_ch;
   g.max_points = static_cast<int>(max_frame_points(n_frames, desc));
@@ -396,43 +412,69 @@ GridLaunch grid_launch(int kind, int prec, int clamp, int ppt, int n_frames, con
   return g;
 }
 
-// A grid launch on device arrays, its scratch from S (released after it on the stream).
-int grid_device(int kind, int prec, int clamp, int n_frames, const int64_t* desc, int64_t tot_ch,
-                const double* pts, const double* x, const double* q, double* out, const Ctx* c, Scratch& S) {
+// A grid launch's plan, and its scratch (from S, released after it on the stream).
+struct GridWork {
   GridTable plan;
-  int ppt = 4, ips = 8;
-  tuned_grid_shape(prec, kind, grid_pair_evals(n_frames, desc), &ppt, &ips);
-  const int rc = plan_grid(prec, n_frames, desc, c->sms, ppt, ips, plan);
-  if (rc != CPETGB_OK) return rc;
-  GridLaunch g = grid_launch(kind, prec, clamp, ppt, n_frames, desc, plan, tot_ch, c);
-  g.points = pts;
-  g.x = x;
-  g.q = q;
-  g.out = out;
-  if (grid_point_fits(g)) {
-    CK(launch_grid_point(g, S.s), "point kernel launch");
-  } else {
-    GridFrame* d_frames = nullptr;
+  GridLaunch g{};
+  int ppt = 4;
+  bool point = false;  // one kernel, no scratch
+  size_t n_list = 0;
+  size_t zero_ints() const { return grid_zero_ints(g.n_frames, g.tau > 0.0); }
+  size_t packed_bytes() const { return size_t(std::max<int64_t>(g.n_charges, 1)) * kGridRecord; }
+  size_t partial_doubles() const { return size_t(plan.n_slots) * grid_slot_doubles(g.kind, ppt); }
+  size_t scratch_bytes() const {
+    if (point) return 0;
+    size_t b = Scratch::bytes_of(packed_bytes()) + Scratch::bytes_of(zero_ints() * sizeof(int));
+    if (g.n_frames != 1) b += Scratch::bytes_of(plan.frames.size() * sizeof(GridFrame));
+    if (plan.n_slots) b += Scratch::bytes_of(partial_doubles() * sizeof(double));
+    if (g.tau > 0.0)
+      b += Scratch::bytes_of(n_list * sizeof(int64_t)) + Scratch::bytes_of(size_t(g.n_charges) * 32);
+    return b;
+  }
+  int prepare(int kind, int prec, int clamp, int n_frames, const int64_t* desc, int64_t tot_ch, const Ctx* c) {
+    int ips = 8;
+    tuned_grid_shape(prec, kind, grid_pair_evals(n_frames, desc), &ppt, &ips);
+    const int rc = plan_grid(prec, n_frames, desc, c->sms, ppt, ips, plan);
+    if (rc != CPETGB_OK) return rc;
+    g = grid_launch(kind, prec, clamp, ppt, n_frames, desc, plan, tot_ch, c);
+    point = grid_point_fits(g);
+    n_list = g.tau > 0.0 ? size_t(refine_list_len(n_frames, desc)) * 2 : 0;
+    return CPETGB_OK;
+  }
+  int allocate(Scratch& S) {
+    if (point) return CPETGB_OK;
     unsigned char* packed = nullptr;
-    CK(S.get(&packed, size_t(std::max<int64_t>(tot_ch, 1)) * kGridRecord), "alloc packed charges");
+    CK(S.get(&packed, packed_bytes()), "alloc packed charges");
     if (reinterpret_cast<uintptr_t>(packed) % 16 != 0)  // bulk async copies need 16-byte sources
       return fail(CPETGB_ECUDA, "scratch allocation is not 16-byte aligned");
     g.packed = packed;
-    CK(h2d(&d_frames, S, plan.frames.data(), plan.frames.size()), "copy frame table");
-    g.frames = d_frames;
-    CK(S.get(&g.zeroed, grid_zero_ints(n_frames, g.tau > 0.0)), "alloc counters");
-    if (plan.n_slots)
-      CK(S.get(&g.partial, size_t(plan.n_slots) * grid_slot_doubles(kind, ppt)), "alloc partial sums");
+    if (g.n_frames != 1) {
+      GridFrame* d_frames = nullptr;
+      CK(h2d(&d_frames, S, plan.frames.data(), plan.frames.size()), "copy frame table");
+      g.frames = d_frames;
+    }
+    CK(S.get(&g.zeroed, zero_ints()), "alloc counters");
+    if (plan.n_slots) CK(S.get(&g.partial, partial_doubles()), "alloc partial sums");
     if (g.tau > 0.0) {
       unsigned char* dfq = nullptr;
-      CK(S.get(&g.list, size_t(refine_list_len(n_frames, desc)) * 2), "alloc refinement list");
-      CK(S.get(&dfq, size_t(tot_ch) * 32), "alloc double-float charges");
+      CK(S.get(&g.list, n_list), "alloc refinement list");
+      CK(S.get(&dfq, size_t(g.n_charges) * 32), "alloc double-float charges");
       g.dfq = dfq;
     }
-    CK(launch_grid(g, S.s), "grid launch");
+    return CPETGB_OK;
   }
-  return CPETGB_OK;
-}
+  int launch(const double* pts, const double* x, const double* q, double* out, cudaStream_t s, bool cleared) {
+    g.points = pts;
+    g.x = x;
+    g.q = q;
+    g.out = out;
+    if (point)
+      CK(launch_grid_point(g, s), "point kernel launch");
+    else
+      CK(launch_grid(g, s, cleared), "grid launch");
+    return CPETGB_OK;
+  }
+};
 
 int grid_batch_impl(int kind, int prec, int mem, int clamp, int n_frames, const int64_t* desc,
                     const double* pts, const double* x, const double* q, double* out,
@@ -459,7 +501,13 @@ int grid_batch_impl(int kind, int prec, int mem, int clamp, int n_frames, const 
   if (mem == CPETGB_HOST && !s) s = c->stream;
   const int NC = kind == CPETGB_FIELD ? 3 : 1;
 
+  GridWork w;
+  rc = w.prepare(kind, prec, clamp, n_frames, desc, tot_ch, c);
+  if (rc != CPETGB_OK) return rc;
   Scratch S(s);
+  if (!w.point) CK(S.reserve(w.scratch_bytes()), "alloc scratch");
+  rc = w.allocate(S);
+  if (rc != CPETGB_OK) return rc;
   const double *dp = pts, *dx = x, *dq = q;
   double* dout = out;
   if (mem == CPETGB_HOST) {
@@ -470,7 +518,7 @@ int grid_batch_impl(int kind, int prec, int mem, int clamp, int n_frames, const 
     }
     CK(S.get(&dout, size_t(tot_pts) * NC), "alloc output");
   }
-  rc = grid_device(kind, prec, clamp, n_frames, desc, tot_ch, dp, dx, dq, dout, c, S);
+  rc = w.launch(dp, dx, dq, dout, s, false);
   if (rc != CPETGB_OK) return rc;
   if (mem == CPETGB_HOST) {
     CK(cudaMemcpyAsync(out, dout, size_t(tot_pts) * NC * sizeof(double), cudaMemcpyDeviceToHost, s),
@@ -498,8 +546,15 @@ int grid_f32_impl(int kind, int prec, int clamp, int P, int N, const float* pts,
       fmt == kRowsField ? size_t(P) * 24 : (fmt == kRowsEspHalf ? size_t(P) * 8 : n_val * sizeof(float));
   const size_t out_bytes = ((row_bytes + 15) & ~size_t(15)) + 16;  // the status word behind the rows
   const size_t in_bytes = (n_in * sizeof(float) + 255) & ~size_t(255);
+  const int64_t desc[4] = {0, N, 0, P};
+  GridWork w;
+  rc = w.prepare(kind, prec, clamp, 1, desc, N, c);
+  if (rc != CPETGB_OK) return rc;
   Staging host(in_bytes + out_bytes, s);
   Scratch S(s);
+  CK(S.reserve(w.scratch_bytes() + Scratch::bytes_of(n_in * sizeof(float)) + Scratch::bytes_of(n_in * sizeof(double)) +
+               Scratch::bytes_of(n_val * sizeof(double)) + Scratch::bytes_of(out_bytes)),
+     "alloc scratch");
   float* d_in = nullptr;
   double *d64 = nullptr, *d_val = nullptr;
   unsigned char* d_rows = nullptr;
@@ -507,6 +562,8 @@ int grid_f32_impl(int kind, int prec, int clamp, int P, int N, const float* pts,
   CK(S.get(&d64, n_in), "alloc inputs");
   CK(S.get(&d_val, n_val), "alloc output");
   CK(S.get(&d_rows, out_bytes), "alloc rows");
+  rc = w.allocate(S);
+  if (rc != CPETGB_OK) return rc;
   if (host.p) {
     float* h = static_cast<float*>(host.p);
     std::memcpy(h, pts, np * sizeof(float));
@@ -522,9 +579,10 @@ int grid_f32_impl(int kind, int prec, int clamp, int P, int N, const float* pts,
       CK(cudaMemcpyAsync(d_in + np + nx, q, nq * sizeof(float), cudaMemcpyHostToDevice, s), "copy charges");
     }
   }
-  CK(launch_widen(static_cast<int64_t>(n_in), d_in, d64, s), "widen inputs");
-  const int64_t desc[4] = {0, N, 0, P};
-  rc = grid_device(kind, prec, clamp, 1, desc, N, d64, d64 + np, d64 + np + nx, d_val, c, S);
+  CK(launch_widen(static_cast<int64_t>(n_in), d_in, d64, w.g.zeroed,
+                  w.point ? 0 : static_cast<int64_t>(w.zero_ints()), s),
+     "widen inputs");
+  rc = w.launch(d64, d64 + np, d64 + np + nx, d_val, s, true);
   if (rc != CPETGB_OK) return rc;
   int* tail = reinterpret_cast<int*>(d_rows + out_bytes - 16);
   CK(launch_rows(fmt, fmt == kRowsPlain ? static_cast<int64_t>(n_val) : P, d_in, d_val, d_rows, c->status, tail, s),

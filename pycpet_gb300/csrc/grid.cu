@@ -962,11 +962,12 @@ constexpr int kRefineThreads = 512;
 // The counts behind the scale are exact integers, so the threshold and the set
 // of points are deterministic.
 __global__ void __launch_bounds__(kFlagThreads)
-    grid_flag_kernel(const GridFrame* __restrict__ frames, const double* __restrict__ out,
+    grid_flag_kernel(const GridFrame* __restrict__ frames, const GridFrame one, const double* __restrict__ out,
                      const float* __restrict__ scale, float tau2, int64_t* __restrict__ list,
                      int* __restrict__ count) {
   __shared__ int part[kFlagThreads / 32 + 1];
-  const int64_t po = frames[blockIdx.x].point_off, P = frames[blockIdx.x].n_points;
+  const int64_t po = gridDim.x == 1 ? one.point_off : frames[blockIdx.x].point_off;
+  const int64_t P = gridDim.x == 1 ? one.n_points : frames[blockIdx.x].n_points;
   const float thr = __fmul_rn(tau2, scale[blockIdx.x]);
   constexpr int kPer = kFlagChunk / kFlagThreads;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1111,7 +1112,7 @@ __device__ __forceinline__ void df_add(float& h, float& l, float bh, float bl) {
 // by a fixed tree.
 template <bool CLAMP>
 __global__ void __launch_bounds__(kRefineThreads, 2)
-    grid_refine_kernel(const GridFrame* __restrict__ frames, const int64_t* __restrict__ list,
+    grid_refine_kernel(const GridFrame* __restrict__ frames, const GridFrame one, const int64_t* __restrict__ list,
                        const int* __restrict__ count, const double* __restrict__ points,
                        const float4* __restrict__ dfq, double* __restrict__ out) {
   __shared__ float red[kRefineThreads / 32][6];
@@ -1120,8 +1121,8 @@ __global__ void __launch_bounds__(kRefineThreads, 2)
   for (int e = blockIdx.x; e < n_list; e += gridDim.x) {
     const int64_t row = list[2 * e];
     const int64_t f = list[2 * e + 1];
-    const int64_t co = frames[f].charge_off;
-    const int n = frames[f].n_charges;
+    const int64_t co = frames ? frames[f].charge_off : one.charge_off;
+    const int n = frames ? frames[f].n_charges : one.n_charges;
     const float4* src = dfq + 2 * co;
     float ph[3], pl[3];
 #pragma unroll
@@ -1338,10 +1339,10 @@ cudaError_t launch_grid_c(const GridLaunch& g, cudaStream_t s) {
     if constexpr (KIND == kField && PREC == kFP32C) {
       final_lanes(std::true_type{});
       const dim3 fgrid(g.n_frames, std::min((g.max_points - 1) / kFlagChunk + 1, 65535));
-      grid_flag_kernel<<<fgrid, kFlagThreads, 0, s>>>(g.frames, g.out, z.scale,
+      grid_flag_kernel<<<fgrid, kFlagThreads, 0, s>>>(g.frames, g.one, g.out, z.scale,
                                                       static_cast<float>(g.tau * g.tau), g.list, z.count);
       grid_refine_kernel<CLAMP><<<std::max(g.num_sms, 1) * 4, kRefineThreads, 0, s>>>(
-          g.frames, g.list, z.count, g.points, dfq, g.out);
+          g.n_frames == 1 ? nullptr : g.frames, g.one, g.list, z.count, g.points, dfq, g.out);
     }
   } else if (g.partial) {
     final_lanes(std::false_type{});
@@ -1429,9 +1430,9 @@ size_t grid_zero_ints(int n_frames, bool refine) {
   return size_t((4 * n_frames + 1 + 3) & ~3) + (refine ? size_t(n_frames) * kMagBins : 0);
 }
 
-cudaError_t launch_grid(const GridLaunch& g, cudaStream_t s) {
+cudaError_t launch_grid(const GridLaunch& g, cudaStream_t s, bool cleared) {
   if (g.n_items <= 0) return cudaSuccess;
-  if (g.n_prep > 0 || g.tau > 0.0) {
+  if (!cleared && (g.n_prep > 0 || g.tau > 0.0)) {
     const cudaError_t e =
         cudaMemsetAsync(g.zeroed, 0, grid_zero_ints(g.n_frames, g.tau > 0.0) * sizeof(int), s);
     if (e != cudaSuccess) return e;

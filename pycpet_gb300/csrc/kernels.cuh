@@ -68,17 +68,16 @@ static_assert(sizeof(GridFrame) == 64, "GridFrame layout");
 // A grid launch.  Scratch (device): packed 32 bytes per charge; partial
 // n_slots * grid_slot_doubles(kind, ppt); lattice and, for the refinement, list
 // (2 int64 per point) and dfq (32 bytes per charge); zeroed: grid_zero_ints()
-// ints, cleared by launch_grid.
+// ints, cleared by launch_grid unless the caller has (cleared).
 struct GridLaunch {
   int prec, kind, clamp, ppt;
   int n_frames;
-  const GridFrame* frames;    // device
-  GridFrame one;              // the frame itself when n_frames == 1 (saves its kernels the table's loads)
+  const GridFrame* frames;    // device; not read when n_frames == 1
+  GridFrame one;              // the frame itself when n_frames == 1 (no table to copy, none to load)
   int n_items;                // items of all frames
   int n_tiles;
   int n_prep;                 // preparation blocks of all frames (0: no look for meshes)
-  int n_few;                  // frames with few != 0 (they come first: their items precede the others)
-  int few_items;              // items of those frames
+  int few_items;              // items of the frames with few != 0 (they come first)
   int64_t n_charges;          // extent of x / q
   int max_points;             // largest frame
   const double *points, *x, *q;
@@ -101,7 +100,7 @@ size_t grid_zero_ints(int n_frames, bool refine);
 // in one kernel, without scratch (g.one, points, x, q, out set).
 bool grid_point_fits(const GridLaunch& g);
 cudaError_t launch_grid_point(const GridLaunch& g, cudaStream_t s);
-cudaError_t launch_grid(const GridLaunch& g, cudaStream_t s);
+cudaError_t launch_grid(const GridLaunch& g, cudaStream_t s, bool cleared = false);
 // Loads the module code of the grid kernels (before a graph capture).
 cudaError_t preload_grid_kernels(int prec, int kind, int clamp, int ppt);
 // Packs x[n][3], q[n] as Charge64 (the FP64 streamline layout) and fills [n,
@@ -210,9 +209,10 @@ cudaError_t launch_pack_topo(int prec, int64_t n, int64_t n_pad, const double* x
 cudaError_t launch_wait_limit_check(int* status, unsigned long long limit_ns, cudaStream_t s);
 
 // rows.cu: conversions of the float32 host calls.  launch_rows writes n float32
-// values (kRowsPlain) or n points' rows, and copies the status word to *tail.
+// values (kRowsPlain) or n points' rows, and copies the status word to *tail;
+// launch_widen also clears n_zero ints.
 enum RowFormat : int { kRowsPlain = 0, kRowsField = 1, kRowsEspHalf = 2 };
-cudaError_t launch_widen(int64_t n, const float* in, double* out, cudaStream_t s);
+cudaError_t launch_widen(int64_t n, const float* in, double* out, int* zeroed, int64_t n_zero, cudaStream_t s);
 cudaError_t launch_rows(int fmt, int64_t n, const float* pts, const double* val, void* rows, const int* status,
                         int* tail, cudaStream_t s);
 

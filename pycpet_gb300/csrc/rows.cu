@@ -15,9 +15,13 @@ namespace {
 
 constexpr int kRowThreads = 256;
 
-__global__ void widen_kernel(int64_t n, const float* __restrict__ in, double* __restrict__ out) {
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
-    out[i] = widen(in[i]);
+// Also clears the counters of the launch that follows (a memset of its own is one
+// more operation on the stream).
+__global__ void widen_kernel(int64_t n, const float* __restrict__ in, double* __restrict__ out,
+                             int* __restrict__ zeroed, int64_t n_zero) {
+  const int64_t i0 = blockIdx.x * int64_t(blockDim.x) + threadIdx.x, stride = int64_t(gridDim.x) * blockDim.x;
+  for (int64_t i = i0; i < n_zero; i += stride) zeroed[i] = 0;
+  for (int64_t i = i0; i < n; i += stride) out[i] = widen(in[i]);
 }
 
 // The device status word goes behind the rows, so that one copy brings both.
@@ -45,9 +49,9 @@ int blocks_of(int64_t n) { return static_cast<int>(std::max<int64_t>(1, std::min
 
 }  // namespace
 
-cudaError_t launch_widen(int64_t n, const float* in, double* out, cudaStream_t s) {
-  if (n <= 0) return cudaSuccess;
-  widen_kernel<<<blocks_of(n), kRowThreads, 0, s>>>(n, in, out);
+cudaError_t launch_widen(int64_t n, const float* in, double* out, int* zeroed, int64_t n_zero, cudaStream_t s) {
+  if (n <= 0 && n_zero <= 0) return cudaSuccess;
+  widen_kernel<<<blocks_of(std::max(n, n_zero)), kRowThreads, 0, s>>>(n, in, out, zeroed, n_zero);
   return cudaGetLastError();
 }
 
