@@ -18,7 +18,7 @@
 // once per charge instead of once per point and charge, in the same order of
 // operations, so the sums are the same bits.  That is 9 instead of 12 FP32-pipe
 // operations per pair (4 instead of 7 for the potential, which is then bound by
-// the MUFU alone), 10 FP64-pipe instructions instead of 13.  The points that do
+// the MUFU alone), 9 FP64-pipe instructions instead of 12.  The points that do
 // not fill a column's last group are evaluated as points without a mesh.
 //
 // Precision forms:
@@ -502,8 +502,8 @@ __global__ void __launch_bounds__(kGridThreads, PREC == kFP32C && PPT == 4 ? (KI
         }
       };
       // the clamp in a loop of its own: as a condition in the others its comparison
-      // is evaluated for every pair (11 FP64-pipe instructions instead of 10; 9,261
-      // points x 5,000 charges 1,115 us, 1,011 so)
+      // is evaluated for every pair (one FP64-pipe instruction more; 9,261 points x
+      // 5,000 charges 1,115 us against 1,011 when a pair took 10 of them)
       if (CLAMP && clamp_tile) {
         points(std::true_type{});
       } else if (column) {

@@ -484,7 +484,7 @@ __device__ __forceinline__ void sweep_slots(int na, const float (&posf)[3], cons
 }
 
 // FP64.  Bound: the FP64 pipe (64 cycles per warp instruction); a charge pair
-// takes 13 of its instructions (3 differences, 3 for r^2, 4 for q r^-3 with
+// takes 12 of its instructions (3 differences, 3 for r^2, 3 for q r^-3 with
 // common.cuh's seed, 3 sums) where rsqrt() and three products took 19.  A run
 // is kLaneRun64 charges per lane, summed plainly; the runs are added in order.
 template <int NA, int S>
@@ -507,7 +507,7 @@ __device__ __forceinline__ void run_f64(const Charge64* __restrict__ g, int base
   }
 }
 
-// FP64 dipoles: the term of dipole_terms, r^-5 dot R - r^-3 mu (22 FP64-pipe
+// FP64 dipoles: the term of dipole_terms, r^-5 dot R - r^-3 mu (21 FP64-pipe
 // instructions, 29 with rsqrt()).
 template <int NA, int S>
 __device__ __forceinline__ void run_f64(const Dipole64* __restrict__ g, int base, int cnt,

@@ -3,7 +3,7 @@ inside r^2 = 2^-100 .. 2^100, the plain form outside) against Coulomb's law in
 extended precision, over distances on both sides of that range and next to
 powers of two.
 
-Tolerance: 1.2e-15 relative.  The weight is off by at most 2.5 units of 2^-53
+Tolerance: 1.2e-15 relative.  The weight is off by at most 3.8 units of 2^-53
 inside the range and 5.5 outside, r^2 by one (x 1.5), the products with the
 component and with the Coulomb constant by one each: 10 units, 1.1e-15."""
 import numpy as np
