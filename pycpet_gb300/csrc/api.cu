@@ -65,21 +65,28 @@ int cuda_fail(cudaError_t e, const char* what) {
     if (e_ != cudaSuccess) return cuda_fail(e_, what); \
   } while (0)
 
-// Pinned staging buffers of the float32 host calls: at most kStagingBytes in all per
-// process, of which kStagingIdle stay for the next calls; a call that gets none copies
-// from and to the caller's pageable arrays.  A buffer belongs to one call at a time
-// (any thread, any stream) and goes back after the call has waited for its copies.
-constexpr size_t kStagingBytes = size_t(64) << 20;
-constexpr size_t kStagingIdle = size_t(16) << 20;
+// Pinned staging buffers of the float32 host calls: kStagingBuffers of kStagingBytes
+// for the whole process, allocated together on the first such call or with the first
+// engine, and never during another call: page-locking memory waits for kernels in
+// flight (2.6 s behind a busy streamline engine).  A call that is larger, or that finds
+// no buffer free, copies from and to the caller's pageable arrays.  A buffer belongs
+// to one call at a time (any thread, any stream) and goes back after the call has
+// waited for its copies.  8 MB hold a call of 51^3 points and 100,000 charges.
+constexpr int kStagingBuffers = 2;
+constexpr size_t kStagingBytes = size_t(8) << 20;
 struct StagingPool {
   std::mutex mu;
-  std::vector<std::pair<void*, size_t>> idle;
-  size_t total = 0, idle_bytes = 0;
-  void drop(size_t i) {
-    cudaFreeHost(idle[i].first);
-    total -= idle[i].second;
-    idle_bytes -= idle[i].second;
-    idle.erase(idle.begin() + static_cast<std::ptrdiff_t>(i));
+  void* buf[kStagingBuffers] = {};
+  bool busy[kStagingBuffers] = {};
+  bool made = false;
+  void make() {  // (mu held)
+    if (made) return;
+    made = true;
+    for (void*& b : buf)
+      if (cudaHostAlloc(&b, kStagingBytes, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        b = nullptr;
+      }
   }
 };
 StagingPool& staging_pool() {
@@ -89,42 +96,27 @@ StagingPool& staging_pool() {
 
 struct Staging {
   void* p = nullptr;
-  size_t size = size_t(1) << 18;
+  int index = -1;
   cudaStream_t stream;
   bool waited = false;  // set once no copy to or from the buffer is in flight
   Staging(size_t need, cudaStream_t s) : stream(s) {
     if (need > kStagingBytes) return;
-    while (size < need) size *= 2;
     StagingPool& pool = staging_pool();
     std::lock_guard<std::mutex> lock(pool.mu);
-    size_t best = pool.idle.size();
-    for (size_t i = 0; i < pool.idle.size(); ++i)
-      if (pool.idle[i].second >= need && (best == pool.idle.size() || pool.idle[i].second < pool.idle[best].second))
-        best = i;
-    if (best < pool.idle.size()) {
-      p = pool.idle[best].first;
-      size = pool.idle[best].second;
-      pool.idle_bytes -= size;
-      pool.idle.erase(pool.idle.begin() + static_cast<std::ptrdiff_t>(best));
-      return;
-    }
-    while (pool.total + size > kStagingBytes && !pool.idle.empty()) pool.drop(pool.idle.size() - 1);
-    if (pool.total + size > kStagingBytes) return;
-    if (cudaHostAlloc(&p, size, cudaHostAllocPortable) != cudaSuccess) {
-      cudaGetLastError();
-      p = nullptr;
-      return;
-    }
-    pool.total += size;
+    pool.make();
+    for (int i = 0; i < kStagingBuffers && !p; ++i)
+      if (pool.buf[i] && !pool.busy[i]) {
+        pool.busy[i] = true;
+        p = pool.buf[i];
+        index = i;
+      }
   }
   ~Staging() {
     if (!p) return;
     if (!waited) cudaStreamSynchronize(stream);
     StagingPool& pool = staging_pool();
     std::lock_guard<std::mutex> lock(pool.mu);
-    pool.idle.emplace_back(p, size);
-    pool.idle_bytes += size;
-    if (pool.idle_bytes > kStagingIdle) pool.drop(pool.idle.size() - 1);
+    pool.busy[index] = false;
   }
   Staging(const Staging&) = delete;
   Staging& operator=(const Staging&) = delete;
@@ -1289,6 +1281,12 @@ int topo_plan_impl(cpetgb_plan** out_plan, int prec, int F, const int64_t* desc,
 }  // namespace
 
 int cpetgb::set_error(int code, const char* msg) { return fail(code, "%s", msg); }
+
+void cpetgb::make_staging() {
+  StagingPool& pool = staging_pool();
+  std::lock_guard<std::mutex> lock(pool.mu);
+  pool.make();
+}
 
 int cpetgb::tuned_topo_slots(int prec, bool resident, int n_lines) {
   const int v = tune_choose(tune_key(kOpTopo, prec, resident ? 1 : 0, double(n_lines)));

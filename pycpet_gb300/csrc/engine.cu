@@ -264,6 +264,10 @@ int cpetgb_engine_create(cpetgb_engine** out, int precision, int64_t charge_capa
   if (err == cudaSuccess) err = cudaHostGetDevicePointer(&e->d_chunks, e->chunks, 0);
   if (err == cudaSuccess) err = cudaHostGetDevicePointer(&e->d_counters, e->counters, 0);
   if (err == cudaSuccess) err = cudaHostGetDevicePointer(&e->d_done, e->done, 0);
+  // grid calls run beside the engine's kernel; none of them may load code or lock pages
+  if (err == cudaSuccess) err = preload_grid_kernels();
+  if (err == cudaSuccess) err = preload_row_kernels();
+  if (err == cudaSuccess) make_staging();
   if (err != cudaSuccess) {
     delete e;
     return ecuda(err, "engine allocation");

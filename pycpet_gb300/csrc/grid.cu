@@ -1373,6 +1373,8 @@ cudaError_t preload_c() {
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, prep_kernel<PREC, false>);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, grid_final_kernel<PREC, KIND, PPT, false, 1>);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, grid_final_kernel<PREC, KIND, PPT, false, kSumLanes>);
+  if constexpr (PREC == kFP32C)
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, grid_point_kernel<KIND, CLAMP>);
   if constexpr (KIND == kField && PREC == kFP32C) {
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, prep_kernel<PREC, true>);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, grid_final_kernel<PREC, KIND, PPT, true, 1>);
@@ -1457,6 +1459,15 @@ cudaError_t preload_grid_kernels(int prec, int kind, int clamp, int ppt) {
       if (clamp) return preload_c<P, K, true, T>();
     return preload_c<P, K, false, T>();
   });
+}
+
+cudaError_t preload_grid_kernels() {
+  cudaError_t e = cudaSuccess;
+  for (int prec : {int(kFP64), int(kFP32C)})
+    for (int ppt : {4, 8})
+      for (int form = 0; form < 3 && e == cudaSuccess; ++form)
+        e = preload_grid_kernels(prec, form < 2 ? kField : kEsp, form == 1, ppt);
+  return e;
 }
 
 cudaError_t launch_pack_f64(int64_t n, int64_t n_pad, const double* x, const double* q, void* packed,

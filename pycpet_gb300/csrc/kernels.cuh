@@ -101,8 +101,11 @@ size_t grid_zero_ints(int n_frames, bool refine);
 bool grid_point_fits(const GridLaunch& g);
 cudaError_t launch_grid_point(const GridLaunch& g, cudaStream_t s);
 cudaError_t launch_grid(const GridLaunch& g, cudaStream_t s, bool cleared = false);
-// Loads the module code of the grid kernels (before a graph capture).
+// Loads the module code of the grid kernels: those of one form (before a graph
+// capture), or all (before a persistent kernel: a first launch loads a kernel's
+// code, which waits until the device is idle).
 cudaError_t preload_grid_kernels(int prec, int kind, int clamp, int ppt);
+cudaError_t preload_grid_kernels();
 // Packs x[n][3], q[n] as Charge64 (the FP64 streamline layout) and fills [n,
 // n_pad) with zero charges placed far outside any box (they contribute exactly
 // zero).
@@ -215,6 +218,9 @@ enum RowFormat : int { kRowsPlain = 0, kRowsField = 1, kRowsEspHalf = 2 };
 cudaError_t launch_widen(int64_t n, const float* in, double* out, int* zeroed, int64_t n_zero, cudaStream_t s);
 cudaError_t launch_rows(int fmt, int64_t n, const float* pts, const double* val, void* rows, const int* status,
                         int* tail, cudaStream_t s);
+cudaError_t preload_row_kernels();  // as preload_grid_kernels()
+// api.cu: allocates the float32 host calls' pinned buffers.
+void make_staging();
 
 // api.cu: records `msg` as the calling thread's last error and returns `code`.
 int set_error(int code, const char* msg);

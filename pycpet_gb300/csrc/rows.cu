@@ -70,4 +70,13 @@ cudaError_t launch_rows(int fmt, int64_t n, const float* pts, const double* val,
   return cudaGetLastError();
 }
 
+cudaError_t preload_row_kernels() {
+  cudaFuncAttributes a;
+  cudaError_t e = cudaFuncGetAttributes(&a, widen_kernel);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, rows_kernel<kRowsPlain>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, rows_kernel<kRowsField>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, rows_kernel<kRowsEspHalf>);
+  return e;
+}
+
 }  // namespace cpetgb
