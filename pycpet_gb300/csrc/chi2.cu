@@ -52,9 +52,7 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
 // MUFU reciprocal, +infinity (of a zero sum) made finite: such a term is
 // 0 * 0 * FLT_MAX = 0, as the definition has it.
 __device__ __forceinline__ float rcp_finite(float x) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return fminf(y, FLT_MAX);
+  return fminf(rcp_mufu(x), FLT_MAX);
 }
 
 __device__ __forceinline__ double pair_value(float s, float c) { return __dsub_rn(widen(s), widen(c)); }

@@ -81,7 +81,10 @@ struct alignas(4 * sizeof(Real)) Feat<Real, 3> {
 __device__ __forceinline__ double chi2_term(double a, double b) {
   const double s = __dadd_rn(a, b);
   const double d = __dsub_rn(a, b);
-  return s != 0.0 ? __ddiv_rn(__dmul_rn(d, d), s) : 0.0;
+  const double t = __dmul_rn(d, d);
+  // (t below 2^900: the quotient's residual stays finite)
+  if (seed_in_range(s) && __double2hiint(t) < (1923 << 20)) return quotient_f64(t, s);
+  return s != 0.0 ? __ddiv_rn(t, s) : 0.0;
 }
 __device__ __forceinline__ double term(const Feat<double, 1>& a, const Feat<double, 1>& b) {
   return chi2_term(a.v, b.v);

@@ -318,7 +318,7 @@ __device__ __forceinline__ void team_lines(const TopoParams& p, const TopoFrame&
   const double half = fr.half[c];
   const float hf = static_cast<float>(half);
   TeamLine ln{};
-  // steps of this round: a share of the box diagonal, at least kTeamMinSteps; no
+  // steps of this launch: a share of the box diagonal, at least kTeamMinSteps; no
   // limit in the last round
   int budget = INT_MAX;
   if (left_out) {
@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(kTeams* kTeamThreads, 1)
   const int team = warp / kTeamWarps, wid = warp % kTeamWarps;
   const int n_frames = p.frames ? p.n_frames : 1;
   const int G = static_cast<int>(gridDim.x);
-  // this round's lines: the frames' tables, or the list of the round before
+  // this launch's lines: the frames' tables, or the list of the launch before
   const bool from_list = !fresh || round > 0;
   const int n_round = fresh ? round - 1 : round;  // lists written before this launch, less one
   const TopoState* in_list = from_list ? p.left + (n_round & 1) * p.left_records : nullptr;

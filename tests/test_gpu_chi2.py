@@ -54,3 +54,23 @@ def test_signed_zeros_negatives_and_non_finite_values(gpu_lib):
         ref = 0.5 * np.where(a + b != 0, (a - b) ** 2 / (a + b), 0.0).sum(-1)
     np.testing.assert_allclose(d[:3, :3], ref, rtol=1e-6, atol=0)
     assert np.all(np.isnan(d[3:, :3])) and np.all(np.isnan(d[:3, 3:])) and np.all(np.diag(d) == 0)
+
+
+def test_fp64_quotients_are_the_divisions(gpu_lib):
+    """Two rows of one bin each give half a quotient (a - b)^2 / (a + b), compared
+    with numpy's division: over sums on both sides of the fast form's range and next
+    to powers of two, squares that overflow or vanish.  Tolerance: one unit of 2^-52
+    (the sum of one term is exact)."""
+    from pycpet_gb300 import chi2_distance_matrix
+
+    rng = np.random.default_rng(5)
+    s = [2.0 ** e for e in range(-110, 111, 3)] + [np.nextafter(2.0 ** e, 0.0) for e in range(-110, 111, 7)]
+    s += list(2.0 ** rng.uniform(-105, 105, 300)) + list(rng.uniform(1e-6, 2.0, 600)) + [1e-310, 1e308, 3.0]
+    s = np.array(s)
+    b = s * rng.random(len(s))
+    a = s - b
+    a[-1], b[-1] = 1e200, -1e200 * (1 - 2.0 ** -50)
+    with np.errstate(all="ignore"):
+        want = 0.5 * ((a - b) ** 2 / (a + b))
+    got = np.array([chi2_distance_matrix(np.array([[x], [y]]), "fp64")[0, 1] for x, y in zip(a, b)])
+    np.testing.assert_allclose(got, want, rtol=2.0 ** -52, atol=5e-324)
