@@ -21,9 +21,10 @@
 // 32 bins or 8-16 points, transposed so that for one feature a thread reads
 // its 4 rows and 4 columns as broadcast loads; each thread owns 4 x 4 matrix
 // entries.
-//   FP64   every operation in IEEE double; the per-point norm is formed as
-//          numpy forms it, (dx*dx + dy*dy) + dz*dz then sqrt, with no fused
-//          multiply-add, so only the order of the final sum differs.
+//   FP64   every operation in IEEE double, the chi2 quotient by quotient_f64 (the
+//          division's bits); the per-point norm is formed as numpy forms it,
+//          (dx*dx + dy*dy) + dz*dz then sqrt, with no fused multiply-add, so only
+//          the order of the final sum differs.
 //   FP32C  values rounded to FP32 once before the launch; field terms use the
 //          MUFU reciprocal square root; each staged chunk is summed plainly and
 //          Kahan-added (Kahan 1965) into a running (sum, compensation) pair.

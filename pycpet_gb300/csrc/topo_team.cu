@@ -41,10 +41,12 @@ constexpr int kTeamThreads = kTeamWarps * 32;
 constexpr int kTeamLines = kTeamLinesPerSm / kTeams;  // lines per team: one per warp in phase B
 constexpr int kTeamUnits = 32;                     // (line, run) sums a team exchanges at a time
 // Rounds: at most kTeamRounds launches, each stepping a kTeamRounds-th of the box
-// diagonal (a line is 0.28 diagonals long on average; about 4% of them reach the
-// last, unlimited round), but at least kTeamMinSteps steps: a round costs about
-// 10 us (launch, charges to shared memory), a step 1 to 3 us.
-constexpr int kTeamRounds = 12;
+// diagonal (a line is 0.28 diagonals long on average, the longest of some thousand
+// 0.75), but at least kTeamMinSteps steps: a round costs about 10 us (launch, charges to
+// shared memory; 3 us once no line is left), a step 1 to 3 us, in FP64 10 and more.
+// 12 rounds against 20 (ms): FP64 1,000 lines x 4,000 charges 82.9 and 77.0, 5,000 lines x
+// 8,000 dipoles 48.7 and 47.7, 1,000 lines x 8,000 charges 9.95 and 10.0.
+constexpr int kTeamRounds = 20;
 constexpr int kTeamMinSteps = 128;
 static_assert(kTeamLines <= kTeamWarps, "phase B gives each line a warp");
 
