@@ -338,13 +338,15 @@ def main():
                      "sweep_loop_pair_evals_per_s": loop_rate,
                      "frac_of_sweep_loop": (pe_step / avg_kern_s) / loop_rate,
                      "kernel": ("topo_kernel (FP32C, charges resident in shared memory)" if prec == "fp32c"
-                                else "topo_kernel (FP64, charges from L2)"),
+                                else "team_kernel (FP64, charges from L2)"),
                      "work": f"{FLOPS_PER_PAIR} flop per pair evaluation x sum_lines N*(max(s,2)+2)",
                      "peak_source": ("FP32 pipe measured in this run (cpetgb_measure_peak): the higher of "
                                      f"FFMA {ffma_scalar / 1e12:.1f} and packed FFMA2 {ffma2 / 1e12:.1f} TFLOP/s"
                                      if prec == "fp32c" else "DFMA throughput measured in this run")
                                     + "; MEASURED_PEAKS.json holds HBM and bf16 figures only"},
-        "gpu_launches": 4 * args.steps,
+        # per step: pack, the persistent kernel (FP32C), 20 rounds of the team kernel for
+        # the last lines (FP64: all), histogram range and bins
+        "gpu_launches": (24 if prec == "fp32c" else 23) * args.steps,
         "clocks": clocks,
     }
 
