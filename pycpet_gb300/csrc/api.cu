@@ -208,6 +208,16 @@ cudaError_t h2d(T** dst, Scratch& S, const T* src, size_t count) {
   return e;
 }
 
+// Hand-over records, without which a streamline launch runs too (its lines end
+// where they started, in one round): no memory for them is no error.
+cudaError_t left_or_none(cudaError_t e, TopoState** left, int* rounds) {
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  *left = nullptr;
+  *rounds = 1;
+  return cudaSuccess;
+}
+
 // Converts a status word read from the device into a return code (and clears it there).
 int status_code(Ctx* c, int st) {
   if (st != kDevOk) {
@@ -638,7 +648,7 @@ int topo_impl(int prec, int mem, int L, int N, const double* starts, const int32
   unsigned char* packed = nullptr;
   int* queue = nullptr;  // the queue counter and, per round, the count of lines handed over
   TopoState* left = nullptr;
-  const int rounds = topo_team_rounds(c->sms, L, topo_diag_steps(half, step));
+  int rounds = topo_team_rounds(c->sms, L, topo_diag_steps(half, step));
   const bool fresh = topo_fresh(prec, topo_resident_count(prec, source, static_cast<int>(n_pad)) == n_pad, L,
                                 c->sms, true);
   const bool hand = rounds > 1 || L > int64_t(c->sms) * kTeamLinesPerSm;
@@ -646,7 +656,7 @@ int topo_impl(int prec, int mem, int L, int N, const double* starts, const int32
   CK(S.get(&packed, size_t(n_pad) * topo_source_bytes(prec, source)), "alloc packed charges");
   CK(S.get(&queue, size_t(1 + rounds)), "alloc queue");
   CK(cudaMemsetAsync(queue, 0, (1 + rounds) * sizeof(int), s), "zero queue");
-  if (left_cap) CK(S.get(&left, 2 * size_t(left_cap)), "alloc hand-over records");
+  if (left_cap) CK(left_or_none(S.get(&left, 2 * size_t(left_cap)), &left, &rounds), "alloc hand-over records");
   if (reinterpret_cast<uintptr_t>(packed) % 16 != 0)
     return fail(CPETGB_ECUDA, "scratch allocation is not 16-byte aligned");
   if (source == kDipoles)
@@ -807,7 +817,8 @@ int topo_batch_impl(int prec, int mem, int F, const int64_t* desc, const double*
   TopoState* left = nullptr;
   CK(S.get(&queues, size_t(1 + t.rounds) * F), "alloc queues");
   CK(cudaMemsetAsync(queues, 0, sizeof(int) * size_t(1 + t.rounds) * F, s), "zero queues");
-  if (t.left_records) CK(S.get(&left, 2 * size_t(t.left_records)), "alloc hand-over records");
+  if (t.left_records)
+    CK(left_or_none(S.get(&left, 2 * size_t(t.left_records)), &left, &t.rounds), "alloc hand-over records");
   CK(launch_pack_topo_frames(prec, F, d_frames, d_src, dx, dq, packed, max_pairs, s),
      "pack charges");
   TopoParams p{};
@@ -1228,7 +1239,8 @@ int topo_plan_impl(cpetgb_plan** out_plan, int prec, int F, const int64_t* desc,
   if (e == cudaSuccess) e = plan_alloc(pl->bufs, &d_frames, t.frames.size());
   if (e == cudaSuccess) e = plan_alloc(pl->bufs, &d_src, t.src.size());
   if (e == cudaSuccess) e = plan_alloc(pl->bufs, &queues, size_t(1 + t.rounds) * std::max(F, 1));
-  if (e == cudaSuccess && t.left_records) e = plan_alloc(pl->bufs, &left, 2 * size_t(t.left_records));
+  if (e == cudaSuccess && t.left_records)
+    e = left_or_none(plan_alloc(pl->bufs, &left, 2 * size_t(t.left_records)), &left, &t.rounds);
   if (e == cudaSuccess && F > 0)
     e = cudaMemcpy(d_frames, t.frames.data(), t.frames.size() * sizeof(TopoFrame),
                    cudaMemcpyHostToDevice);
