@@ -23,8 +23,8 @@
 // cycles, and a loop of this body on registers alone 16.9 cycles per pair of terms
 // (10.3 without the reciprocals); two terms can't share one, 1 / (s t) rounds
 // differently.  1,024 histograms of 400 bins: pack 3, tiles 59 (51 at 16.9 cycles),
-// merge 9 us; 96 us per call before, with row-major staging, a
-// select around each reciprocal, and the splits summed in double.  3 CTAs per SM: 59.4 us,
+// merge 9 us; 96 us per call before, with row-major staging and the splits summed in
+// double.  3 CTAs per SM: 59.4 us,
 // against 63.5 with the 2 that unlimited registers leave and 60.3 with 4; 2 x 4 and
 // 4 x 2 entries per thread 59.4 to 65.5; 32 x 16 tiles in one pass without splits 65.6.
 #include <algorithm>
@@ -49,10 +49,13 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
   return d;
 }
 
-// MUFU reciprocal, +infinity (of a zero sum) made finite: such a term is
-// 0 * 0 * FLT_MAX = 0, as the definition has it.
-__device__ __forceinline__ float rcp_finite(float x) {
-  return fminf(rcp_mufu(x), FLT_MAX);
+// Reciprocal of a bin's sum a + b by the MUFU; 0 for a sum of zero, whose bin does
+// not contribute whatever a - b is, and for a subnormal one, which the MUFU takes for
+// zero (the values it comes from have a square that vanishes).  The reciprocal cut off
+// at FLT_MAX instead, which is enough where no value is negative, runs 2% faster on
+// large matrices (3,000 x 900 980 us against 998) and alike on 1,024 x 400 (78 us).
+__device__ __forceinline__ float rcp_sum(float s) {
+  return fabsf(s) >= FLT_MIN ? rcp_mufu(s) : 0.f;
 }
 
 __device__ __forceinline__ double pair_value(float s, float c) { return __dsub_rn(widen(s), widen(c)); }
@@ -82,8 +85,7 @@ __global__ void __launch_bounds__(kThreads)
     }
     __syncthreads();  // the previous step's reads
 #pragma unroll
-    for (int u = 0; u < kLoads; ++u)  // + 0: a sum of two zeros is +0 whatever their signs
-      t[tid % kBins][tid / kBins + u * (kThreads / kBins)] = __fadd_rn(narrow(v[u]), 0.f);
+    for (int u = 0; u < kLoads; ++u) t[tid % kBins][tid / kBins + u * (kThreads / kBins)] = narrow(v[u]);
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < kLoads; ++u) {
@@ -161,7 +163,7 @@ __global__ void __launch_bounds__(kThreads, 3)
           const uint64_t d = sub2(aa, b[h]);
           float s0, s1;
           upk2(add2(aa, b[h]), s0, s1);
-          p[r][h] = fma2(mul2(d, d), pk2(rcp_finite(s0), rcp_finite(s1)), p[r][h]);
+          p[r][h] = fma2(mul2(d, d), pk2(rcp_sum(s0), rcp_sum(s1)), p[r][h]);
         }
       }
     }
