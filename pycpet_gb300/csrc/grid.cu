@@ -731,6 +731,11 @@ __device__ __forceinline__ float field_norm2(const double* e) {
   return __fmaf_rn(x, x, __fmaf_rn(y, y, __fmul_rn(z, z)));
 }
 
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
 // One frame of few points, FP32C, in one launch: as grid_few_kernel and the sum
 // over the splits, by one cluster of CTAs that read the caller's arrays.  CTA r
 // takes the splits r, r + kPointCtas, ...; the splits' results go to CTA 0's shared
@@ -750,6 +755,9 @@ __global__ void __cluster_dims__(kPointCtas, 1, 1) __launch_bounds__(kPointThrea
   constexpr int NC = (KIND == kField) ? 3 : 1;
   extern __shared__ __align__(16) unsigned char point_smem[];
   const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  // CTA 0's shared memory may be written once all CTAs of the cluster run: arrived
+  // at here, waited for before the first of those stores, behind the charges' loads
+  cluster_arrive();
   const int rank = static_cast<int>(cluster.block_rank());
   const int tid = threadIdx.x;
   const int P = fr.n_points, ns = fr.n_split, chunk = fr.chunk, n_all = fr.n_charges;
@@ -803,6 +811,7 @@ __global__ void __cluster_dims__(kPointCtas, 1, 1) __launch_bounds__(kPointThrea
     for (int c = 0; c < NC; ++c) sums[c * units + i] = part[c];
   }
   __syncthreads();
+  cluster_wait();
   double* v_0 = cluster.map_shared_rank(v_s, 0);
   for (int i = tid; i < mine * NC * P; i += kPointThreads) {
     const int k = i / (NC * P), cp = i - k * (NC * P), c = cp / P, p = cp - c * P;
