@@ -125,7 +125,10 @@ __device__ __forceinline__ void run_frame(const TopoParams& p, const FrameCtx& f
     const unsigned active = __ballot_sync(0xffffffffu, lane < S && sl.line >= 0);
     const int na = __popc(active);
     if (na == 0) break;
-    if (hand.cap > 0 && *reinterpret_cast<volatile int*>(s_idle) >= kTopoWarps * S - kTeamLinesPerSm &&
+    // (other warps count s_idle up meanwhile: a vote, so that the warp's lanes, whatever
+    // each of them read, take the same branch to the shuffles of hand_over)
+    if (hand.cap > 0 &&
+        __any_sync(0xffffffffu, *reinterpret_cast<volatile int*>(s_idle) >= kTopoWarps * S - kTeamLinesPerSm) &&
         hand_over(hand, sl, *my_rec, active, lane))
       break;
     // owner lane of each active slot, in order; this lane's rank among them

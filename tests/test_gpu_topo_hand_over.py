@@ -1,0 +1,37 @@
+"""Launches whose CTAs run out of lines and hand their last ones over while other
+warps of the CTA are between two steps: the same bits as the launch that hands
+nothing over (the allocation-free entry point), many times over.  Line counts
+around what a CTA holds (64 slots; 16 lines are handed over), step caps that make
+slots run empty one by one, in groups and all at once."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("caps_of", ["spread", "groups", "equal"])
+def test_handed_over_lines_keep_their_bits(gpu_lib, caps_of):
+    import torch
+    from pycpet_gb300 import _lib, topo_lines
+
+    sms = gpu_lib.cpetgb_device_sms()
+    rng = np.random.default_rng(8)
+    x = rng.uniform(-30.0, 30.0, (900, 3))
+    x = torch.from_numpy(x[np.linalg.norm(x, axis=1) > 3.0][:300].copy()).cuda()
+    q = torch.from_numpy(rng.normal(0.0, 0.4, 300)).cuda()
+    half = np.array([1.5, 1.5, 1.2])
+    for per_sm in (21, 40, 64, 65, 90):
+        L = sms * per_sm + 3
+        starts = torch.from_numpy(rng.uniform(-1.2, 1.2, (L, 3))).cuda()
+        caps = {"spread": rng.integers(0, 300, L), "groups": 40 * rng.integers(1, 5, L), "equal": np.full(L, 60)}[caps_of]
+        caps = torch.from_numpy(caps.astype(np.int32)).cuda()
+        res = torch.empty((L, 2), dtype=torch.float64, device="cuda")
+        steps = torch.empty(L, dtype=torch.int32, device="cuda")
+        stream = torch.cuda.current_stream().cuda_stream
+        rc = gpu_lib.cpetgb_topo_lines_noalloc(_lib.FP32C, L, 300, starts.data_ptr(), caps.data_ptr(), 0.01,
+                                               half.ctypes.data, x.data_ptr(), q.data_ptr(), res.data_ptr(), None,
+                                               steps.data_ptr(), stream)
+        assert rc == 0, _lib.last_error()
+        for _ in range(10):
+            r, s = topo_lines(starts, caps, x, q, 0.01, half, precision="fp32c", return_steps=True)
+            assert torch.equal(r, res) and torch.equal(s, steps)
