@@ -1432,9 +1432,12 @@ cudaError_t launch_grid_point(const GridLaunch& g, cudaStream_t s) {
   const PointSizes n(g);
   const size_t smem = size_t(n.charges) * sizeof(float4) + size_t(n.results) * sizeof(double) +
                       size_t(n.units) * (g.kind == kField ? 3 : 1) * sizeof(float);
+  // the limit belongs to the kernel, not to the calling thread: always the largest size,
+  // so that a thread cannot lower it between another's setting and its launch
+  constexpr int kMost = kPointCharges * sizeof(float4) + kPointResults * sizeof(double) +
+                        kPointUnits * 3 * sizeof(float);
   auto run = [&](auto kernel) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
     if (e != cudaSuccess) return e;
     kernel<<<kPointCtas, kPointThreads, smem, s>>>(g.one, g.points, g.x, g.q, g.out);
     return cudaGetLastError();

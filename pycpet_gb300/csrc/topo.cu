@@ -661,8 +661,11 @@ template <int PREC, int S, bool DIP, int SRC>
 cudaError_t launch_topo_t(const TopoParams& p, const TopoFrame& f0, int total_lines, int num_sms,
                           cudaStream_t s) {
   const size_t smem = topo_smem_bytes(S, PREC == kFP32C ? p.max_resident_pad : 0, DIP);
+  // the limit belongs to the kernel, not to the calling thread: always the largest size,
+  // so that a thread cannot lower it between another's setting and its launch
+  const size_t most = topo_smem_bytes(S, static_cast<int>(topo_resident_limit(PREC, DIP ? kDipoles : kCharges)), DIP);
   const cudaError_t err = cudaFuncSetAttribute(
-      topo_kernel<PREC, S, DIP, SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+      topo_kernel<PREC, S, DIP, SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most));
   if (err != cudaSuccess) return err;
   // one CTA per SM: its 512 threads take more than half of an SM's registers
   const int grid = std::max(1, std::min(num_sms, total_lines));

@@ -525,13 +525,26 @@ __global__ void __launch_bounds__(kTeams* kTeamThreads, 1)
   }
 }
 
+// Sources a CTA can hold in shared memory beside the exchanged sums (0: FP64).
+int team_resident_limit(int prec, int source) {
+  if (prec != kFP32C) return 0;
+  int dev = 0, optin = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  const int64_t room = int64_t(optin) - static_cast<int64_t>(team_fixed_bytes<kFP32C>()) - 256;
+  if (room <= 0) return 0;
+  return static_cast<int>(room / (source == kDipoles ? 24 : 16)) / kChargePad32 * kChargePad32;
+}
+
 template <int PREC, bool DIP>
 cudaError_t launch_team_t(const TopoParams& p, const TopoFrame& f0, int fresh, int num_sms,
                           cudaStream_t s) {
-  const size_t smem = team_fixed_bytes<PREC>() +
-                      (PREC == kFP32C ? static_cast<size_t>(p.max_team_resident) * (DIP ? 24 : 16) : 0);
+  const auto bytes = [](int resident) { return team_fixed_bytes<PREC>() + static_cast<size_t>(resident) * (DIP ? 24 : 16); };
+  const size_t smem = bytes(PREC == kFP32C ? p.max_team_resident : 0);
+  // (always the largest size: see launch_topo_t)
   const cudaError_t err = cudaFuncSetAttribute(
-      team_kernel<PREC, DIP>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+      team_kernel<PREC, DIP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      static_cast<int>(bytes(team_resident_limit(PREC, DIP ? kDipoles : kCharges))));
   if (err != cudaSuccess) return err;
   const int64_t lines = p.frames ? p.sum_lines : p.n_lines;
   const int grid = fresh ? static_cast<int>(std::min<int64_t>(num_sms, lines)) : num_sms;
@@ -547,13 +560,8 @@ cudaError_t launch_team_t(const TopoParams& p, const TopoFrame& f0, int fresh, i
 
 // As topo_resident_count, less the space of the exchanged sums.
 int topo_team_resident(int prec, int source, int n_pad) {
-  if (prec != kFP32C) return 0;
-  int dev = 0, optin = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  const int64_t room = int64_t(optin) - static_cast<int64_t>(team_fixed_bytes<kFP32C>()) - 256;
-  if (room <= 0) return 0;
-  const int limit = static_cast<int>(room / (source == kDipoles ? 24 : 16)) / kChargePad32 * kChargePad32;
+  const int limit = team_resident_limit(prec, source);
+  if (limit <= 0) return 0;
   if (n_pad <= limit) return n_pad;
   constexpr int kRun = 2 * 32 * kLanePairs;
   return limit / kRun * kRun;
