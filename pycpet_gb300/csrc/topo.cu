@@ -878,7 +878,8 @@ int topo_left_capacity(int num_sms, int64_t n_lines, bool fresh) {
 }
 
 cudaError_t launch_topo_frames(int prec, const TopoParams& p, int num_sms, cudaStream_t s) {
-  if (p.n_frames <= 0 || p.n_lines <= 0) return cudaSuccess;
+  // (line offsets alone can make n_lines positive)
+  if (p.n_frames <= 0 || p.n_lines <= 0 || p.sum_lines <= 0) return cudaSuccess;
   TopoFrame dummy{};
   if (topo_fresh(prec, p.all_resident != 0, p.sum_lines, num_sms, p.left != nullptr))
     return launch_topo_team(prec, p, dummy, 1, num_sms, s);
