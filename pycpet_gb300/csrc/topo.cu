@@ -57,27 +57,27 @@ constexpr int kTopoWarps = kTopoThreads / 32;
 // Hand-over of a frame's last lines.  Once the queue is empty and a CTA holds at
 // most kTeamLinesPerSm lines, most of its warps have nothing to do and the rest
 // sweep a line alone; its warps then write their lines' states to the frame's
-// records and leave, and the team kernel finishes them, spread over all SMs.
+// records and leave, and the team kernel finishes them, spread over all SMs.  A CTA
+// hands over at most kTeamLinesPerSm lines of a frame (it has that many left when its
+// first warp does, and gets no more), so a frame with records for that many from
+// every CTA, or for all of its lines, never runs out of them; one with fewer has none.
 struct HandOver {
-  TopoState* rec;  // the frame's records
+  TopoState* rec;  // the frame's records; null: no hand-over
   int* count;      // records written
-  int cap;         // 0: no hand-over
 };
 
-__device__ __forceinline__ bool hand_over(const HandOver& h, const Slot& sl, const SlotRec& rec,
-                                       unsigned active, int lane) {
+__device__ __forceinline__ HandOver hand_over_of(const TopoParams& p, const TopoFrame& fr, int f) {
+  const bool room = fr.left_cap > 0 && fr.left_cap >= min(fr.n_lines, static_cast<int>(gridDim.x) * kTeamLinesPerSm);
+  return HandOver{p.left && room ? p.left + fr.left_off : nullptr, p.left_count + f};
+}
+
+__device__ __forceinline__ void hand_over(const HandOver& h, const Slot& sl, const SlotRec& rec,
+                                          unsigned active, int lane) {
   const int na = __popc(active);
   const int leader = __ffs(active) - 1;
   int base = 0;
-  if (lane == leader) {
-    base = atomicAdd(h.count, na);
-    if (base + na > h.cap) {  // no room: taken back, the warp keeps its lines
-      atomicSub(h.count, na);
-      base = -1;
-    }
-  }
+  if (lane == leader) base = atomicAdd(h.count, na);
   base = __shfl_sync(0xffffffffu, base, leader);
-  if (base < 0) return false;
   if ((active >> lane) & 1u) {
     TopoState* t = h.rec + base + __popc(active & ((1u << lane) - 1u));
     for (int k = 0; k < 3; ++k) {
@@ -93,7 +93,6 @@ __device__ __forceinline__ bool hand_over(const HandOver& h, const Slot& sl, con
     t->steps = sl.steps;
     t->cap = sl.cap;
   }
-  return true;
 }
 
 // One line slot set per warp; processes the lines of frame `fc` (g: its sources
@@ -127,10 +126,11 @@ __device__ __forceinline__ void run_frame(const TopoParams& p, const FrameCtx& f
     if (na == 0) break;
     // (other warps count s_idle up meanwhile: a vote, so that the warp's lanes, whatever
     // each of them read, take the same branch to the shuffles of hand_over)
-    if (hand.cap > 0 &&
-        __any_sync(0xffffffffu, *reinterpret_cast<volatile int*>(s_idle) >= kTopoWarps * S - kTeamLinesPerSm) &&
-        hand_over(hand, sl, *my_rec, active, lane))
+    if (hand.rec &&
+        __any_sync(0xffffffffu, *reinterpret_cast<volatile int*>(s_idle) >= kTopoWarps * S - kTeamLinesPerSm)) {
+      hand_over(hand, sl, *my_rec, active, lane);
       break;
+    }
     // owner lane of each active slot, in order; this lane's rank among them
     int src_of[S];
     int my_rank = -1;
@@ -300,10 +300,7 @@ __global__ void __launch_bounds__(kTopoThreads, 1) topo_kernel(TopoParams p, Top
       fc.half[k] = fr.half[k];
       fc.hf[k] = static_cast<float>(fr.half[k]);
     }
-    HandOver hand;
-    hand.rec = p.left + fr.left_off;
-    hand.count = p.left_count + f;
-    hand.cap = p.left ? fr.left_cap : 0;
+    const HandOver hand = hand_over_of(p, fr, f);
     run_frame<PREC, S, DIP, SRC>(p, fc, queue, reinterpret_cast<const ulonglong2*>(src), sm_off, fr.resident / 2,
                             fr.n_pad, my_rec, lane, hand, &s_idle);
   }

@@ -35,3 +35,28 @@ def test_handed_over_lines_keep_their_bits(gpu_lib, caps_of):
         for _ in range(10):
             r, s = topo_lines(starts, caps, x, q, 0.01, half, precision="fp32c", return_steps=True)
             assert torch.equal(r, res) and torch.equal(s, steps)
+
+
+def test_frames_beyond_the_records(gpu_lib):
+    """A table of so many lines that its last frames have no hand-over records: their
+    lines end where they started, with the bits of a launch of their own."""
+    from pycpet_gb300 import TopoBatch, topo_lines
+
+    per_frame = 16 * gpu_lib.cpetgb_device_sms() + 70
+    n_frames = (1 << 18) // (16 * gpu_lib.cpetgb_device_sms()) + 4
+    rng = np.random.default_rng(9)
+    x = rng.uniform(-30.0, 30.0, (400, 3))
+    x = x[np.linalg.norm(x, axis=1) > 3.0]
+    frames = []
+    for f in range(n_frames):
+        n = 40 + f % 3
+        frames.append({"x": x[:n], "q": rng.normal(0.0, 0.4, n), "starts": rng.uniform(-1.2, 1.2, (per_frame, 3)),
+                       "n_iter": rng.integers(0, 30, per_frame).astype(np.int32), "step": 0.02,
+                       "half_dims": [1.5, 1.5, 1.2]})
+    res, steps = TopoBatch(frames, precision="fp32c").run(return_steps=True)
+    for f in (0, 1, n_frames // 2, n_frames - 5, n_frames - 3, n_frames - 1):
+        fr = frames[f]
+        r, s = topo_lines(fr["starts"], fr["n_iter"], fr["x"], fr["q"], 0.02, [1.5, 1.5, 1.2], return_steps=True)
+        at = slice(f * per_frame, (f + 1) * per_frame)
+        np.testing.assert_array_equal(res[at], r)
+        np.testing.assert_array_equal(steps[at], s)
