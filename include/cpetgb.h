@@ -91,6 +91,12 @@ double cpetgb_field_refinement(void);
  * wait works (the device stays usable).  No counterpart in the reference,
  * whose CPU code has no device waits. */
 int cpetgb_check_wait_limit(double seconds);
+
+/* Whether the calling thread's streamline calls, and the plans that it makes, ask for
+ * memory for hand-over records (up to 84 MB; default 1).  0: they run as they do when
+ * there is no memory for them: the same results, lines not dealt out again over the
+ * SMs while they run.  For callers with a tight budget, and to check that path. */
+int cpetgb_set_hand_over_records(int on);
 /* Pipe throughput microbenchmark on the current device (roofline denominators):
  * kind 0 FP32 FFMA flop/s, 1 FP64 DFMA flop/s, 2 MUFU rsqrt op/s, 3 FP32x2 FFMA2 flop/s,
  * 4 pair evaluations/s of the FP32C streamline sweep's inner loop alone. */

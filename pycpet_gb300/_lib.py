@@ -54,6 +54,7 @@ SIGNATURES = {
     "cpetgb_compute_esp_grid_p": [_i, _i, _i, _vp, _vp, _vp, _vp],
     "cpetgb_set_field_refinement": [_d],
     "cpetgb_check_wait_limit": [_d],
+    "cpetgb_set_hand_over_records": [_i],
     "cpetgb_field_grid": [_i, _i, _i, _i, _vp, _vp, _vp, _i, _vp, _vp],
     "cpetgb_esp_grid": [_i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp],
     "cpetgb_grid_batch": [_i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp],

@@ -208,9 +208,14 @@ cudaError_t h2d(T** dst, Scratch& S, const T* src, size_t count) {
   return e;
 }
 
-// Hand-over records, without which a streamline launch runs too (its lines end
-// where they started, in one round): no memory for them is no error.
-cudaError_t left_or_none(cudaError_t e, TopoState** left, int* rounds) {
+// Hand-over records (cpetgb_set_hand_over_records).
+thread_local bool g_hand_over = true;
+
+// Allocates hand-over records by alloc(), without which a streamline launch runs too
+// (its lines end where they started, in one round): no memory for them is no error.
+template <typename Alloc>
+cudaError_t left_or_none(Alloc alloc, TopoState** left, int* rounds) {
+  const cudaError_t e = g_hand_over ? alloc() : cudaErrorMemoryAllocation;
   if (e != cudaErrorMemoryAllocation) return e;
   cudaGetLastError();
   *left = nullptr;
@@ -651,12 +656,12 @@ int topo_impl(int prec, int mem, int L, int N, const double* starts, const int32
   int rounds = topo_team_rounds(c->sms, L, topo_diag_steps(half, step));
   const bool fresh = topo_fresh(prec, topo_resident_count(prec, source, static_cast<int>(n_pad)) == n_pad, L,
                                 c->sms, true);
-  const bool hand = rounds > 1 || L > int64_t(c->sms) * kTeamLinesPerSm;
-  const int left_cap = hand ? topo_left_capacity(c->sms, L, fresh) : 0;
+  const int left_cap = fresh && rounds == 1 ? 0 : topo_left_capacity(c->sms, L, fresh);
   CK(S.get(&packed, size_t(n_pad) * topo_source_bytes(prec, source)), "alloc packed charges");
   CK(S.get(&queue, size_t(1 + rounds)), "alloc queue");
   CK(cudaMemsetAsync(queue, 0, (1 + rounds) * sizeof(int), s), "zero queue");
-  if (left_cap) CK(left_or_none(S.get(&left, 2 * size_t(left_cap)), &left, &rounds), "alloc hand-over records");
+  if (left_cap)
+    CK(left_or_none([&] { return S.get(&left, 2 * size_t(left_cap)); }, &left, &rounds), "alloc hand-over records");
   if (reinterpret_cast<uintptr_t>(packed) % 16 != 0)
     return fail(CPETGB_ECUDA, "scratch allocation is not 16-byte aligned");
   if (source == kDipoles)
@@ -680,6 +685,7 @@ int topo_impl(int prec, int mem, int L, int N, const double* starts, const int32
   p.left_records = left_cap;
   p.left_count = queue + 1;
   p.rounds = rounds;
+  p.fresh = fresh;
   p.status = c->status;
   CK(launch_topo(prec, p, c->sms, s), "topo kernel launch");
   if (mem == CPETGB_HOST) {
@@ -703,6 +709,7 @@ struct TopoTables {
   int64_t sum_lines = 0;      // lines of all frames (frames may share ranges)
   int64_t left_records = 0;   // hand-over records of all frames
   int rounds = 1;             // team kernel launches
+  bool fresh = false;         // every line in them from its start point
   double diag_steps = 0.0;    // the frames' largest box diagonal in steps
   int max_res = 0, max_team_res = 0, max_pairs = 0;
   bool all_resident = true;  // every frame entirely in shared memory (tuner class 1)
@@ -756,10 +763,9 @@ int build_topo_tables(int prec, int F, const int64_t* desc, const double* params
 
 void plan_hand_over(int prec, int sms, TopoTables& t) {
   t.rounds = topo_team_rounds(sms, t.sum_lines, t.diag_steps);
-  const bool fresh = topo_fresh(prec, t.all_resident, t.sum_lines, sms, true);
-  const bool hand = t.rounds > 1 || t.sum_lines > int64_t(sms) * kTeamLinesPerSm;
+  t.fresh = topo_fresh(prec, t.all_resident, t.sum_lines, sms, true);
   for (TopoFrame& fr : t.frames) {
-    const int64_t cap = hand ? topo_left_capacity(sms, fr.n_lines, fresh) : 0;
+    const int64_t cap = t.fresh && t.rounds == 1 ? 0 : topo_left_capacity(sms, fr.n_lines, t.fresh);
     fr.left_off = static_cast<int32_t>(t.left_records);
     fr.left_cap = t.left_records + cap <= kMaxLeft ? static_cast<int32_t>(cap) : 0;
     t.left_records += fr.left_cap;
@@ -818,7 +824,8 @@ int topo_batch_impl(int prec, int mem, int F, const int64_t* desc, const double*
   CK(S.get(&queues, size_t(1 + t.rounds) * F), "alloc queues");
   CK(cudaMemsetAsync(queues, 0, sizeof(int) * size_t(1 + t.rounds) * F, s), "zero queues");
   if (t.left_records)
-    CK(left_or_none(S.get(&left, 2 * size_t(t.left_records)), &left, &t.rounds), "alloc hand-over records");
+    CK(left_or_none([&] { return S.get(&left, 2 * size_t(t.left_records)); }, &left, &t.rounds),
+       "alloc hand-over records");
   CK(launch_pack_topo_frames(prec, F, d_frames, d_src, dx, dq, packed, max_pairs, s),
      "pack charges");
   TopoParams p{};
@@ -834,6 +841,7 @@ int topo_batch_impl(int prec, int mem, int F, const int64_t* desc, const double*
   p.left_records = t.left_records;
   p.left_count = queues + F;
   p.rounds = t.rounds;
+  p.fresh = t.fresh;
   p.status = c->status;
   p.frames = d_frames;
   p.n_frames = F;
@@ -1240,7 +1248,7 @@ int topo_plan_impl(cpetgb_plan** out_plan, int prec, int F, const int64_t* desc,
   if (e == cudaSuccess) e = plan_alloc(pl->bufs, &d_src, t.src.size());
   if (e == cudaSuccess) e = plan_alloc(pl->bufs, &queues, size_t(1 + t.rounds) * std::max(F, 1));
   if (e == cudaSuccess && t.left_records)
-    e = left_or_none(plan_alloc(pl->bufs, &left, 2 * size_t(t.left_records)), &left, &t.rounds);
+    e = left_or_none([&] { return plan_alloc(pl->bufs, &left, 2 * size_t(t.left_records)); }, &left, &t.rounds);
   if (e == cudaSuccess && F > 0)
     e = cudaMemcpy(d_frames, t.frames.data(), t.frames.size() * sizeof(TopoFrame),
                    cudaMemcpyHostToDevice);
@@ -1267,6 +1275,7 @@ int topo_plan_impl(cpetgb_plan** out_plan, int prec, int F, const int64_t* desc,
   p.left_records = t.left_records;
   p.left_count = queues + F;
   p.rounds = t.rounds;
+  p.fresh = t.fresh;
   p.status = c->status;
   p.frames = d_frames;
   p.n_frames = F;
@@ -1350,6 +1359,11 @@ int cpetgb_check_wait_limit(double seconds) {
   const unsigned long long ns = static_cast<unsigned long long>(seconds * 1e9);
   CK(launch_wait_limit_check(c->status, ns, c->stream), "wait check launch");
   return finish(c, c->stream);
+}
+
+int cpetgb_set_hand_over_records(int on) {
+  g_hand_over = on != 0;
+  return CPETGB_OK;
 }
 
 int cpetgb_set_field_refinement(double tau) {

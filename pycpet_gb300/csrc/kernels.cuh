@@ -151,7 +151,8 @@ struct TopoParams {
   TopoState* left = nullptr;   // two lists of left_records hand-over records, or null: no hand-over
   int64_t left_records = 0;
   int* left_count = nullptr;   // records written: [rounds][n_frames] counters (zeroed by the caller)
-  int rounds = 1;              // team kernel launches (topo_team_rounds)
+  int rounds = 1;              // team kernel launches (topo_team_rounds); 1 without lists
+  bool fresh = false;          // all lines go to the team kernel from their start points (topo_fresh)
   int* status;
   const TopoFrame* frames;   // device frame table (multi-frame launches) or null
   int n_frames;              // frames in the table
@@ -188,8 +189,9 @@ double topo_diag_steps(const double* half, double step);
 constexpr int kTeamLinesPerSm = 16;
 constexpr int64_t kMaxLeft = int64_t(1) << 18;  // hand-over records of a launch: two lists of 42 MB
 // Whether a launch's lines go to the team kernel from their start points
-// (resident: every frame's sources fit shared memory; lists: hand-over records
-// can be had).
+// (resident: every frame's sources fit shared memory; lists: hand-over records may
+// be asked for).  Decided once, by who plans the launch; that there is no memory for
+// the records in the end does not change it.
 bool topo_fresh(int prec, bool resident, int64_t sum_lines, int num_sms, bool lists);
 
 // max sources (charges or dipoles) held resident in shared memory

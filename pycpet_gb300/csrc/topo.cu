@@ -841,9 +841,8 @@ cudaError_t launch_topo(int prec, const TopoParams& p_in, int num_sms, cudaStrea
   p.max_resident_pad = f0.resident;
   p.max_team_resident = f0.team_resident;
   const bool whole = f0.resident == f0.n_pad;
-  const bool fresh = topo_fresh(prec, whole, p.n_lines, num_sms, p.left != nullptr);
-  f0.left_cap = p.left ? topo_left_capacity(num_sms, p.n_lines, fresh) : 0;
-  if (fresh) return launch_topo_team(prec, p, f0, 1, num_sms, s);
+  f0.left_cap = p.left ? topo_left_capacity(num_sms, p.n_lines, p.fresh) : 0;
+  if (p.fresh) return launch_topo_team(prec, p, f0, 1, num_sms, s);
   const int slots = tuned_topo_slots(prec, whole, p.n_lines);
   const cudaError_t e = p.source == kDipoles
                             ? launch_topo_prec<true>(prec, whole, p, f0, num_sms, s, slots)
@@ -878,8 +877,7 @@ cudaError_t launch_topo_frames(int prec, const TopoParams& p, int num_sms, cudaS
   // (line offsets alone can make n_lines positive)
   if (p.n_frames <= 0 || p.n_lines <= 0 || p.sum_lines <= 0) return cudaSuccess;
   TopoFrame dummy{};
-  if (topo_fresh(prec, p.all_resident != 0, p.sum_lines, num_sms, p.left != nullptr))
-    return launch_topo_team(prec, p, dummy, 1, num_sms, s);
+  if (p.fresh) return launch_topo_team(prec, p, dummy, 1, num_sms, s);
   const int slots = tuned_topo_slots(prec, p.all_resident != 0, p.n_lines);
   const cudaError_t e = launch_topo_prec<false>(prec, p.all_resident != 0, p, dummy, num_sms, s, slots);
   if (e != cudaSuccess || !p.left) return e;
