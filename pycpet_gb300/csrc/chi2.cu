@@ -12,12 +12,13 @@
 //            packed f32x2 instruction, one MUFU reciprocal per term.  Each chunk
 //            is summed plainly and Kahan-added (Kahan 1965) into a running
 //            (sum, compensation) pair per entry;
-//   merge    the splits' pairs added in split order (TwoSum, the rounding errors
-//            beside the compensations: 48 bits), halved, and written to the entry
+//   merge    the splits' pairs added in split order (TwoSum, the rounding errors and
+//            the compensations beside the sum, their own rounding errors as a third
+//            float: more bits than a double holds), halved, and written to the entry
 //            and its mirror image through shared memory.
 //            With one split the tile kernel writes the matrix itself.
-// Sums stay in FP32 pairs until the single double subtraction at the end: an FP64
-// warp instruction holds a scheduler's FP64 pipe for 64 cycles, and 48 of them per
+// Sums stay in floats until the double additions at the end: an FP64 warp
+// instruction holds a scheduler's FP64 pipe for 64 cycles, and 48 of them per
 // thread (conversions included) were a quarter of the time.
 // Bound: the MUFU reciprocals, one per term: a warp's takes a scheduler's unit 8
 // cycles, and a loop of this body on registers alone 16.9 cycles per pair of terms
@@ -208,18 +209,22 @@ __global__ void __launch_bounds__(kThreads)
   int ib, jb;
   tile_of(blockIdx.x, ib, jb);
   const float2* src = part + int64_t(blockIdx.x) * splits * kEntries + 4 * r * kThreads + 64 * g + owner;
-  float s[4] = {}, c[4] = {};
+  float s[4] = {}, c[4] = {}, d[4] = {};
 #pragma unroll 4
   for (int z = 0; z < splits; ++z)
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const float2 v = src[int64_t(z) * kEntries + k * kThreads];
-      float e;
+      float e, w, ew, ec;
       two_sum(s[k], v.x, s[k], e);
-      c[k] = __fadd_rn(c[k], __fsub_rn(v.y, e));
+      two_sum(e, -v.y, w, ew);
+      two_sum(c[k], w, c[k], ec);
+      d[k] = __fadd_rn(d[k], __fadd_rn(ew, ec));
     }
 #pragma unroll
-  for (int k = 0; k < 4; ++k) t[4 * (owner >> 4) + r][4 * (owner & 15) + k] = 0.5 * pair_value(s[k], c[k]);
+  for (int k = 0; k < 4; ++k)
+    t[4 * (owner >> 4) + r][4 * (owner & 15) + k] =
+        0.5 * __dadd_rn(widen(s[k]), __dadd_rn(widen(c[k]), widen(d[k])));
   __syncthreads();
   const int64_t i0 = int64_t(ib) * kTile + kRows * g, j0 = int64_t(jb) * kTile;
   for (int e = tid; e < kRows * kTile; e += kThreads) {
