@@ -56,6 +56,7 @@
 
 #include "common.cuh"
 #include "kernels.cuh"
+#include "point_map.cuh"
 
 namespace cpetgb {
 namespace {
@@ -269,40 +270,6 @@ __device__ __forceinline__ GridFrame load_frame(const GridFrame* frames, int n_f
   *f = find_frame<OFF>(frames, n_frames, i);
   return frames[*f];
 }
-
-// Which points a frame's threads take (u: thread of the frame, k: its k-th
-// point): -1 for none.  stride: the lattice stride S, or 0.
-struct PointMap {
-  int stride, lat_threads, lat_end, rest;  // columns x groups; rounded up to a warp; first other point
-  int n_points;
-
-  template <int PPT>
-  __device__ __forceinline__ void set(int s, int P) {
-    n_points = P;
-    stride = s;
-    const int groups = s > 0 ? P / s / PPT : 0;
-    lat_threads = s * groups;
-    lat_end = (lat_threads + 31) & ~31;
-    rest = lat_threads * PPT;
-  }
-  // Threads of the frame that have points, rounded up to a warp.
-  template <int PPT>
-  __device__ __forceinline__ int threads() const {
-    return lat_end + (n_points - rest + 32 * PPT - 1) / (32 * PPT) * 32;
-  }
-  __device__ __forceinline__ bool column(int u) const { return u < lat_end; }  // uniform across a warp
-  template <int PPT>
-  __device__ __forceinline__ int point(int u, int k) const {
-    if (u < lat_end) {
-      if (u >= lat_threads) return -1;
-      const int g = u / stride;
-      return (g * PPT + k) * stride + (u - g * stride);
-    }
-    const int v = u - lat_end;
-    const int p = rest + (v >> 5) * (32 * PPT) + 32 * k + (v & 31);
-    return p < n_points ? p : -1;
-  }
-};
 
 // FP32C with 4 points per thread: four CTAs (16 warps) per SM for the field,
 // whose column loop needs more than 80 registers to keep the FP32 pipe fed (24
