@@ -369,7 +369,7 @@ int plan_grid(int prec, int n_frames, const int64_t* desc, int sms, int ppt, int
     if (fr.n_split > 1) t.n_slots += items;
     if (fr.few) {
       t.few_items += items;
-    } else if (mesh) {
+    } else if (mesh && fr.n_charges >= (prec == CPETGB_FP64 ? kGridMeshChargesFp64 : kGridMeshChargesFp32)) {
       t.n_prep += (int64_t(fr.n_points) + kGridPrepPoints - 1) / kGridPrepPoints;
     }
     if (t.n_items > INT_MAX || t.n_tiles * ppt > INT_MAX)

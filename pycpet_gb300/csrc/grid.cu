@@ -13,7 +13,7 @@
 // PPT points.
 //
 // Lattices: the points of a volume are a mesh, x slowest.  The preparation
-// kernel looks for the stride S after which (y, z) repeat, and for meshes a
+// kernel looks for the stride S at which x changes and (y, z) repeat, and for meshes a
 // thread takes PPT points of one (y, z) column: dy, dz and dy^2 + dz^2 are formed
 // once per charge instead of once per point and charge, in the same order of
 // operations, so the sums are the same bits.  That is 9 instead of 12 FP32-pipe
@@ -48,7 +48,6 @@
 // floats, about 48 significant bits, on the FP32 pipe: GB300's FP64 pipe is
 // 1/64 of its FP32 pipe).
 #include <algorithm>
-#include <climits>
 #include <cstddef>
 #include <type_traits>
 
@@ -1168,7 +1167,6 @@ __global__ void __launch_bounds__(kRefineThreads, 2)
 
 constexpr int kPrepThreads = 256;
 constexpr int kPrepCharges = 1024;   // charges per preparation block
-constexpr int kMaxStride = 16384;    // longest lattice stride looked for
 
 __device__ __forceinline__ bool same_yz(const double* a, const double* b, bool f32) {
   if (f32)  // the FP32C kernels see the FP32 images
@@ -1178,12 +1176,16 @@ __device__ __forceinline__ bool same_yz(const double* a, const double* b, bool f
          __double_as_longlong(a[2]) == __double_as_longlong(b[2]);
 }
 
+__device__ __forceinline__ bool same_x(const double* a, const double* b, bool f32) {
+  return f32 ? __float_as_uint(narrow(a[0])) == __float_as_uint(narrow(b[0]))
+             : __double_as_longlong(a[0]) == __double_as_longlong(b[0]);
+}
+
 // Preparation, one launch: blocks [0, n_charge_blocks) pack the charges (FP32C:
 // every component duplicated; FP64: Charge64) and, for the refinement, their
 // double-float records {xh, yh, zh, qh} {xl, yl, zl, ql}; the others look for the
-// frames' lattice strides, kGridPrepPoints points each.  A frame's stride is the
-// first index whose (y, z) equal those of point 0; it holds if every point's
-// (y, z) equal those one stride earlier.  stride[f] is written by the frame's
+// frames' lattice strides, kGridPrepPoints points each.  A frame's stride is where x
+// first changes; it holds if every point's (y, z) equal those one stride earlier.  stride[f] is written by the frame's
 // first block, broken[f] (zeroed by the caller) by any block that finds a
 // difference.
 template <int PREC, bool DF>
@@ -1221,23 +1223,30 @@ __global__ void __launch_bounds__(kPrepThreads)
   const int P = fr.n_points;
   const double* pts = points + 3 * fr.point_off;
   constexpr bool kF32 = PREC == kFP32C;
-  __shared__ int s_stride;
-  if (threadIdx.x == 0) s_stride = INT_MAX;
-  __syncthreads();
-  const int limit = min(P / min_rows, kMaxStride);  // at least min_rows rows
-  constexpr int kLook = kPrepThreads * 4;
-  for (int i0 = 1; i0 <= limit; i0 += kLook) {
-    int hit = INT_MAX;
+  __shared__ int s_first[kPrepThreads / 32];
+  // x is constant over a mesh's first S points and another after them: S by search over
+  // the block's threads, 257 intervals at a time (two looks for up to 66,000 points).
+  // Points that are no mesh may give any S; the comparison below decides.
+  const int limit = P / min_rows;  // at least min_rows rows
+  int lo = 0, span = limit + 1;    // x[lo] is point 0's, x[lo + span] another's, or lies past the limit
+  while (span > 1) {
+    const int part = (span + kPrepThreads) / (kPrepThreads + 1);
+    const int i = lo + (static_cast<int>(threadIdx.x) + 1) * part;
+    const bool other = i >= lo + span || !same_x(pts, pts + 3 * static_cast<int64_t>(i), kF32);
+    // the first thread that sees another x, from each warp's first
+    const unsigned seen = __ballot_sync(0xffffffffu, other);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0)
+      s_first[threadIdx.x >> 5] = seen ? static_cast<int>(threadIdx.x) + __ffs(seen) - 1 : kPrepThreads;
+    __syncthreads();
+    int first = kPrepThreads;
 #pragma unroll
-    for (int k = 3; k >= 0; --k) {
-      const int i = i0 + k * kPrepThreads + static_cast<int>(threadIdx.x);
-      if (i <= limit && i < P && same_yz(pts, pts + 3 * static_cast<int64_t>(i), kF32)) hit = i;
-    }
-    if (hit != INT_MAX) atomicMin(&s_stride, hit);
-    if (__syncthreads_or(hit != INT_MAX)) break;
+    for (int w = 0; w < kPrepThreads / 32; ++w) first = min(first, s_first[w]);
+    lo += first * part;
+    span = min(part, span - first * part);
   }
-  const int S = s_stride;
-  const bool mesh = S != INT_MAX && P % S == 0;
+  const int S = lo + 1;
+  const bool mesh = S <= limit && P % S == 0 && same_yz(pts, pts + 3 * static_cast<int64_t>(S), kF32);
   if (part == 0 && threadIdx.x == 0) stride[f] = mesh ? S : 0;
   if (!mesh) return;
   const int64_t j0 = max(static_cast<int64_t>(part) * kGridPrepPoints, static_cast<int64_t>(S));

@@ -43,6 +43,12 @@ constexpr int kGridFewPointsFp32 = 32;
 // Launches with fewer pairs than this don't look for meshes: the look costs about
 // 5 us, a quarter of so small a launch's kernel less.
 constexpr double kGridMeshPairsFp32 = 2.0e7, kGridMeshPairsFp64 = 1.0e6;
+// Nor is a frame of fewer charges than this looked at: the look reads every point
+// twice, and a column saves little per charge.  Potential of 159^3 points x 256 charges:
+// 269 us without a look, 282 with it as columns; x 500 charges 487 as columns, 511 as
+// points in no order (look included).  In FP64 20 charges already repay it (1,418 us
+// against 1,818).
+constexpr int kGridMeshChargesFp32 = 512, kGridMeshChargesFp64 = 16;
 
 // One frame of a grid launch (device table, sorted by charge chunk, longest
 // first).  Its points are cut into tiles of kGridThreads threads with 4 or 8
