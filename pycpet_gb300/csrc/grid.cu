@@ -806,6 +806,86 @@ __global__ void __cluster_dims__(kPointCtas, 1, 1) __launch_bounds__(kPointThrea
 
 constexpr int kMagBins = 4096;  // bits 30..19 of the float |E|^2: exponent + 4 mantissa bits
 
+// A frame's scale from its histogram, by a whole block: the lower edge of the bin that
+// holds the lower median.
+__device__ __forceinline__ void frame_scale(const int* row, float* scale) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  // 32 consecutive bins per thread
+  constexpr int kPer = kMagBins / kGridThreads;
+  __shared__ int warp_sum[kGridThreads / 32];
+  int own[kPer], mine = 0;
+#pragma unroll
+  for (int b = 0; b < kPer; b += 4) {
+    const int4 h = __ldcg(reinterpret_cast<const int4*>(row + tid * kPer + b));
+    own[b] = h.x;
+    own[b + 1] = h.y;
+    own[b + 2] = h.z;
+    own[b + 3] = h.w;
+    mine += h.x + h.y + h.z + h.w;
+  }
+  int incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int w = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += w;
+  }
+  if (lane == 31) warp_sum[tid >> 5] = incl;
+  __syncthreads();
+  int total = 0;
+#pragma unroll
+  for (int w = 0; w < kGridThreads / 32; ++w) {
+    if (w < (tid >> 5)) incl += warp_sum[w];
+    total += warp_sum[w];
+  }
+  const int rank = (total - 1) / 2;
+  if (total > 0 && incl > rank && incl - mine <= rank) {
+    int cum = incl - mine, bin_of_rank = tid * kPer;
+#pragma unroll
+    for (int b = 0; b < kPer; ++b) {
+      if (cum <= rank && cum + own[b] > rank) bin_of_rank = tid * kPer + b;
+      cum += own[b];
+    }
+    *scale = __uint_as_float(static_cast<uint32_t>(bin_of_rank) << 19);
+  }  // no finite value: the scale stays 0 and nothing is refined
+}
+
+// A row's bin; -1: not finite (NaN compares false).
+__device__ __forceinline__ int mag_bin(const double (&v)[3]) {
+  const float m2 = field_norm2(v);
+  return m2 <= 3.0e38f ? static_cast<int>(__float_as_uint(m2) >> 19) : -1;
+}
+
+// A point's sum over its frame's splits, by one thread (th: thread of the tile t).
+template <int NC, int PPT>
+__device__ __forceinline__ void thread_sums(const GridFrame& fr, const double* __restrict__ partial, int t, int k,
+                                            int th, int ns, double (&v)[NC]) {
+  constexpr int kTilePts = kGridThreads * PPT;
+  const double* in = partial + (static_cast<int64_t>(fr.slot_base + t) * NC) * kTilePts + k * kGridThreads + th;
+  const int64_t step = static_cast<int64_t>(fr.n_tiles) * NC * kTilePts;
+  double w[NC][kSumLanes];
+#pragma unroll
+  for (int c = 0; c < NC; ++c)
+#pragma unroll
+    for (int s = 0; s < kSumLanes; ++s) w[c][s] = s < ns ? in[s * step + c * kTilePts] : 0.0;
+  for (int s0 = kSumLanes; s0 < ns; s0 += kSumLanes) {
+#pragma unroll
+    for (int s = 0; s < kSumLanes; ++s)
+      if (s0 + s < ns) {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) w[c][s] = __dadd_rn(w[c][s], in[(s0 + s) * step + c * kTilePts]);
+      }
+  }
+#pragma unroll
+  for (int c = 0; c < NC; ++c) v[c] = sum_thread(w[c]);
+}
+
+// The k-th point of thread th of a frame's tile t; -1 for none.
+template <int PPT>
+__device__ __forceinline__ int tile_point(const GridFrame& fr, const PointMap& map, int t, int th, int k) {
+  if (fr.few) return k * kGridThreads + th < fr.n_points ? k * kGridThreads + th : -1;
+  return map.point<PPT>(t * kGridThreads + th, k);
+}
+
 // Sums of the splits.  LANES = 1: block (tile, k), a thread takes the k-th point of
 // a tile's thread; LANES = 8: eight lanes per point and eight blocks.  HIST
 // (FP32C field refinement): also counts |E|^2 in 1/16-octave bins (of |E|^2; 1/32
@@ -828,39 +908,20 @@ __global__ void __launch_bounds__(kGridThreads)
   int f;
   const GridFrame fr = load_frame<offsetof(GridFrame, tile_base)>(frames, n_frames, one, tile, &f);
   const int t = tile - fr.tile_base;
-  int pl;
-  if (fr.few) {
-    pl = k * kGridThreads + th < fr.n_points ? k * kGridThreads + th : -1;
-  } else {
-    PointMap map;
-    map.set<PPT>(stride && !broken[f] ? stride[f] : 0, fr.n_points);
-    pl = map.point<PPT>(t * kGridThreads + th, k);
-  }
+  PointMap map;
+  map.set<PPT>(stride && !broken[f] ? stride[f] : 0, fr.n_points);
+  const int pl = tile_point<PPT>(fr, map, t, th, k);
   double v[NC];
 #pragma unroll
   for (int c = 0; c < NC; ++c) v[c] = 0.0;
   double* o = out + NC * (fr.point_off + max(pl, 0));
   if (fr.slot_base >= 0) {
-    const double* in = partial + (static_cast<int64_t>(fr.slot_base + t) * NC) * kTilePts + k * kGridThreads + th;
-    const int64_t step = static_cast<int64_t>(fr.n_tiles) * NC * kTilePts;
     const int ns = pl >= 0 ? fr.n_split : 0;
     if constexpr (LANES == 1) {
-      double w[NC][kSumLanes];
-#pragma unroll
-      for (int c = 0; c < NC; ++c)
-#pragma unroll
-        for (int s = 0; s < kSumLanes; ++s) w[c][s] = s < ns ? in[s * step + c * kTilePts] : 0.0;
-      for (int s0 = kSumLanes; s0 < ns; s0 += kSumLanes) {
-#pragma unroll
-        for (int s = 0; s < kSumLanes; ++s)
-          if (s0 + s < ns) {
-#pragma unroll
-            for (int c = 0; c < NC; ++c) w[c][s] = __dadd_rn(w[c][s], in[(s0 + s) * step + c * kTilePts]);
-          }
-      }
-#pragma unroll
-      for (int c = 0; c < NC; ++c) v[c] = sum_thread(w[c]);
+      thread_sums<NC, PPT>(fr, partial, t, k, th, ns, v);
     } else {
+      const double* in = partial + (static_cast<int64_t>(fr.slot_base + t) * NC) * kTilePts + k * kGridThreads + th;
+      const int64_t step = static_cast<int64_t>(fr.n_tiles) * NC * kTilePts;
 #pragma unroll
       for (int c = 0; c < NC; ++c) v[c] = l < ns ? in[l * step + c * kTilePts] : 0.0;
 #pragma unroll 4
@@ -879,8 +940,7 @@ __global__ void __launch_bounds__(kGridThreads)
   }
   if constexpr (HIST) {
     int* row = hist + static_cast<int64_t>(f) * kMagBins;
-    const float m2 = pl >= 0 && l == 0 ? field_norm2(v) : 4.0e38f;
-    const int bin = m2 <= 3.0e38f ? static_cast<int>(__float_as_uint(m2) >> 19) : -1;  // finite (NaN compares false)
+    const int bin = pl >= 0 && l == 0 ? mag_bin(v) : -1;
     const unsigned same = __match_any_sync(0xffffffffu, bin);
     if (bin >= 0 && lane == __ffs(same) - 1) atomicAdd(&row[bin], __popc(same));
     __shared__ int s_last;
@@ -890,43 +950,73 @@ __global__ void __launch_bounds__(kGridThreads)
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    // 32 consecutive bins per thread
-    constexpr int kPer = kMagBins / kGridThreads;
-    __shared__ int warp_sum[kGridThreads / 32];
-    int own[kPer], mine = 0;
+    frame_scale(row, scale + f);
+  }
+}
+
+// The same with one thread per point for many points (FP32C field): a block takes
+// `per` tiles and counts in shared memory, so that a frame's hot bins get one addition
+// per block instead of one per warp, and a frame one last-block check per block.  A
+// call of 101^3 points in no order x 20 charges 84 us (158 with the kernel above, 4e6
+// points 219 and 271); below about 300 tiles the blocks' 4,096 bins cost more than they
+// save (51^3 x 5,000, 260 tiles, 331 and 326; 24 frames of 20,000 points 670 and 674).
+// Eight blocks per SM: 219 us, 223 with six, 241 with the four of 128 registers.
+constexpr int kManyTiles = 300;
+template <int PPT>
+__global__ void __launch_bounds__(kGridThreads, 8)
+    grid_final_many_kernel(const GridFrame* __restrict__ frames, int n_frames, const GridFrame one, int n_tiles,
+                           int per, const int* __restrict__ stride, const int* __restrict__ broken,
+                           const double* __restrict__ partial, double* __restrict__ out, int* __restrict__ hist,
+                           int* __restrict__ done, float* __restrict__ scale) {
+  __shared__ int h[kMagBins];
+  __shared__ int s_last;
+  const int tid = threadIdx.x;
+  for (int b = tid; b < kMagBins; b += kGridThreads) h[b] = 0;
+  __syncthreads();
+  const int t1 = min(n_tiles, (static_cast<int>(blockIdx.x) + 1) * per);
+  int tile = static_cast<int>(blockIdx.x) * per;
+  while (tile < t1) {
+    int f;
+    const GridFrame fr = load_frame<offsetof(GridFrame, tile_base)>(frames, n_frames, one, tile, &f);
+    PointMap map;
+    map.set<PPT>(stride && !broken[f] ? stride[f] : 0, fr.n_points);
+    const int first = tile, end = min(t1, fr.tile_base + fr.n_tiles);
+    for (; tile < end; ++tile) {
 #pragma unroll
-    for (int b = 0; b < kPer; b += 4) {
-      const int4 h = __ldcg(reinterpret_cast<const int4*>(row + tid * kPer + b));
-      own[b] = h.x;
-      own[b + 1] = h.y;
-      own[b + 2] = h.z;
-      own[b + 3] = h.w;
-      mine += h.x + h.y + h.z + h.w;
-    }
-    int incl = mine;
+      for (int k = 0; k < PPT; ++k) {
+        const int pl = tile_point<PPT>(fr, map, tile - fr.tile_base, tid, k);
+        if (pl < 0) continue;
+        double* o = out + 3 * (fr.point_off + pl);
+        double v[3];
+        if (fr.slot_base >= 0) {
+          thread_sums<3, PPT>(fr, partial, tile - fr.tile_base, k, tid, fr.n_split, v);
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int w = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += w;
-    }
-    if (lane == 31) warp_sum[tid >> 5] = incl;
-    __syncthreads();
-    int total = 0;
+          for (int c = 0; c < 3; ++c) o[c] = v[c];
+        } else {
 #pragma unroll
-    for (int w = 0; w < kGridThreads / 32; ++w) {
-      if (w < (tid >> 5)) incl += warp_sum[w];
-      total += warp_sum[w];
-    }
-    const int rank = (total - 1) / 2;
-    if (total > 0 && incl > rank && incl - mine <= rank) {
-      int cum = incl - mine, bin_of_rank = tid * kPer;
-#pragma unroll
-      for (int b = 0; b < kPer; ++b) {
-        if (cum <= rank && cum + own[b] > rank) bin_of_rank = tid * kPer + b;
-        cum += own[b];
+          for (int c = 0; c < 3; ++c) v[c] = o[c];
+        }
+        const int bin = mag_bin(v);
+        if (bin >= 0) atomicAdd(&h[bin], 1);
       }
-      scale[f] = __uint_as_float(static_cast<uint32_t>(bin_of_rank) << 19);
-    }  // no finite value: the scale stays 0 and nothing is refined
+    }
+    // this block's part of the frame, and the frame's scale by its last block
+    int* row = hist + static_cast<int64_t>(f) * kMagBins;
+    __syncthreads();
+    for (int b = tid; b < kMagBins; b += kGridThreads)
+      if (h[b]) {
+        atomicAdd(&row[b], h[b]);
+        h[b] = 0;
+      }
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(&done[f], end - first) + (end - first) == fr.n_tiles;
+    __syncthreads();
+    if (s_last) {
+      __threadfence();
+      frame_scale(row, scale + f);
+    }
+    __syncthreads();
   }
 }
 
@@ -1330,7 +1420,13 @@ cudaError_t launch_grid_c(const GridLaunch& g, cudaStream_t s) {
   };
   if (refine) {
     if constexpr (KIND == kField && PREC == kFP32C) {
-      final_lanes(std::true_type{});
+      if (!lanes && g.n_tiles >= kManyTiles) {
+        const int per = std::max(1, g.n_tiles / (8 * std::max(g.num_sms, 1)));
+        grid_final_many_kernel<PPT><<<(g.n_tiles + per - 1) / per, kGridThreads, 0, s>>>(
+            g.frames, g.n_frames, g.one, g.n_tiles, per, stride, z.broken, g.partial, g.out, z.hist, z.done, z.scale);
+      } else {
+        final_lanes(std::true_type{});
+      }
       const dim3 fgrid(g.n_frames, std::min((g.max_points - 1) / kFlagChunk + 1, 65535));
       grid_flag_kernel<<<fgrid, kFlagThreads, 0, s>>>(g.frames, g.one, g.out, z.scale,
                                                       static_cast<float>(g.tau * g.tau), g.list, z.count);
@@ -1364,6 +1460,7 @@ cudaError_t preload_c() {
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, prep_kernel<PREC, true>);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, grid_final_kernel<PREC, KIND, PPT, true, 1>);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, grid_final_kernel<PREC, KIND, PPT, true, kSumLanes>);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, grid_final_many_kernel<PPT>);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, grid_flag_kernel);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, grid_refine_kernel<CLAMP>);
   }
