@@ -326,6 +326,27 @@ int plan_grid(int prec, int n_frames, const int64_t* desc, int sms, int ppt, int
   const double target = std::max(1.0, total / (double(std::max(sms, 1)) * items_per_sm));
   const bool mesh =
       grid_pair_evals(n_frames, desc) >= (prec == CPETGB_FP64 ? kGridMeshPairsFp64 : kGridMeshPairsFp32);
+  // Is a frame looked at for a mesh?  Not when columns may need a tile more and such
+  // spare tiles are a sixth of the launch's tiles or above: mesh or not, their CTAs fall
+  // on the same SMs again and again (tiles side by side, an even number of SMs) and cost
+  // the launch more than columns save.  Potential, without a look and with one: 100 frames
+  // of 512 points x 1,000 charges 28 and 44 us, of 11^3 x 1,000 52 and 60, one of 11^3 x
+  // 40,000 43 and 50; 64 of 16^3 x 4,000, eight tiles and one, 269 and 255.  (Splits side
+  // by side instead spread them, but 24 frames' fields took 2.19 ms instead of 2.13.)
+  const int64_t few = prec == CPETGB_FP64 ? kGridFewPoints : kGridFewPointsFp32;
+  auto worth = [&](int64_t n, int64_t P) {
+    return mesh && P > few && n >= (prec == CPETGB_FP64 ? kGridMeshChargesFp64 : kGridMeshChargesFp32);
+  };
+  auto column_tiles = [&](int64_t P) { return ((P + ppt - 1) / ppt + 64 + kGridThreads - 1) / kGridThreads; };
+  int64_t tiles = 0, spare = 0;
+  for (int f = 0; f < n_frames; ++f) {
+    const int64_t n = desc[4 * f + 1], P = desc[4 * f + 3];
+    if (P > few) tiles += full_tiles(P);
+    if (worth(n, P)) spare += column_tiles(P) - full_tiles(P);
+  }
+  auto looks = [&](int64_t n, int64_t P) {
+    return worth(n, P) && (6 * spare < tiles || column_tiles(P) == full_tiles(P));
+  };
   t.frames.resize(size_t(n_frames));
   for (int f = 0; f < n_frames; ++f) {
     const int64_t n = desc[4 * f + 1], P = desc[4 * f + 3];
@@ -335,7 +356,7 @@ int plan_grid(int prec, int n_frames, const int64_t* desc, int sms, int ppt, int
     fr.point_off = desc[4 * f + 2];
     fr.n_charges = static_cast<int32_t>(n);
     fr.n_points = static_cast<int32_t>(P);
-    fr.few = P > 0 && P <= (prec == CPETGB_FP64 ? kGridFewPoints : kGridFewPointsFp32);
+    fr.few = P > 0 && P <= few;
     int64_t split = 1;
     if (n > 0) {
       split = static_cast<int64_t>(std::ceil(double(tile) * double(n) / target));
@@ -349,9 +370,8 @@ int plan_grid(int prec, int n_frames, const int64_t* desc, int sms, int ppt, int
     if (n > 0) split = (n + chunk - 1) / chunk;
     fr.chunk = static_cast<int32_t>(chunk);
     fr.n_split = static_cast<int32_t>(split);
-    // mesh columns and the other points are rounded up to warps separately
-    const int64_t threads = (P + ppt - 1) / ppt + 64;
-    fr.n_tiles = P == 0 ? 0 : (fr.few ? 1 : static_cast<int32_t>((threads + kGridThreads - 1) / kGridThreads));
+    // (a mesh's columns and its other points are rounded up to warps separately)
+    fr.n_tiles = P == 0 ? 0 : (fr.few ? 1 : static_cast<int32_t>(looks(n, P) ? column_tiles(P) : full_tiles(P)));
   }
   // few-points frames first; the others longest chunk first, so the last wave
   // holds the shortest items
@@ -369,7 +389,7 @@ int plan_grid(int prec, int n_frames, const int64_t* desc, int sms, int ppt, int
     if (fr.n_split > 1) t.n_slots += items;
     if (fr.few) {
       t.few_items += items;
-    } else if (mesh && fr.n_charges >= (prec == CPETGB_FP64 ? kGridMeshChargesFp64 : kGridMeshChargesFp32)) {
+    } else if (looks(fr.n_charges, fr.n_points)) {
       t.n_prep += (int64_t(fr.n_points) + kGridPrepPoints - 1) / kGridPrepPoints;
     }
     if (t.n_items > INT_MAX || t.n_tiles * ppt > INT_MAX)

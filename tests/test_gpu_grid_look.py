@@ -79,3 +79,24 @@ def test_frames_with_and_without_a_look(no_refinement, precision):
         np.testing.assert_array_equal(esp_grid(p[order], x, q, precision=precision), ref[order])
         tol = 1e-12 if precision == "fp64" else 2e-6   # other charge chunks than alone
         assert np.abs(out.reshape(-1) - ref).max() <= tol * max(np.abs(ref).max(), 1e-300)
+
+
+@pytest.mark.parametrize("kind", ["field", "esp"])
+@pytest.mark.parametrize("precision", ["fp32c", "fp64"])
+def test_tables_of_small_frames(no_refinement, kind, precision):
+    """Frames of one to nine tiles with room for columns in their last one and without,
+    meshes and not: the bits of the same table with every frame's points shuffled."""
+    from pycpet_gb300 import GridBatch
+
+    shapes = [(8, 8, 8), (7, 8, 8), (5, 10, 10), (11, 11, 11), (12, 12, 14), (16, 16, 8), (16, 16, 16), (15, 15, 15), (6, 6, 6)]
+    frames, shuffled, orders = [], [], []
+    for i, s in enumerate(shapes * 3):
+        pts = _mesh(*s)
+        x, q = _charges((600, 900, 40)[i // len(shapes)])
+        order = np.random.default_rng(i).permutation(len(pts))
+        frames.append((pts, x, q))
+        shuffled.append((pts[order], x, q))
+        orders.append(order)
+    a, b = (GridBatch(f, kind=kind, precision=precision) for f in (frames, shuffled))
+    for order, u, v in zip(orders, a.split(a.run()), b.split(b.run())):
+        np.testing.assert_array_equal(u[order], v)
