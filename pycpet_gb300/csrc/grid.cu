@@ -226,7 +226,8 @@ __device__ __forceinline__ void grid_tile_f32x2(const ChargeDup* __restrict__ tl
 #pragma unroll 8
       for (int j = j0; j < j1; ++j) column_terms_f32x2<KIND, G>(tl[j], px, y, z, part);
     } else {
-#pragma unroll 4
+// (potential: 522 us per 101^3 points in no order x 2,000 charges, 528 with four)
+#pragma unroll (KIND == kEsp ? 8 : 4)
       for (int j = j0; j < j1; ++j) pair_terms_f32x2<KIND, false, G>(tl[j], px, py, pz, part);
     }
 #pragma unroll
@@ -1256,7 +1257,9 @@ __global__ void __launch_bounds__(kRefineThreads, 2)
 }
 
 constexpr int kPrepThreads = 256;
-constexpr int kPrepCharges = 1024;   // charges per preparation block
+// Charges per preparation block: one per thread, as the loads' latency is what a small
+// launch waits for (2,000 charges 3.3 us, 5.3 with four per thread).
+constexpr int kPrepCharges = 256;
 
 __device__ __forceinline__ bool same_yz(const double* a, const double* b, bool f32) {
   if (f32)  // the FP32C kernels see the FP32 images
