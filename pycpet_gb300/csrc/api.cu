@@ -673,10 +673,12 @@ int topo_impl(int prec, int mem, int L, int N, const double* starts, const int32
   unsigned char* packed = nullptr;
   int* queue = nullptr;  // the queue counter and, per round, the count of lines handed over
   TopoState* left = nullptr;
-  int rounds = topo_team_rounds(c->sms, L, topo_diag_steps(half, step));
-  const bool fresh = topo_fresh(prec, topo_resident_count(prec, source, static_cast<int>(n_pad)) == n_pad, L,
-                                c->sms, true);
-  const int left_cap = fresh && rounds == 1 ? 0 : topo_left_capacity(c->sms, L, fresh);
+  const double diag_steps = topo_diag_steps(half, step);
+  int rounds = topo_team_rounds(c->sms, L, diag_steps);
+  const bool whole = topo_resident_count(prec, source, static_cast<int>(n_pad)) == n_pad;
+  const bool fresh = topo_fresh(prec, source, whole, double(n_pad), L, c->sms, true);
+  const bool records = fresh ? rounds > 1 : topo_hands_over(prec, source, whole, static_cast<int>(n_pad), diag_steps);
+  const int left_cap = records ? topo_left_capacity(c->sms, L, fresh) : 0;
   CK(S.get(&packed, size_t(n_pad) * topo_source_bytes(prec, source)), "alloc packed charges");
   CK(S.get(&queue, size_t(1 + rounds)), "alloc queue");
   CK(cudaMemsetAsync(queue, 0, (1 + rounds) * sizeof(int), s), "zero queue");
@@ -727,6 +729,7 @@ struct TopoTables {
   std::vector<int64_t> src;  // per frame {charge offset, charge count} into x/q
   int64_t tot_lines = 0, tot_ch = 0, packed_elems = 0;
   int64_t sum_lines = 0;      // lines of all frames (frames may share ranges)
+  double line_sources = 0.0;  // sources of all lines
   int64_t left_records = 0;   // hand-over records of all frames
   int rounds = 1;             // team kernel launches
   bool fresh = false;         // every line in them from its start point
@@ -766,6 +769,7 @@ int build_topo_tables(int prec, int F, const int64_t* desc, const double* params
     fr.team_resident = topo_team_resident(prec, kCharges, fr.n_pad);
     t.max_team_res = std::max(t.max_team_res, int(fr.team_resident));
     t.sum_lines += L;
+    t.line_sources += double(L) * double(fr.n_pad);
     t.diag_steps = std::max(t.diag_steps, topo_diag_steps(pr + 1, pr[0]));
     fr.step = pr[0];
     for (int k = 0; k < 3; ++k) fr.half[k] = pr[1 + k];
@@ -783,9 +787,13 @@ int build_topo_tables(int prec, int F, const int64_t* desc, const double* params
 
 void plan_hand_over(int prec, int sms, TopoTables& t) {
   t.rounds = topo_team_rounds(sms, t.sum_lines, t.diag_steps);
-  t.fresh = topo_fresh(prec, t.all_resident, t.sum_lines, sms, true);
+  t.fresh = topo_fresh(prec, kCharges, t.all_resident, t.line_sources / double(std::max<int64_t>(t.sum_lines, 1)),
+                       t.sum_lines, sms, true);
   for (TopoFrame& fr : t.frames) {
-    const int64_t cap = t.fresh && t.rounds == 1 ? 0 : topo_left_capacity(sms, fr.n_lines, t.fresh);
+    const bool records = t.fresh ? t.rounds > 1
+                                 : topo_hands_over(prec, kCharges, fr.resident == fr.n_pad, fr.n_pad,
+                                                   topo_diag_steps(fr.half, fr.step));
+    const int64_t cap = records ? topo_left_capacity(sms, fr.n_lines, t.fresh) : 0;
     fr.left_off = static_cast<int32_t>(t.left_records);
     fr.left_cap = t.left_records + cap <= kMaxLeft ? static_cast<int32_t>(cap) : 0;
     t.left_records += fr.left_cap;

@@ -195,10 +195,12 @@ double topo_diag_steps(const double* half, double step);
 constexpr int kTeamLinesPerSm = 16;
 constexpr int64_t kMaxLeft = int64_t(1) << 18;  // hand-over records of a launch: two lists of 42 MB
 // Whether a launch's lines go to the team kernel from their start points
-// (resident: every frame's sources fit shared memory; lists: hand-over records may
-// be asked for).  Decided once, by who plans the launch; that there is no memory for
-// the records in the end does not change it.
-bool topo_fresh(int prec, bool resident, int64_t sum_lines, int num_sms, bool lists);
+// (resident: every frame's sources fit shared memory; n_pad: a line's sources, on
+// average; lists: hand-over records may be asked for).  Decided once, by who plans the
+// launch; that there is no memory for the records in the end does not change it.
+bool topo_fresh(int prec, int source, bool resident, double n_pad, int64_t sum_lines, int num_sms, bool lists);
+// Whether a frame's last lines are worth handing over (diag_steps: steps across its box).
+bool topo_hands_over(int prec, int source, bool resident, int n_pad, double diag_steps);
 
 // max sources (charges or dipoles) held resident in shared memory
 size_t topo_resident_limit(int prec, int source = kCharges);

@@ -112,7 +112,7 @@ extern "C" int cpetgb_topo_lines_noalloc(int precision, int n_lines, int n_charg
     p.queue = counters;
     p.status = counters + 1;
     const bool whole = topo_resident_count(precision, kCharges, static_cast<int>(n_pad)) == n_pad;
-    p.fresh = topo_fresh(precision, whole, n_lines, sms, false);
+    p.fresh = topo_fresh(precision, kCharges, whole, double(n_pad), n_lines, sms, false);
     e = launch_topo(precision, p, sms, s);
   }
   int st = 0;

@@ -37,6 +37,7 @@
 //   FP64   every operation in IEEE double; charges read from global memory
 //          (L2-resident) as (x,y,z,q) doubles.
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 #include "common.cuh"
@@ -851,21 +852,50 @@ cudaError_t launch_topo(int prec, const TopoParams& p_in, int num_sms, cudaStrea
   return launch_topo_team(prec, p, f0, 0, num_sms, s);
 }
 
-// Up to 16 lines per SM the persistent kernel has less than a line per warp.  Above
-// that, all lines kept in the rounds of teams, against the persistent kernel and
-// rounds for its last lines (GB300, lines per SM: ms, box of 3 A, ends at the box):
-//   FP64    1,000 charges  24: 21.6 against 27.7   64: 54.1 / 62.4   256: 198 / 213
-//           4,000 charges, 52 steps across the box  24: 7.3 / 7.8  128: 31.7 / 34.9
-//   FP32C   3,000 charges  17: 17.2 / 19.6  20: 18.9 / 20.6  24: 21.6 / 21.8  33: 26.3 / 24.5
-//           8,000 charges  17: 19.9 / 22.4  24: 25.4 / 27.9  48: 44.4 / 40.1
-//           40,000 charges 17: 49.5 / 63.4  24: 64.3 / 76.6  33: 87.9 / 96.6, larger
-//           steps  33: 19.6 / 20.4  40: 23.6 / 22.3
-// A team has the FP64 pipe busy with a line per warp; in FP32C the persistent kernel
-// reaches the pipe's rate from 32 lines per SM on, later where sources come from L2.
-bool topo_fresh(int prec, bool resident, int64_t sum_lines, int num_sms, bool lists) {
-  int64_t per_sm = kTeamLinesPerSm;
-  if (lists) per_sm = prec == kFP64 ? kMaxLeft : (resident ? 20 : 32);
+// FP64: a team has the FP64 pipe busy with a line per warp.  All lines in the rounds of
+// teams against the persistent kernel with rounds for its last lines (GB300, lines per
+// SM: ms):
+//   1,000 charges  24: 21.6 against 27.7   64: 54.1 / 62.4   256: 198 / 213
+//   4,000 charges, 52 steps across the box  24: 7.3 / 7.8  128: 31.7 / 34.9
+// FP32C: teams / the persistent kernel with hand-over / without, us, box of 3 A, 5,200
+// steps across it (step 0.001 A), lines per SM:
+//             2                     8                      16                     20                     24                     32
+//   charges
+//   1,000     5790 / -  /  5169     6743 / -  /  5940      8157 / -  /  7496      9431 / 10678 /  7923                          12506 / 11601 /  9522
+//   2,000     5853 / -  /  4854     6925 / -  /  5961      8822 / -  /  8314     10448 / 11783 /  9409                          14273 / 13356 / 11211
+//   3,000     7174 / -  /  7981     9205 / -  /  9361     11831 / -  / 12105     14058 / 16183 / 13613   16233 / 17228 / 13886  18766 / 17371 / 16634
+//   4,000     7615 / -  /  9372     9776 / -  / 10892     12622 / -  / 13777     15138 / 15592 / 14935   17181 / 18431 / 16630  19858 / 19640 / 19232
+//   6,000     8311 / -  / 12029    12804 / -  / 15484     17832 / -  / 21737     21625 / 24633 / 26980   25612 / 28730 / 27059  30210 / 32381 / 32623
+//   8,000     7580 / -  / 12616    11926 / -  / 17704     18056 / -  / 22583     22245 / 26988 / 31413   26041 / 30187 / 30920  32153 / 36388 / 39136
+//   dipoles
+//   2,000     9106 / -  /  7581    10565 / -  /  9206     13228 / -  / 13443     15715 / 17253 / 14344                          20135 / 19568 / 17889
+//   4,000     9604 / -  / 12086    13185 / -  / 16321     18836 / -  / 20941     23929 / 26773 / 26980   27096 / 28859 / 28319  31800 / 36513 / 36416
+// and with a tenth of the steps (rounds of 128 steps at least, so a launch's 10 us count):
+//   3,000      755 / -  /   823     1006 / -  /   968      1352 / -  /  1251      1715 /  1793 /  1408                           2064 /  1911 /  1728
+//   8,000      800 / -  /  1310     1439 / -  /  1829      2062 / -  /  2343      2716 /  3040 /  3246    3060 /  3425 /  3198   3745 /  3930 /  4028
+//   8,000 dip 1098 / -  /  2090     2025 / -  /  2876      3169 / -  /  3752      3824 /  4296 /  4730    4442 /  4803 /  5920   5352 /  5478 /  6082
+//   30,000    1865 / -  /  8113     3948 / -  /  9229      6880 / -  / 10177      9370 / 10075 / 13370   10260 / 12245 / 14168  12191 / 13756 / 16096
+// A frame of one Kahan run (2,048 sources) has nothing to split, so teams only add their
+// barriers and rounds; with two runs they pay up to 9 to 16 lines per SM, from three on
+// to 20, and to 32 where the persistent kernel reads sources from L2.  Hand-over
+// pays where a line alone on a warp is slow (sources from L2, 200 pairs' work per lane), or
+// with less work where lines are long.
+bool topo_fresh(int prec, int source, bool resident, double n_pad, int64_t sum_lines, int num_sms, bool lists) {
+  int64_t per_sm = kMaxLeft;
+  if (prec != kFP64) {
+    const double lane_pairs = n_pad / 64.0;
+    if (lane_pairs <= kLanePairs) return false;
+    per_sm = std::min<int64_t>(resident ? 20 : 32,
+                               static_cast<int64_t>(std::ceil(lane_pairs / (source == kDipoles ? 3 : 4))));
+  }
+  if (!lists) per_sm = std::min<int64_t>(per_sm, kTeamLinesPerSm);
   return sum_lines <= std::min(per_sm * num_sms, std::max(kMaxLeft, int64_t(kTeamLinesPerSm) * num_sms));
+}
+
+bool topo_hands_over(int prec, int source, bool resident, int n_pad, double diag_steps) {
+  if (prec == kFP64 || !resident) return true;
+  const double work = n_pad / 64.0 * (source == kDipoles ? 1.75 : 1.0);  // charge pairs per lane
+  return work >= 200.0 || (work >= 120.0 && diag_steps >= 2000.0);
 }
 
 int topo_left_capacity(int num_sms, int64_t n_lines, bool fresh) {

@@ -60,3 +60,37 @@ def test_frames_beyond_the_records(gpu_lib):
         at = slice(f * per_frame, (f + 1) * per_frame)
         np.testing.assert_array_equal(res[at], r)
         np.testing.assert_array_equal(steps[at], s)
+
+
+# both sides of a Kahan run (2,048 sources) and of the work from which lines are handed
+# over (7,680 charges when lines are long), with few and many lines per SM
+@pytest.mark.parametrize("n,step,per_sm", [(2048, 0.01, 3), (2049, 0.01, 9), (2049, 0.01, 11), (4000, 0.01, 17),
+                                           (7616, 0.0015, 22), (7680, 0.0015, 22), (7680, 0.02, 22)])
+def test_routes_agree(gpu_lib, n, step, per_sm):
+    """The launch as planned against the allocation-free one, a table of two such frames,
+    and a table whose other frame's size puts it on the other route."""
+    import torch
+    from pycpet_gb300 import TopoBatch, _lib, topo_lines
+
+    rng = np.random.default_rng(n)
+    x = rng.uniform(-40.0, 40.0, (2 * n, 3))
+    x = x[np.linalg.norm(x, axis=1) > 3.0][:n]
+    q = rng.normal(0.0, 0.4, n)
+    L = per_sm * gpu_lib.cpetgb_device_sms() - 5
+    starts, caps = rng.uniform(-1.2, 1.2, (L, 3)), rng.integers(0, 150, L).astype(np.int32)
+    half = np.array([1.5, 1.5, 1.2])
+    want, want_steps = topo_lines(starts, caps, x, q, step, half, return_steps=True)
+    dev = [torch.from_numpy(a).cuda() for a in (starts, caps, x, q)]
+    res = torch.empty((L, 2), dtype=torch.float64, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    rc = gpu_lib.cpetgb_topo_lines_noalloc(_lib.FP32C, L, n, dev[0].data_ptr(), dev[1].data_ptr(), step,
+                                           half.ctypes.data, dev[2].data_ptr(), dev[3].data_ptr(), res.data_ptr(),
+                                           None, None, stream)
+    assert rc == 0, _lib.last_error()
+    np.testing.assert_array_equal(res.cpu().numpy(), want)
+    frame = {"x": x, "q": q, "starts": starts, "n_iter": caps, "step": step, "half_dims": half}
+    other = dict(frame, x=x[: n // 3], q=q[: n // 3], starts=starts[:300], n_iter=caps[:300])
+    for frames in ([frame, frame], [other, frame]):
+        r, s = TopoBatch(frames, precision="fp32c").run(return_steps=True)
+        np.testing.assert_array_equal(r[-L:], want)
+        np.testing.assert_array_equal(s[-L:], want_steps)
