@@ -821,6 +821,18 @@ cudaError_t launch_topo_prec(int prec, bool whole, const TopoParams& p, const To
                : launch_topo_s<kFP32C, DIP, kSrcSplit>(p, f0, num_sms, s, slots);
 }
 
+// Line slots per warp: the tuned variant of the launch's class, which knows its lines
+// but not its sources; 4 for frames of at most 1,024 sources once a CTA's slots are filled
+// more than once, as a step then is mostly what a warp pays once for all of its lines.
+// Four slots and two, 108 / 197 / 395 lines per SM (us): 60 charges 925 and 1,207 / 1,398
+// and 1,946 / 2,359 and 3,563; 1,000 charges 1,848 and 2,141 / 2,892 and 3,405 / 5,129 and
+// 6,362; but 2,000 charges 2,697 and 2,447 / 4,130 and 4,007 / 7,279 and 7,522.
+constexpr int kFewSources = 1024;
+int topo_slots(int prec, bool whole, const TopoParams& p, int64_t lines, int num_sms) {
+  if (prec == kFP32C && whole && p.max_resident_pad <= kFewSources && lines > 96 * int64_t(num_sms)) return 4;
+  return tuned_topo_slots(prec, whole, p.n_lines);
+}
+
 // Single frame: p.packed holds round_up(n_charges, topo_charge_pad(prec)) charges
 // packed by launch_pack_topo (the tail being zero charges far from the box).
 cudaError_t launch_topo(int prec, const TopoParams& p_in, int num_sms, cudaStream_t s) {
@@ -844,7 +856,7 @@ cudaError_t launch_topo(int prec, const TopoParams& p_in, int num_sms, cudaStrea
   const bool whole = f0.resident == f0.n_pad;
   f0.left_cap = p.left ? topo_left_capacity(num_sms, p.n_lines, p.fresh) : 0;
   if (p.fresh) return launch_topo_team(prec, p, f0, 1, num_sms, s);
-  const int slots = tuned_topo_slots(prec, whole, p.n_lines);
+  const int slots = topo_slots(prec, whole, p, p.n_lines, num_sms);
   const cudaError_t e = p.source == kDipoles
                             ? launch_topo_prec<true>(prec, whole, p, f0, num_sms, s, slots)
                             : launch_topo_prec<false>(prec, whole, p, f0, num_sms, s, slots);
@@ -908,7 +920,7 @@ cudaError_t launch_topo_frames(int prec, const TopoParams& p, int num_sms, cudaS
   if (p.n_frames <= 0 || p.n_lines <= 0 || p.sum_lines <= 0) return cudaSuccess;
   TopoFrame dummy{};
   if (p.fresh) return launch_topo_team(prec, p, dummy, 1, num_sms, s);
-  const int slots = tuned_topo_slots(prec, p.all_resident != 0, p.n_lines);
+  const int slots = topo_slots(prec, p.all_resident != 0, p, p.sum_lines, num_sms);
   const cudaError_t e = launch_topo_prec<false>(prec, p.all_resident != 0, p, dummy, num_sms, s, slots);
   if (e != cudaSuccess || !p.left) return e;
   return launch_topo_team(prec, p, dummy, 0, num_sms, s);
