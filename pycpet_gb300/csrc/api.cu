@@ -12,6 +12,7 @@
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -206,6 +207,33 @@ cudaError_t h2d(T** dst, Scratch& S, const T* src, size_t count) {
   if (e == cudaSuccess && count)
     e = cudaMemcpyAsync(*dst, src, count * sizeof(T), cudaMemcpyHostToDevice, S.s);
   return e;
+}
+
+// A table of the call's own.  Where the call is recorded into a caller's CUDA graph the
+// copy is a node that reads its source at every replay, long after the call has freed its
+// table, so the graph gets a copy of the table to keep.
+template <typename T>
+cudaError_t h2d_table(T** dst, Scratch& S, const T* src, size_t count) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  cudaGraph_t graph = nullptr;
+  cudaError_t e = cudaStreamGetCaptureInfo(S.s, &status, nullptr, &graph, nullptr, nullptr, nullptr);
+  if (e != cudaSuccess) return e;
+  if (status != cudaStreamCaptureStatusActive || count == 0) return h2d(dst, S, src, count);
+  T* kept = static_cast<T*>(std::malloc(count * sizeof(T)));
+  if (!kept) return cudaErrorMemoryAllocation;
+  std::memcpy(kept, src, count * sizeof(T));
+  cudaUserObject_t owner;
+  e = cudaUserObjectCreate(&owner, kept, [](void* p) { std::free(p); }, 1, cudaUserObjectNoDestructorSync);
+  if (e != cudaSuccess) {
+    std::free(kept);
+    return e;
+  }
+  e = cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove);
+  if (e != cudaSuccess) {
+    cudaUserObjectRelease(owner, 1);
+    return e;
+  }
+  return h2d(dst, S, static_cast<const T*>(kept), count);
 }
 
 // Hand-over records (cpetgb_set_hand_over_records).
@@ -477,7 +505,8 @@ struct GridWork {
     g.packed = packed;
     if (g.n_frames != 1) {
       GridFrame* d_frames = nullptr;
-      CK(h2d(&d_frames, S, plan.frames.data(), plan.frames.size()), "copy frame table");
+      CK(h2d_table(&d_frames, S, static_cast<const GridFrame*>(plan.frames.data()), plan.frames.size()),
+         "copy frame table");
       g.frames = d_frames;
     }
     CK(S.get(&g.zeroed, zero_ints()), "alloc counters");
@@ -846,8 +875,8 @@ int topo_batch_impl(int prec, int mem, int F, const int64_t* desc, const double*
      "alloc packed charges");
   if (reinterpret_cast<uintptr_t>(packed) % 16 != 0)
     return fail(CPETGB_ECUDA, "scratch allocation is not 16-byte aligned");
-  CK(h2d(&d_frames, S, frames.data(), frames.size()), "copy frame table");
-  CK(h2d(&d_src, S, src.data(), src.size()), "copy frame sources");
+  CK(h2d_table(&d_frames, S, static_cast<const TopoFrame*>(frames.data()), frames.size()), "copy frame table");
+  CK(h2d_table(&d_src, S, static_cast<const int64_t*>(src.data()), src.size()), "copy frame sources");
   TopoState* left = nullptr;
   CK(S.get(&queues, size_t(1 + t.rounds) * F), "alloc queues");
   CK(cudaMemsetAsync(queues, 0, sizeof(int) * size_t(1 + t.rounds) * F, s), "zero queues");
@@ -962,7 +991,7 @@ int hist_sets_impl(int mem, int n_sets, const int64_t* offsets, const double* va
   if (mem == CPETGB_HOST || !counts) CK(S.get(&dc, total), "alloc counts");
   if (mem == CPETGB_HOST && hists) CK(S.get(&dh, total), "alloc histograms");
   CK(S.get(&de, size_t(nb0 + nb1 + 2)), "alloc edges");
-  CK(h2d(&doff, S, offsets, size_t(n_sets) + 1), "copy offsets");
+  CK(h2d_table(&doff, S, offsets, size_t(n_sets) + 1), "copy offsets");
   CK(cudaMemsetAsync(dc, 0, total * sizeof(unsigned long long), s), "zero counts");
   CK(launch_hist2d_sets(n_sets, doff, max_set, dv, nb0, nb1, range, de, dc, hists ? dh : nullptr,
                         c->status, s),
