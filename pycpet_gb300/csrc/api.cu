@@ -67,9 +67,10 @@ int cuda_fail(cudaError_t e, const char* what) {
   } while (0)
 
 // Pinned staging buffers of the float32 host calls: kStagingBuffers of kStagingBytes
-// for the whole process, allocated together on the first such call or with the first
-// engine, and never during another call: page-locking memory waits for kernels in
-// flight (2.6 s behind a busy streamline engine).  A call that is larger, or that finds
+// for the whole process, allocated together with the first engine, or else on the first
+// such call.  Page-locking memory waits for kernels in flight on the device (2.6 s behind
+// a busy streamline engine), so that one call may wait for other threads' kernels; none
+// after it does.  A call that is larger, or that finds
 // no buffer free, copies from and to the caller's pageable arrays.  A buffer belongs
 // to one call at a time (any thread, any stream) and goes back after the call has
 // waited for its copies.  8 MB hold a call of 51^3 points and 100,000 charges.

@@ -23,11 +23,11 @@
 // Bound: the MUFU reciprocals, one per term: a warp's takes a scheduler's unit 8
 // cycles, and a loop of this body on registers alone 16.9 cycles per pair of terms
 // (10.3 without the reciprocals); two terms can't share one, 1 / (s t) rounds
-// differently.  1,024 histograms of 400 bins: pack 3, tiles 59 (51 at 16.9 cycles),
-// merge 9 us; 96 us per call before, with row-major staging and the splits summed in
-// double.  3 CTAs per SM: 59.4 us,
-// against 63.5 with the 2 that unlimited registers leave and 60.3 with 4; 2 x 4 and
-// 4 x 2 entries per thread 59.4 to 65.5; 32 x 16 tiles in one pass without splits 65.6.
+// differently.  1,024 histograms of 400 bins: pack 3, tiles 60 (51 at 16.9 cycles),
+// merge 11 us, 78 us per call; 96 before, with row-major staging and the splits summed
+// in double.  A call with 3 or 4 CTAs per SM and 1, 2 or 4 bins per turn: 3 and 2
+// 78 us, 3 and 1 86, 3 and 4 82, 4 and 1 to 4 82 to 84; 2 x 4 and 4 x 2 entries per
+// thread, and 32 x 16 tiles in one pass without splits, up to 6 us longer.
 #include <algorithm>
 #include <cfloat>
 #include <cstdint>

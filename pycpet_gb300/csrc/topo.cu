@@ -606,8 +606,6 @@ __global__ void pack_pairs_kernel(int64_t n, int64_t n_pad, const double* __rest
   }
 }
 
-// Dynamic shared memory: slot records, the mbarrier, and the resident sources
-// (16 bytes per FP32C charge, 24 per FP32C dipole).
 // Dipoles, FP32C: A[p] = {x, x', y, y'}, B[p] = {z, z', 3 mu_x, 3 mu_x'},
 // C[p] = {mu_y, mu_y', mu_z, mu_z'} for the pair (2p, 2p + 1); padding =
 // zero moments far outside any box (they add exactly 0).
@@ -650,6 +648,8 @@ __global__ void pack_dipole64_kernel(int64_t n, int64_t n_pad, const double* __r
   }
 }
 
+// Dynamic shared memory: slot records, the mbarrier, and the resident sources
+// (16 bytes per FP32C charge, 24 per FP32C dipole).
 size_t topo_smem_bytes(int S, int max_resident_pad, bool dip = false) {
   return sizeof(SlotRec) * kTopoWarps * S + 128 +
          static_cast<size_t>(max_resident_pad) * (dip ? 24 : 16);
@@ -869,24 +869,24 @@ cudaError_t launch_topo(int prec, const TopoParams& p_in, int num_sms, cudaStrea
 // SM: ms):
 //   1,000 charges  24: 21.6 against 27.7   64: 54.1 / 62.4   256: 198 / 213
 //   4,000 charges, 52 steps across the box  24: 7.3 / 7.8  128: 31.7 / 34.9
-// FP32C: teams / the persistent kernel with hand-over / without, us, box of 3 A, 5,200
-// steps across it (step 0.001 A), lines per SM:
-//             2                     8                      16                     20                     24                     32
-//   charges
-//   1,000     5790 / -  /  5169     6743 / -  /  5940      8157 / -  /  7496      9431 / 10678 /  7923                          12506 / 11601 /  9522
-//   2,000     5853 / -  /  4854     6925 / -  /  5961      8822 / -  /  8314     10448 / 11783 /  9409                          14273 / 13356 / 11211
-//   3,000     7174 / -  /  7981     9205 / -  /  9361     11831 / -  / 12105     14058 / 16183 / 13613   16233 / 17228 / 13886  18766 / 17371 / 16634
-//   4,000     7615 / -  /  9372     9776 / -  / 10892     12622 / -  / 13777     15138 / 15592 / 14935   17181 / 18431 / 16630  19858 / 19640 / 19232
-//   6,000     8311 / -  / 12029    12804 / -  / 15484     17832 / -  / 21737     21625 / 24633 / 26980   25612 / 28730 / 27059  30210 / 32381 / 32623
-//   8,000     7580 / -  / 12616    11926 / -  / 17704     18056 / -  / 22583     22245 / 26988 / 31413   26041 / 30187 / 30920  32153 / 36388 / 39136
-//   dipoles
-//   2,000     9106 / -  /  7581    10565 / -  /  9206     13228 / -  / 13443     15715 / 17253 / 14344                          20135 / 19568 / 17889
-//   4,000     9604 / -  / 12086    13185 / -  / 16321     18836 / -  / 20941     23929 / 26773 / 26980   27096 / 28859 / 28319  31800 / 36513 / 36416
-// and with a tenth of the steps (rounds of 128 steps at least, so a launch's 10 us count):
-//   3,000      755 / -  /   823     1006 / -  /   968      1352 / -  /  1251      1715 /  1793 /  1408                           2064 /  1911 /  1728
-//   8,000      800 / -  /  1310     1439 / -  /  1829      2062 / -  /  2343      2716 /  3040 /  3246    3060 /  3425 /  3198   3745 /  3930 /  4028
-//   8,000 dip 1098 / -  /  2090     2025 / -  /  2876      3169 / -  /  3752      3824 /  4296 /  4730    4442 /  4803 /  5920   5352 /  5478 /  6082
-//   30,000    1865 / -  /  8113     3948 / -  /  9229      6880 / -  / 10177      9370 / 10075 / 13370   10260 / 12245 / 14168  12191 / 13756 / 16096
+// FP32C: teams / the persistent kernel with hand-over (from 20 lines per SM) / without
+// (us; box of 3 A, 5,200 steps across it):
+//   lines per SM       2            8            16               20                   32
+//   1,000 charges   5790/ 5169   6743/ 5940   8157/ 7496    9431/10678/ 7923   12506/11601/ 9522
+//   2,000 charges   5853/ 4854   6925/ 5961   8822/ 8314   10448/11783/ 9409   14273/13356/11211
+//   3,000 charges   7174/ 7981   9205/ 9361  11831/12105   14058/16183/13613   18766/17371/16634
+//   4,000 charges   7615/ 9372   9776/10892  12622/13777   15138/15592/14935   19858/19640/19232
+//   6,000 charges   8311/12029  12804/15484  17832/21737   21625/24633/26980   30210/32381/32623
+//   8,000 charges   7580/12616  11926/17704  18056/22583   22245/26988/31413   32153/36388/39136
+//   2,000 dipoles   9106/ 7581  10565/ 9206  13228/13443   15715/17253/14344   20135/19568/17889
+//   4,000 dipoles   9604/12086  13185/16321  18836/20941   23929/26773/26980   31800/36513/36416
+// and with 520 steps (rounds are 128 steps at least, so a launch's 10 us count):
+//   3,000 charges    755/  823   1006/  968   1352/ 1251    1715/ 1793/ 1408    2064/ 1911/ 1728
+//   8,000 charges    800/ 1310   1439/ 1829   2062/ 2343    2716/ 3040/ 3246    3745/ 3930/ 4028
+//   8,000 dipoles   1098/ 2090   2025/ 2876   3169/ 3752    3824/ 4296/ 4730    5352/ 5478/ 6082
+//   30,000 charges  1865/ 8113   3948/ 9229   6880/10177    9370/10075/13370   12191/13756/16096
+// (Above 20 lines per SM teams still win for 6,000 and more charges of long lines; at 24
+// with short ones they lose to hand-over or to neither.)
 // A frame of one Kahan run (2,048 sources) has nothing to split, so teams only add their
 // barriers and rounds; with two runs they pay up to 9 to 16 lines per SM, from three on
 // to 20, and to 32 where the persistent kernel reads sources from L2.  Hand-over

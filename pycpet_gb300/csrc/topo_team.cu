@@ -25,7 +25,7 @@
 // others still step several.
 //
 // Bound: FP32 pipe while lines x runs fill the warps, then the latency of one
-// run (32 dependent pair steps per lane) plus phases B and C.
+// run (32 dependent pair steps per lane) plus phase B and its two barriers.
 #include <algorithm>
 #include <climits>
 #include <cmath>
