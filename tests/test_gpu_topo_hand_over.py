@@ -1,7 +1,7 @@
 """Launches whose CTAs run out of lines and hand their last ones over while other
 warps of the CTA are between two steps: the same bits as the launch that hands
-nothing over (the allocation-free entry point), many times over.  Line counts
-around what a CTA holds (64 slots; 16 lines are handed over), step caps that make
+nothing over (the allocation-free entry point), many times over.  Frames of 12,800
+charges, whose lines are handed over whatever their length; line counts around what a CTA holds (64 slots; 16 lines are handed over), step caps that make
 slots run empty one by one, in groups and all at once."""
 import numpy as np
 import pytest
@@ -16,9 +16,10 @@ def test_handed_over_lines_keep_their_bits(gpu_lib, caps_of):
 
     sms = gpu_lib.cpetgb_device_sms()
     rng = np.random.default_rng(8)
-    x = rng.uniform(-30.0, 30.0, (900, 3))
-    x = torch.from_numpy(x[np.linalg.norm(x, axis=1) > 3.0][:300].copy()).cuda()
-    q = torch.from_numpy(rng.normal(0.0, 0.4, 300)).cuda()
+    n = 12800
+    x = rng.uniform(-40.0, 40.0, (2 * n, 3))
+    x = torch.from_numpy(x[np.linalg.norm(x, axis=1) > 3.0][:n].copy()).cuda()
+    q = torch.from_numpy(rng.normal(0.0, 0.4, n)).cuda()
     half = np.array([1.5, 1.5, 1.2])
     for per_sm in (21, 40, 64, 65, 90):
         L = sms * per_sm + 3
@@ -28,11 +29,11 @@ def test_handed_over_lines_keep_their_bits(gpu_lib, caps_of):
         res = torch.empty((L, 2), dtype=torch.float64, device="cuda")
         steps = torch.empty(L, dtype=torch.int32, device="cuda")
         stream = torch.cuda.current_stream().cuda_stream
-        rc = gpu_lib.cpetgb_topo_lines_noalloc(_lib.FP32C, L, 300, starts.data_ptr(), caps.data_ptr(), 0.01,
+        rc = gpu_lib.cpetgb_topo_lines_noalloc(_lib.FP32C, L, n, starts.data_ptr(), caps.data_ptr(), 0.01,
                                                half.ctypes.data, x.data_ptr(), q.data_ptr(), res.data_ptr(), None,
                                                steps.data_ptr(), stream)
         assert rc == 0, _lib.last_error()
-        for _ in range(10):
+        for _ in range(6):
             r, s = topo_lines(starts, caps, x, q, 0.01, half, precision="fp32c", return_steps=True)
             assert torch.equal(r, res) and torch.equal(s, steps)
 
@@ -45,13 +46,13 @@ def test_frames_beyond_the_records(gpu_lib):
     per_frame = 16 * gpu_lib.cpetgb_device_sms() + 70
     n_frames = (1 << 18) // (16 * gpu_lib.cpetgb_device_sms()) + 4
     rng = np.random.default_rng(9)
-    x = rng.uniform(-30.0, 30.0, (400, 3))
+    x = rng.uniform(-40.0, 40.0, (26000, 3))
     x = x[np.linalg.norm(x, axis=1) > 3.0]
     frames = []
     for f in range(n_frames):
-        n = 40 + f % 3
+        n = 12800 + f % 3
         frames.append({"x": x[:n], "q": rng.normal(0.0, 0.4, n), "starts": rng.uniform(-1.2, 1.2, (per_frame, 3)),
-                       "n_iter": rng.integers(0, 30, per_frame).astype(np.int32), "step": 0.02,
+                       "n_iter": rng.integers(0, 12, per_frame).astype(np.int32), "step": 0.02,
                        "half_dims": [1.5, 1.5, 1.2]})
     res, steps = TopoBatch(frames, precision="fp32c").run(return_steps=True)
     for f in (0, 1, n_frames // 2, n_frames - 5, n_frames - 3, n_frames - 1):

@@ -24,14 +24,16 @@ def _lines(L, seed):
     return rng.uniform(-1.2, 1.2, (L, 3)), rng.integers(0, 300, L).astype(np.int32)
 
 
-# 2 and 16 lines per SM: team kernel; 17 to 40: team or persistent kernel by precision and sources
+# 2 to 20 lines per SM: team kernel in FP64 and for 12,800 sources; 40: persistent kernel
+# with hand-over for those; 600 sources in FP32C: never either
 @pytest.mark.parametrize("dipoles", [False, True])
-@pytest.mark.parametrize("precision,step", [("fp32c", 0.01), ("fp32c", 0.3), ("fp64", 0.01), ("fp64", 0.3)])
-def test_single_frames(records, precision, step, dipoles):
+@pytest.mark.parametrize("precision,n,step", [("fp32c", 600, 0.01), ("fp32c", 12800, 0.01), ("fp32c", 12800, 0.3),
+                                              ("fp64", 600, 0.01), ("fp64", 600, 0.3)])
+def test_single_frames(records, precision, n, step, dipoles):
     from pycpet_gb300 import _lib, topo_dipole_lines, topo_lines
 
     sms = _lib.device_sms()
-    x, q, mu = _frame(600, 3)
+    x, q, mu = _frame(n, 3)
     fn, src = (topo_dipole_lines, mu) if dipoles else (topo_lines, q)
     for per_sm in (2, 16, 17, 20, 21, 40):
         starts, caps = _lines(sms * per_sm, per_sm)
@@ -44,15 +46,15 @@ def test_single_frames(records, precision, step, dipoles):
             np.testing.assert_array_equal(a, b)
 
 
-@pytest.mark.parametrize("precision", ["fp32c", "fp64"])
+@pytest.mark.parametrize("precision,sizes", [("fp32c", (300, 13900, 12800)), ("fp64", (300, 2049, 700))])
 @pytest.mark.parametrize("counts", [[3, 0, 40, 1], [900, 0, 1300, 700], [3000, 5, 2500]])
-def test_tables_and_plans(records, precision, counts):
+def test_tables_and_plans(records, precision, sizes, counts):
     import torch
     from pycpet_gb300 import TopoBatch
 
     frames = []
     for i, L in enumerate(counts):
-        x, q, _ = _frame((300, 2049, 700)[i % 3], i)
+        x, q, _ = _frame(sizes[i % 3], i)
         starts, caps = _lines(max(L, 1), 40 + i)
         frames.append({"x": x, "q": q, "starts": starts[:L], "n_iter": caps[:L], "step": 0.01 + 0.01 * (i % 2),
                        "half_dims": [1.5, 1.5, 1.2]})
@@ -75,8 +77,8 @@ def test_the_setting_is_the_threads_own(records):
 
     from pycpet_gb300 import topo_lines
 
-    x, q, _ = _frame(300, 4)
-    starts, caps = _lines(3000, 5)
+    x, q, _ = _frame(12800, 4)
+    starts, caps = _lines(5000, 5)
     want = topo_lines(starts, caps, x, q, 0.01, [1.5, 1.5, 1.2])
     assert records(0) == 0
     got = []
